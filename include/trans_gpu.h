@@ -343,7 +343,9 @@ const char* trans_tuning(void* ctx);
  * conversions, on n bit patterns (1..2^32) drawn from seed plus a fixed set of edge cases
  * (signed zeros, infinities, NaN, the float range limits, rounding ties).  mismatches[0]
  * counts double -> float results that differ in any bit, mismatches[1] float -> double (NaN
- * equals NaN); both are 0 on a correct build.  Errors: TRANS_E_ARG, TRANS_E_CUDA (message in
+ * equals NaN); both are 0 on a correct build.  The patterns, taken in pairs, also check the FP64
+ * path's integer-pipe quotients (counted in mismatches[0]) and square roots (mismatches[1])
+ * against the hardware's.  Errors: TRANS_E_ARG, TRANS_E_CUDA (message in
  * trans_last_error(NULL)). */
 int trans_check_conversions(long long n, unsigned long long seed, long long* mismatches);
 /* Message of the last failed call on ctx; with ctx = NULL, of the last failed context-free call

@@ -16,6 +16,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "soft64.cuh"
 #include "tmath.cuh"
 
 namespace tg {
@@ -166,6 +167,9 @@ struct CaseDev {
 };
 template <typename R> __host__ __device__ inline const ParamsT<R>& cparams(const CaseDev& c);
 template <> __host__ __device__ inline const ParamsT<double>& cparams<double>(const CaseDev& c) { return c.p; }
+template <> __host__ __device__ inline const ParamsT<f64>& cparams<f64>(const CaseDev& c) {
+    return reinterpret_cast<const ParamsT<f64>&>(c.p);
+}
 template <> __host__ __device__ inline const ParamsT<float>& cparams<float>(const CaseDev& c) { return c.pf; }
 
 __host__ __device__ inline int cidx(const DevBlock& b, int i, int j, int k) {
@@ -179,6 +183,7 @@ __device__ inline float* fslot(const DevBlock& b, int s) { return b.fbase + (siz
 // slot s in the arithmetic type R: the FP64 arrays, or their FP32 copies in the mixed path
 template <typename R> __device__ inline R* rs(const DevBlock& b, int s);
 template <> __device__ inline double* rs<double>(const DevBlock& b, int s) { return slot(b, s); }
+template <> __device__ inline f64* rs<f64>(const DevBlock& b, int s) { return reinterpret_cast<f64*>(slot(b, s)); }
 template <> __device__ inline float* rs<float>(const DevBlock& b, int s) { return fslot(b, s); }
 
 // face average of a cell quantity at the face stored at cell cf (Space/SPACEINTERP_GetSurfCenterVars.F90)
@@ -189,27 +194,30 @@ __device__ inline R favg(const R* q, const R* al, const R* ainv, int cf, int s) 
 
 template <typename R> __device__ inline R dmax(R a, R b) { return (a < b) ? b : a; }   // std::max
 template <typename R> __device__ inline R dmin(R a, R b) { return (b < a) ? b : a; }   // std::min
+__device__ inline f64 dmax(f64 a, f64 b) { return (a < b) ? b : a; }
+__device__ inline f64 dmin(f64 a, f64 b) { return (b < a) ? b : a; }
 template <typename R> __device__ inline R sgn1(R b) { return b >= R(0) ? R(1) : R(-1); }
 template <typename R> __device__ inline R sq(R x) { return x * x; }
 template <typename R> __device__ inline R p15(R x) { return x * sqrt(x); }
 // tanh: the bit-reproducible FP64 restatement, or the CUDA single-precision function
 template <typename R> __device__ inline R ttanh(R x);
-template <> __device__ inline double ttanh<double>(double x) { return tmx::tanh_(x); }
+template <> __device__ inline f64 ttanh<f64>(f64 x) { return f64(tmx::tanh_(x.v)); }
 template <> __device__ inline float ttanh<float>(float x) { return tanhf(x); }
 
 // atan: the bit-reproducible FP64 restatement, or the CUDA single-precision function
 template <typename R> __device__ inline R tatan(R x);
-template <> __device__ inline double tatan<double>(double x) { return tmx::atan_(x); }
+template <> __device__ inline f64 tatan<f64>(f64 x) { return f64(tmx::atan_(x.v)); }
 template <> __device__ inline float tatan<float>(float x) { return atanf(x); }
 // exp: the bit-reproducible FP64 restatement, or the CUDA single-precision function
 template <typename R> __device__ inline R texp(R x);
-template <> __device__ inline double texp<double>(double x) { return tmx::exp_(x); }
+template <> __device__ inline f64 texp<f64>(f64 x) { return f64(tmx::exp_(x.v)); }
+__device__ inline f64 tpow(f64 x, f64 y) { return f64(tmx::pow_(x.v, y.v)); }
 template <> __device__ inline float texp<float>(float x) { return expf(x); }
 // x**2. of a Fortran real exponent: the product, the correctly rounded power; x**10.: the pow
 // of tmath in FP64 (as the oracle), products in FP32
 template <typename R> __device__ inline R pow2_real(R x) { return x * x; }
 template <typename R> __device__ inline R pow10_real(R x);
-template <> __device__ inline double pow10_real<double>(double x) { return tmx::pow_(x, 10.0); }
+template <> __device__ inline f64 pow10_real<f64>(f64 x) { return f64(tmx::pow_(x.v, 10.0)); }
 template <> __device__ inline float pow10_real<float>(float x) {
     const float x2 = x * x, x4 = x2 * x2;
     return x4 * x4 * x2;
@@ -226,7 +234,7 @@ template <typename R> __device__ inline R mu_suth_nocs(const ParamsT<R>& p, R TT
 
 // x**3. of a Fortran real exponent: the pow of tmath in FP64 (as the oracle), x*x*x in FP32
 template <typename R> __device__ inline R cube_pow(R x);
-template <> __device__ inline double cube_pow<double>(double x) { return tmx::pow_(x, 3.0); }
+template <> __device__ inline f64 cube_pow<f64>(f64 x) { return f64(tmx::pow_(x.v, 3.0)); }
 template <> __device__ inline float cube_pow<float>(float x) { return x * x * x; }
 
 // x**2.0 of a Fortran real exponent (a base of either sign): the product, the correctly
@@ -277,17 +285,17 @@ __device__ inline void precond_apply(R* A, const R* t) {
 // PrecondDW coefficients of the cell at slot index c (FP64 slots; TIME_LUSGS.F90:113-160 and
 // every neighbour of the sweeps, :235-248): ubetac2 from getPrecondPara with the cell's
 // Rmiu and its smallest Alagm
-__device__ inline void precond_terms_at(const Params& p, const DevBlock& b, int c, double* t) {
-    const double pRo = slot(b, S_V)[c];
-    const double roinv = 1.0 / pRo;
-    const double pVx = slot(b, S_V + 1)[c] * roinv, pVy = slot(b, S_V + 2)[c] * roinv, pVz = slot(b, S_V + 3)[c] * roinv;
-    const double pE = slot(b, S_V + 4)[c] * roinv;
-    const double pPP = slot(b, S_PP)[c], pTT = slot(b, S_T)[c];
-    const double AAc = sqrt(1.4 * pPP * roinv);
-    const double UVW2 = pVx * pVx + pVy * pVy + pVz * pVz;
-    const double ALL = dmin(dmin(slot(b, S_ALAGM)[c], slot(b, S_ALAGM + 1)[c]), slot(b, S_ALAGM + 2)[c]);
-    const double ub = get_precond_para<double>(p, UVW2, AAc * AAc, pRo, pTT, slot(b, S_RMIU)[c], ALL);
-    precond_terms<double>(p, pRo, pVx, pVy, pVz, pE, AAc, ub, pTT, t);
+__device__ inline void precond_terms_at(const ParamsT<f64>& p, const DevBlock& b, int c, f64* t) {
+    const f64 pRo = rs<f64>(b, S_V)[c];
+    const f64 roinv = 1.0 / pRo;
+    const f64 pVx = rs<f64>(b, S_V + 1)[c] * roinv, pVy = rs<f64>(b, S_V + 2)[c] * roinv, pVz = rs<f64>(b, S_V + 3)[c] * roinv;
+    const f64 pE = rs<f64>(b, S_V + 4)[c] * roinv;
+    const f64 pPP = rs<f64>(b, S_PP)[c], pTT = rs<f64>(b, S_T)[c];
+    const f64 AAc = sqrt(1.4 * pPP * roinv);
+    const f64 UVW2 = pVx * pVx + pVy * pVy + pVz * pVz;
+    const f64 ALL = dmin(dmin(rs<f64>(b, S_ALAGM)[c], rs<f64>(b, S_ALAGM + 1)[c]), rs<f64>(b, S_ALAGM + 2)[c]);
+    const f64 ub = get_precond_para<f64>(p, UVW2, AAc * AAc, pRo, pTT, rs<f64>(b, S_RMIU)[c], ALL);
+    precond_terms<f64>(p, pRo, pVx, pVy, pVz, pE, AAc, ub, pTT, t);
 }
 
 // Space/UTIL_MUSCL.F90:2-18
@@ -302,7 +310,7 @@ template <typename R> __device__ inline R alimiter(R var1, R var2) {
 template <typename R> __device__ inline R muscl2_limiter(R var1, R var2) {
     const R epsm = R(1.0e-6);
     R smooth = (R(2.0) * var1 * var2 + epsm) / (var1 * var1 + var2 * var2 + epsm);
-    return ((R(1.0) + smooth) * var1 + (R(1.0) - smooth) * var2) * smooth / R(2.0);
+    return ((R(1.0) + smooth) * var1 + (R(1.0) - smooth) * var2) * smooth * R(0.5);
 }
 
 // Space/CONVECT_MDCD.F90:62-120: left (ql) and right (qr) face states from six cells
@@ -408,8 +416,8 @@ __device__ inline void roe_rot_common(const ParamsT<R>& p, R PLo, R PRo, R TLo, 
     const R eig1 = fabs(unormaln), eig2 = fabs(unormaln + am), eig3 = fabs(unormaln - am);
     const R alf = R(0.0), ubetac2 = R(1.0);
     const R dunormaln = (sav1n * (URo - ULo) + sav2n * (VRo - VLo) + sav3n * (WRo - WLo));
-    const R astar = (eig2 + eig3) / R(2.0);
-    const R Mstar = (eig2 - eig3) / R(2.0) / am;
+    const R astar = (eig2 + eig3) * R(0.5);
+    const R Mstar = (eig2 - eig3) * R(0.5) / am;
     const R dW1 = DENRo - DENLo, dU1 = URo - ULo, dU2 = VRo - VLo, dU3 = WRo - WLo, dP1 = PRo - PLo;
     const R dW2 = rm * dU1 + dW1 * um, dW3 = rm * dU2 + dW1 * vm, dW4 = rm * dU3 + dW1 * wm;
     const R dW5 = dP1 / ga1 + R(0.5) * vm2 * dW1 + rm * um * dU1 + rm * vm * dU2 + rm * wm * dU3;
@@ -491,7 +499,7 @@ __device__ inline void roe_flux(const ParamsT<R>& p, R PLo, R PRo, R TLo, R TRo,
     if (p.IF_Precondition) {        // Space/CONVECT_Roe_Original.F90:319-331 (RmiuT = VL(d,8), AlagmR = Alagm(d))
         R TTL = am2 / ga / R(p.PPF);
         ubetac2 = get_precond_para<R>(p, vm2, am2, rm, TTL, RmiuT, AlagmR);
-        alf = (R(1.0) - ubetac2) / R(2.0);
+        alf = (R(1.0) - ubetac2) * R(0.5);
         R unrev = unormaln * (R(1.0) - alf);
         amrev = sqrt(pow2r<R>(alf * unormaln) + ubetac2 * am2);
         eig1 = fabs(unormaln);
@@ -510,8 +518,8 @@ __device__ inline void roe_flux(const ParamsT<R>& p, R PLo, R PRo, R TLo, R TRo,
         amrev = am;
     }
     R dunormaln = (sav1n * (URo - ULo) + sav2n * (VRo - VLo) + sav3n * (WRo - WLo));
-    R astar = (eig2 + eig3) / R(2.0);
-    R Mstar = (eig2 - eig3) / R(2.0) / amrev;
+    R astar = (eig2 + eig3) * R(0.5);
+    R Mstar = (eig2 - eig3) * R(0.5) / amrev;
     R dW1 = DENRo - DENLo;
     R dU1 = URo - ULo, dU2 = VRo - VLo, dU3 = WRo - WLo;
     R dP1 = PRo - PLo;

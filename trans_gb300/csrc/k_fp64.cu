@@ -1,6 +1,6 @@
 // k_fp64.cu -- FP64 kernels of the hot path.  Compiled with -fmad=false so that every FP64
 // expression rounds exactly as the reference's (built with -fp-model strict) would.
-#define TG_R double
+#define TG_R tg::f64
 #define TG_NAME flux_launchers_f64
 #define TG_COMMON_KERNELS
 #include "flux_inst.cuh"

@@ -201,12 +201,32 @@ __device__ __forceinline__ unsigned long long cvt_mix(unsigned long long z) {
     z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
     return z ^ (z >> 31);
 }
+// soft64.cuh's quotient and root of a pair of patterns against the hardware's: any exponents, or
+// (one in two) exponents near each other, with dense, short, equal or all-ones significands
+__device__ __forceinline__ bool same_bits(double a, double h) {
+    return __double_as_longlong(a) == __double_as_longlong(h) || (isnan(a) && isnan(h));
+}
+__device__ void check_arith(unsigned long long x, unsigned long long y, unsigned long long* bad) {
+    const unsigned long long F = 0xfffffffffffffull;
+    const int k = (int)(y & 7);
+    if (k & 1) {
+        x = (x & (F | 1ull << 63)) | ((1003ull + (x >> 52) % 40ull) << 52);
+        y = (y & (F | 1ull << 63)) | ((1003ull + (y >> 52) % 40ull) << 52);
+    }
+    if (k >> 1 == 1) { x &= ~0xffffffffull; y &= ~0xfffffffffull; }
+    if (k >> 1 == 2) y = (y & ~F) | ((x + (y >> 8) % 5ull - 2ull) & F);
+    if (k >> 1 == 3) { x = (x & ~F) | (F - (x & 3ull)); y = (y & ~F) | (y >> 40 & 3ull); }
+    const double a = __longlong_as_double((long long)x), b = __longlong_as_double((long long)y);
+    if (!same_bits(sx::div(a, b), a / b)) atomicAdd(bad, 1ull);
+    if (!same_bits(sx::sqrt(fabs(a)), ::sqrt(fabs(a)))) atomicAdd(bad + 1, 1ull);
+}
 __global__ void k_check_cvt(long long n, unsigned long long seed, unsigned long long* __restrict__ bad) {
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
     const unsigned long long z = cvt_mix((unsigned long long)g ^ (seed * 0x2545f4914f6cdd1dull));
     unsigned long long u;
     const int kind = (int)(g & 3);
+    check_arith(z, cvt_mix(z), bad);
     if (g < CVT_NSPECIAL) {
         u = cvt_special[g];
         const unsigned f = (unsigned)(u >> 32) ^ (unsigned)u;     // a float pattern from it too

@@ -65,82 +65,81 @@ __global__ void k_specrad(const DevBlock* __restrict__ blks, const Tile* __restr
     const Tile t = tiles[blockIdx.x];
     if ((int)threadIdx.x >= t.count) return;
     const DevBlock b = blks[t.blk];
-    const Params p = cdev[b.cs].p;
-    const double CFL_sub = cdev[b.cs].CFL_sub;
+    const ParamsT<f64> p = cparams<f64>(cdev[b.cs]);
+    const f64 CFL_sub = cdev[b.cs].CFL_sub;
     int n = t.start + threadIdx.x;
     int I = n % b.NI1 + 1, J = (n / b.NI1) % b.NJ1 + 1, K = n / (b.NI1 * b.NJ1) + 1;
     int c = cidx(b, I, J, K);
-    const double* V = slot(b, S_V);
-    double Den = V[c];
-    double Vxi = slot(b, S_V + 1)[c] / Den;
-    double Vyi = slot(b, S_V + 2)[c] / Den;
-    double Vzi = slot(b, S_V + 3)[c] / Den;
-    double AAc = sqrt(1.4 * slot(b, S_PP)[c] / Den);
-    double TT = slot(b, S_T)[c];
-    double RmiuL = mu_suth<double>(p, TT);
-    double RmiuTL = slot(b, S_RMIU)[c];
-    double uvmu = (RmiuL + RmiuTL + 1.0e-20) * 4.0 / 3.0;
-    double uvmupr = (RmiuL / 0.72 + RmiuTL / 0.9 + 1.0e-20) * 1.4;
-    double pruvmu = dmax(uvmu, uvmupr) / Den;
-    double vol = slot(b, S_VOL)[c];
-    double rs = 0.0;
-    double Rd[3];
+    const f64* V = rs<f64>(b, S_V);
+    f64 Den = V[c];
+    f64 Vxi = rs<f64>(b, S_V + 1)[c] / Den;
+    f64 Vyi = rs<f64>(b, S_V + 2)[c] / Den;
+    f64 Vzi = rs<f64>(b, S_V + 3)[c] / Den;
+    f64 AAc = sqrt(1.4 * rs<f64>(b, S_PP)[c] / Den);
+    f64 TT = rs<f64>(b, S_T)[c];
+    f64 RmiuL = mu_suth<f64>(p, TT);
+    f64 RmiuTL = rs<f64>(b, S_RMIU)[c];
+    f64 uvmu = (RmiuL + RmiuTL + 1.0e-20) * 4.0 / 3.0;
+    f64 uvmupr = (RmiuL / 0.72 + RmiuTL / 0.9 + 1.0e-20) * 1.4;
+    f64 pruvmu = dmax(uvmu, uvmupr) / Den;
+    f64 vol = rs<f64>(b, S_VOL)[c];
+    f64 Rd[3];
     // low-Mach preconditioning (Time/SpectralRadius.F90:91-127): the acoustic speed and the
     // convective weight of each direction from ubetac2 and its viscous limit
-    double UVW2 = 0.0, ubetac2 = 1.0, RmiuAll = 0.0;
+    f64 UVW2 = 0.0, ubetac2 = 1.0, RmiuAll = 0.0;
     if (p.IF_Precondition) {
         UVW2 = Vxi * Vxi + Vyi * Vyi + Vzi * Vzi;
-        ubetac2 = get_precond_para<double>(p, UVW2, AAc * AAc, Den, 0.0, 0.0, 1.0);
+        ubetac2 = get_precond_para<f64>(p, UVW2, AAc * AAc, Den, 0.0, 0.0, 1.0);
         RmiuAll = RmiuL + RmiuTL;
     }
     for (int d = 0; d < 3; ++d) {
-        double ARX = slot(b, S_ASD + 3 * d)[c], ARY = slot(b, S_ASD + 3 * d + 1)[c], ARZ = slot(b, S_ASD + 3 * d + 2)[c];
-        double STsq = ARX * ARX + ARY * ARY + ARZ * ARZ;
-        double UU = Vxi * ARX + Vyi * ARY + Vzi * ARZ + 0.0;
-        double alf = 0.0, AAcd = AAc;
+        f64 ARX = rs<f64>(b, S_ASD + 3 * d)[c], ARY = rs<f64>(b, S_ASD + 3 * d + 1)[c], ARZ = rs<f64>(b, S_ASD + 3 * d + 2)[c];
+        f64 STsq = ARX * ARX + ARY * ARY + ARZ * ARZ;
+        f64 UU = Vxi * ARX + Vyi * ARY + Vzi * ARZ + 0.0;
+        f64 alf = 0.0, AAcd = AAc;
         if (p.IF_Precondition) {
-            double ubd = dmax(ubetac2, pow2r<double>(RmiuAll / Den / p.Ref / slot(b, S_ALAGM + d)[c] / AAc));
+            f64 ubd = dmax(ubetac2, pow2r<f64>(RmiuAll / Den / p.Ref / rs<f64>(b, S_ALAGM + d)[c] / AAc));
             alf = (1.0 - ubd) / 2.0;
             AAcd = sqrt(alf * alf * UVW2 + ubd * AAc * AAc);
         }
         Rd[d] = fabs(UU) * (1.0 - alf) + sqrt(STsq) * AAcd + 2.0 * STsq / vol * pruvmu / p.Ref;
-        slot(b, S_RDS + d)[c] = Rd[d];
+        rs<f64>(b, S_RDS + d)[c] = Rd[d];
     }
-    rs = Rd[0] + Rd[1] + Rd[2];
-    double Dtm_local = vol / rs;
-    double dtm = p.IF_Local_Main == 1 ? p.CFL_Main * Dtm_local : p.DT_LUSGS_Main;
+    const f64 rsum = Rd[0] + Rd[1] + Rd[2];
+    f64 Dtm_local = vol / rsum;
+    f64 dtm = p.IF_Local_Main == 1 ? p.CFL_Main * Dtm_local : p.DT_LUSGS_Main;
     if (p.Kind_Dual != 0) dtm = p.IF_Local_Sub == 1 ? CFL_sub * Dtm_local : p.DT_LUSGS_Sub;
-    slot(b, S_DTM)[c] = dtm;
+    rs<f64>(b, S_DTM)[c] = dtm;
 }
 
 // ---------------------------------------------------------------------------------------
 // BC/BC_Wall.F90, BC/BC_far.F90, BC/BC_Symm.F90, BC/BC_Inlet.F90, BC/BC_P2P.F90 (sweep -1)
 // ---------------------------------------------------------------------------------------
-__device__ inline void farbond(double XM, double P2, double RR, double Vxi, double Vyi, double Vzi, double DNx, double DNy,
-                               double DNz, double VxF, double VyF, double VzF, double& PP0, double& RR0, double& VX0,
-                               double& VY0, double& VZ0, double& dir) {
-    const double pGam = 1.4;
-    double AF = 1.0 / XM;
-    double AE = sqrt(pGam * P2 / RR);
-    double QNE = Vxi * DNx + Vyi * DNy + Vzi * DNz;
-    double QNF = VxF * DNx + VyF * DNy + VzF * DNz;
-    double RF = QNF - 5.0 * AF;
-    double RE = QNE + 5.0 * AE;
-    double QN = 0.5 * (RE + RF);
-    double AS = 0.1 * (RE - RF);
+__device__ inline void farbond(f64 XM, f64 P2, f64 RR, f64 Vxi, f64 Vyi, f64 Vzi, f64 DNx, f64 DNy,
+                               f64 DNz, f64 VxF, f64 VyF, f64 VzF, f64& PP0, f64& RR0, f64& VX0,
+                               f64& VY0, f64& VZ0, f64& dir) {
+    const f64 pGam = 1.4;
+    f64 AF = 1.0 / XM;
+    f64 AE = sqrt(pGam * P2 / RR);
+    f64 QNE = Vxi * DNx + Vyi * DNy + Vzi * DNz;
+    f64 QNF = VxF * DNx + VyF * DNy + VzF * DNz;
+    f64 RF = QNF - 5.0 * AF;
+    f64 RE = QNE + 5.0 * AE;
+    f64 QN = 0.5 * (RE + RF);
+    f64 AS = 0.1 * (RE - RF);
     if (QN > -AS && QN < 0.0) {
-        double SON = 1.0 / pGam / (XM * XM);
-        double QTX = VxF - QNF * DNx, QTY = VyF - QNF * DNy, QTZ = VzF - QNF * DNz;
+        f64 SON = 1.0 / pGam / (XM * XM);
+        f64 QTX = VxF - QNF * DNx, QTY = VyF - QNF * DNy, QTZ = VzF - QNF * DNz;
         VX0 = QTX + QN * DNx; VY0 = QTY + QN * DNy; VZ0 = QTZ + QN * DNz;
-        RR0 = tmx::pow_(AS * AS / SON / pGam, 2.5);
+        RR0 = tpow(AS * AS / SON / pGam, 2.5);
         PP0 = AS * AS * RR0 / pGam;
         dir = -1.0;
     }
     if (QN >= 0.0 && QN < AS) {
-        double SON = P2 / tmx::pow_(RR, pGam);
-        double QTX = Vxi - QNE * DNx, QTY = Vyi - QNE * DNy, QTZ = Vzi - QNE * DNz;
+        f64 SON = P2 / tpow(RR, pGam);
+        f64 QTX = Vxi - QNE * DNx, QTY = Vyi - QNE * DNy, QTZ = Vzi - QNE * DNz;
         VX0 = QTX + QN * DNx; VY0 = QTY + QN * DNy; VZ0 = QTZ + QN * DNz;
-        RR0 = tmx::pow_(AS * AS / SON / pGam, 2.5);
+        RR0 = tpow(AS * AS / SON / pGam, 2.5);
         PP0 = AS * AS * RR0 / pGam;
         dir = 1.0;
     }
@@ -164,38 +163,38 @@ __global__ void k_bc_state(const DevBlock* __restrict__ blks, const BCEntry* __r
     const BCEntry E = ent[e];
     if (E.kind == 7) return;                       // outlets run line by line in k_bc_outlet
     const DevBlock b = blks[E.blk];
-    const Params p = cdev[b.cs].p;
+    const ParamsT<f64> p = cparams<f64>(cdev[b.cs]);
     const int turb = cdev[b.cs].turb;
-    double* V[7];
-    for (int m = 0; m < 7; ++m) V[m] = slot(b, S_V + m);
-    double* PP = slot(b, S_PP);
-    double* T = slot(b, S_T);
-    double* Rm = slot(b, S_RMIU);
+    f64* V[7];
+    for (int m = 0; m < 7; ++m) V[m] = rs<f64>(b, S_V + m);
+    f64* PP = rs<f64>(b, S_PP);
+    f64* T = rs<f64>(b, S_T);
+    f64* Rm = rs<f64>(b, S_RMIU);
     const int s0 = E.s[0], l0 = E.l[0];
     if (E.kind == 1) {                              // BC/BC_Wall.F90:42-117
         // wall velocity of the frame Kindsub_BC * omega (BC_Wall.F90:46-52), as the reference
         // evaluates it (its sign of zero included)
-        const double ztemp = 0.5 * (slot(b, S_ZC)[s0] + slot(b, S_ZC)[l0]);
-        const double ytemp = 0.5 * (slot(b, S_YC)[s0] + slot(b, S_YC)[l0]);
-        const double vibc = 0.0;
-        const double vjbc = (double)E.kindsub * p.omega0 * ztemp;
-        const double vkbc = -(double)E.kindsub * p.omega0 * ytemp;
+        const f64 ztemp = 0.5 * (rs<f64>(b, S_ZC)[s0] + rs<f64>(b, S_ZC)[l0]);
+        const f64 ytemp = 0.5 * (rs<f64>(b, S_YC)[s0] + rs<f64>(b, S_YC)[l0]);
+        const f64 vibc = 0.0;
+        const f64 vjbc = (f64)E.kindsub * p.omega0 * ztemp;
+        const f64 vkbc = -(f64)E.kindsub * p.omega0 * ytemp;
         for (int L = 0; L < 3; ++L) {
             int is = E.s[L], il = E.l[L];
             PP[il] = PP[is];
             T[il] = T[is];
             V[0][il] = PP[il] / (T[il] + p.Tiny) * p.RXM2;
-            double den = V[0][il];
+            f64 den = V[0][il];
             V[1][il] = vibc * den;
             V[2][il] = vjbc * den;
             V[3][il] = vkbc * den;
         }
         if (turb) {
-            double Dn = slot(b, S_DST)[l0];
-            double Den = V[0][l0];
-            double TT = T[l0];
-            double Rmiuw = mu_suth<double>(p, TT);
-            double Omegaw = 60.0 * Rmiuw / (Den * 0.075 * Dn * Dn * p.Ref * p.Ref);
+            f64 Dn = rs<f64>(b, S_DST)[l0];
+            f64 Den = V[0][l0];
+            f64 TT = T[l0];
+            f64 Rmiuw = mu_suth<f64>(p, TT);
+            f64 Omegaw = 60.0 * Rmiuw / (Den * 0.075 * Dn * Dn * p.Ref * p.Ref);
             Rmiuw = Rm[s0];
             for (int L = 0; L < 3; ++L) {
                 int il = E.l[L];
@@ -206,19 +205,19 @@ __global__ void k_bc_state(const DevBlock* __restrict__ blks, const BCEntry* __r
         }
     } else if (E.kind == 2) {                       // BC/BC_far.F90:40-118
         int d = E.dir - 1;
-        double out_n = (double)(2 * E.lor - 4);
-        double grad = slot(b, S_GRAD + d)[E.face];
-        double Sout1 = slot(b, S_SD + 3 * d)[E.face] / grad;
-        double Sout2 = slot(b, S_SD + 3 * d + 1)[E.face] / grad;
-        double Sout3 = slot(b, S_SD + 3 * d + 2)[E.face] / grad;
-        double Dnx = Sout1 * out_n, Dny = Sout2 * out_n, Dnz = Sout3 * out_n;
-        double Den = V[0][s0];
-        double Vxi = V[1][s0] / Den, Vyi = V[2][s0] / Den, Vzi = V[3][s0] / Den;
-        double P2 = PP[s0];
-        double PP0 = 0, Den0 = 0, Vx0 = 0, Vy0 = 0, Vz0 = 0, dir = 0;
+        f64 out_n = (f64)(2 * E.lor - 4);
+        f64 grad = rs<f64>(b, S_GRAD + d)[E.face];
+        f64 Sout1 = rs<f64>(b, S_SD + 3 * d)[E.face] / grad;
+        f64 Sout2 = rs<f64>(b, S_SD + 3 * d + 1)[E.face] / grad;
+        f64 Sout3 = rs<f64>(b, S_SD + 3 * d + 2)[E.face] / grad;
+        f64 Dnx = Sout1 * out_n, Dny = Sout2 * out_n, Dnz = Sout3 * out_n;
+        f64 Den = V[0][s0];
+        f64 Vxi = V[1][s0] / Den, Vyi = V[2][s0] / Den, Vzi = V[3][s0] / Den;
+        f64 P2 = PP[s0];
+        f64 PP0 = 0, Den0 = 0, Vx0 = 0, Vy0 = 0, Vz0 = 0, dir = 0;
         farbond(p.XM, P2, Den, Vxi, Vyi, Vzi, Dnx, Dny, Dnz, p.VxF, p.VyF, p.VzF, PP0, Den0, Vx0, Vy0, Vz0, dir);
         V[0][l0] = 2 * Den0 - V[0][s0];
-        double den = V[0][l0];
+        f64 den = V[0][l0];
         V[1][l0] = 2.0 * Vx0 - Vxi;
         V[2][l0] = 2.0 * Vy0 - Vyi;
         V[3][l0] = 2.0 * Vz0 - Vzi;
@@ -236,9 +235,9 @@ __global__ void k_bc_state(const DevBlock* __restrict__ blks, const BCEntry* __r
                 V[6][l0] = V[6][s0];
                 Rm[l0] = Rm[s0];
             } else {
-                double TT = T[l0];
-                double Dn = V[0][l0];
-                double RmiuFar = mu_suth<double>(p, TT);
+                f64 TT = T[l0];
+                f64 Dn = V[0][l0];
+                f64 RmiuFar = mu_suth<f64>(p, TT);
                 Rm[l0] = 2.0 * p.VisRatio * RmiuFar - Rm[s0];
                 V[5][l0] = 2.0 * 1.5 * p.FSTI * p.FSTI * Dn - V[5][s0];
                 V[6][l0] = V[5][l0] / (Rm[l0] + p.Tiny) * Dn;
@@ -252,13 +251,13 @@ __global__ void k_bc_state(const DevBlock* __restrict__ blks, const BCEntry* __r
         }
     } else if (E.kind == 3) {                       // BC/BC_Symm.F90:42-110
         int d = E.dir - 1;
-        double grad = slot(b, S_GRAD + d)[E.face];
-        double Sout1 = slot(b, S_SD + 3 * d)[E.face] / grad;
-        double Sout2 = slot(b, S_SD + 3 * d + 1)[E.face] / grad;
-        double Sout3 = slot(b, S_SD + 3 * d + 2)[E.face] / grad;
-        double den = V[0][s0];
-        double Vxi = V[1][s0] / den, Vyi = V[2][s0] / den, Vzi = V[3][s0] / den;
-        double Vc1 = Vxi * Sout1 + Vyi * Sout2 + Vzi * Sout3;
+        f64 grad = rs<f64>(b, S_GRAD + d)[E.face];
+        f64 Sout1 = rs<f64>(b, S_SD + 3 * d)[E.face] / grad;
+        f64 Sout2 = rs<f64>(b, S_SD + 3 * d + 1)[E.face] / grad;
+        f64 Sout3 = rs<f64>(b, S_SD + 3 * d + 2)[E.face] / grad;
+        f64 den = V[0][s0];
+        f64 Vxi = V[1][s0] / den, Vyi = V[2][s0] / den, Vzi = V[3][s0] / den;
+        f64 Vc1 = Vxi * Sout1 + Vyi * Sout2 + Vzi * Sout3;
         for (int L = 0; L < 3; ++L) {
             int is = E.s[L], il = E.l[L];
             if (L != 1) V[0][il] = V[0][is];       // the second ghost layer keeps its density (BC_Symm.F90:70-75)
@@ -277,19 +276,19 @@ __global__ void k_bc_state(const DevBlock* __restrict__ blks, const BCEntry* __r
                 Rm[il] = Rm[is];
             }
     } else if (E.kind == 5) {                       // BC/BC_Inlet.F90:38-110
-        double PsIn = PP[s0];
+        f64 PsIn = PP[s0];
         PsIn = dmin(PsIn, 0.999 * p.P0in);
-        double comm = dmax(1.0, tmx::pow_(p.P0in / PsIn, 1.0 / 3.5));
-        double mach = sqrt((comm - 1.0) * 2 / 0.4);
-        double TsIn = p.T0in / comm;
-        double Roin = p.RXM2 * PsIn / TsIn;
-        double asonic = sqrt(1.4 * PsIn / Roin);
-        double Vabs = mach * asonic;
+        f64 comm = dmax(1.0, tpow(p.P0in / PsIn, 1.0 / 3.5));
+        f64 mach = sqrt((comm - 1.0) * 2 / 0.4);
+        f64 TsIn = p.T0in / comm;
+        f64 Roin = p.RXM2 * PsIn / TsIn;
+        f64 asonic = sqrt(1.4 * PsIn / Roin);
+        f64 Vabs = mach * asonic;
         V[0][l0] = Roin;
         V[1][l0] = Roin * Vabs;
-        V[2][l0] = Roin * (p.omega0 * slot(b, S_ZC)[s0]);
-        V[3][l0] = Roin * (-p.omega0 * slot(b, S_YC)[s0]);
-        double rr = p.omega0 * slot(b, S_RAD)[l0];
+        V[2][l0] = Roin * (p.omega0 * rs<f64>(b, S_ZC)[s0]);
+        V[3][l0] = Roin * (-p.omega0 * rs<f64>(b, S_YC)[s0]);
+        f64 rr = p.omega0 * rs<f64>(b, S_RAD)[l0];
         V[4][l0] = PsIn / 0.4 + 0.5 * (sq(V[1][l0]) + sq(V[2][l0]) + sq(V[3][l0])) / Roin - 0.5 * sq(rr) * Roin;
         PP[l0] = PsIn;
         T[l0] = TsIn;
@@ -300,10 +299,10 @@ __global__ void k_bc_state(const DevBlock* __restrict__ blks, const BCEntry* __r
             T[ig] = TsIn;
         }
         if (turb) {
-            double TT = T[l0];
-            double RmiuIn = mu_suth<double>(p, TT);
+            f64 TT = T[l0];
+            f64 RmiuIn = mu_suth<f64>(p, TT);
             Rm[l0] = p.VisRatio * RmiuIn;
-            double Den = V[0][l0];
+            f64 Den = V[0][l0];
             V[5][l0] = 1.5 * p.FSTI * p.FSTI * Den;
             V[6][l0] = V[5][l0] / (Rm[l0] + p.Tiny) * Den;
             for (int L = 1; L < 3; ++L) {
@@ -315,18 +314,18 @@ __global__ void k_bc_state(const DevBlock* __restrict__ blks, const BCEntry* __r
         }
     } else if (E.kind == 9) {                       // BC/BC_P2P.F90:76-139
         const DevBlock r = blks[E.src_blk];
-        const double cost = E.cost, sint = E.sint;
+        const f64 cost = E.cost, sint = E.sint;
         for (int L = 0; L < 3; ++L) {
             int is = E.s[L], il = E.l[L];
-            V[0][il] = slot(r, S_V)[is];
-            V[1][il] = slot(r, S_V + 1)[is];
-            double txy = slot(r, S_V + 2)[is], txz = slot(r, S_V + 3)[is];
+            V[0][il] = rs<f64>(r, S_V)[is];
+            V[1][il] = rs<f64>(r, S_V + 1)[is];
+            f64 txy = rs<f64>(r, S_V + 2)[is], txz = rs<f64>(r, S_V + 3)[is];
             V[2][il] = cost * txy + sint * txz;
             V[3][il] = -sint * txy + cost * txz;
-            for (int m = 4; m < 7; ++m) V[m][il] = slot(r, S_V + m)[is];
-            PP[il] = slot(r, S_PP)[is];
-            T[il] = slot(r, S_T)[is];
-            Rm[il] = slot(r, S_RMIU)[is];
+            for (int m = 4; m < 7; ++m) V[m][il] = rs<f64>(r, S_V + m)[is];
+            PP[il] = rs<f64>(r, S_PP)[is];
+            T[il] = rs<f64>(r, S_T)[is];
+            Rm[il] = rs<f64>(r, S_RMIU)[is];
         }
     }
 }
@@ -432,17 +431,17 @@ __global__ void k_prims(const DevBlock* __restrict__ blks, int nblk, long long t
     while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (off[mid] <= g) lo = mid; else hi = mid - 1; }
     const DevBlock b = blks[lo];
     int c = (int)(g - off[lo]);
-    double v1 = slot(b, S_V)[c];
-    slot(b, S_PRIM)[c] = slot(b, S_V + 1)[c] / v1;
-    slot(b, S_PRIM + 1)[c] = slot(b, S_V + 2)[c] / v1;
-    slot(b, S_PRIM + 2)[c] = slot(b, S_V + 3)[c] / v1;
-    slot(b, S_PRIM + 3)[c] = slot(b, S_V + 5)[c] / v1;
-    slot(b, S_PRIM + 4)[c] = slot(b, S_V + 6)[c] / v1;
-    double ri = 1.0 / v1;
-    slot(b, S_RINV)[c] = ri;
-    slot(b, S_SVEL)[c] = slot(b, S_V + 1)[c] * ri;
-    slot(b, S_SVEL + 1)[c] = slot(b, S_V + 2)[c] * ri;
-    slot(b, S_SVEL + 2)[c] = slot(b, S_V + 3)[c] * ri;
+    f64 v1 = rs<f64>(b, S_V)[c];
+    rs<f64>(b, S_PRIM)[c] = rs<f64>(b, S_V + 1)[c] / v1;
+    rs<f64>(b, S_PRIM + 1)[c] = rs<f64>(b, S_V + 2)[c] / v1;
+    rs<f64>(b, S_PRIM + 2)[c] = rs<f64>(b, S_V + 3)[c] / v1;
+    rs<f64>(b, S_PRIM + 3)[c] = rs<f64>(b, S_V + 5)[c] / v1;
+    rs<f64>(b, S_PRIM + 4)[c] = rs<f64>(b, S_V + 6)[c] / v1;
+    f64 ri = 1.0 / v1;
+    rs<f64>(b, S_RINV)[c] = ri;
+    rs<f64>(b, S_SVEL)[c] = rs<f64>(b, S_V + 1)[c] * ri;
+    rs<f64>(b, S_SVEL + 1)[c] = rs<f64>(b, S_V + 2)[c] * ri;
+    rs<f64>(b, S_SVEL + 2)[c] = rs<f64>(b, S_V + 3)[c] * ri;
 }
 
 // FP32 copies of FP64 slot ranges over every padded cell (mixed path)
@@ -512,7 +511,7 @@ __global__ void k_gradient(const DevBlock* __restrict__ blks, const Tile* __rest
     R DuDx = gq[0][0], DuDy = gq[0][1], DuDz = gq[0][2];
     R DvDx = gq[1][0], DvDy = gq[1][1], DvDz = gq[1][2];
     R DwDx = gq[2][0], DwDy = gq[2][1], DwDz = gq[2][2];
-    R W12 = (DuDy - DvDx) / R(2.0), W13 = (DuDz - DwDx) / R(2.0), W23 = (DvDz - DwDy) / R(2.0);
+    R W12 = (DuDy - DvDx) * R(0.5), W13 = (DuDz - DwDx) * R(0.5), W23 = (DvDz - DwDy) * R(0.5);
     R Vort = sqrt(R(2.0) * (R(2.0) * W12 * W12 + R(2.0) * W13 * W13 + R(2.0) * W23 * W23));
     R DivU = sqrt(DuDx * DuDx + DvDy * DvDy + DwDz * DwDz);
     rs<R>(b, S_SHOCK)[c] = DivU * DivU / dmax(DivU * DivU + Vort * Vort, R(1.0));
@@ -521,8 +520,8 @@ __global__ void k_gradient(const DevBlock* __restrict__ blks, const Tile* __rest
         // the hybrid blend Fscheme (Space/DIFF_DqDxyz.F90:311-380), read only by the rotated Roe
         // scheme: CH1 = 3, CH2 = 1, CH3 = 2, cmu = 0.09, tau = 1; real exponents 2 and 3 as
         // products, 0.5 as a square root
-        R S11 = (DuDx + DuDx) / R(2.), S22 = (DvDy + DvDy) / R(2.), S33 = (DwDz + DwDz) / R(2.);
-        R S12 = (DuDy + DvDx) / R(2.), S13 = (DuDz + DwDx) / R(2.), S23 = (DwDy + DvDz) / R(2.);
+        R S11 = (DuDx + DuDx) * R(0.5), S22 = (DvDy + DvDy) * R(0.5), S33 = (DwDz + DwDz) * R(0.5);
+        R S12 = (DuDy + DvDx) * R(0.5), S13 = (DuDz + DwDx) * R(0.5), S23 = (DwDy + DvDz) * R(0.5);
         R Skl = sqrt(R(2.) * (R(1.) * S11 * S11 + R(1.) * S22 * S22 + R(1.) * S33 * S33 + R(2.) * S12 * S12 +
                               R(2.) * S13 * S13 + R(2.) * S23 * S23));
         R Den = rs<R>(b, S_V)[c], RmiuT = rs<R>(b, S_RMIU)[c], TT = rs<R>(b, S_T)[c];
@@ -539,9 +538,9 @@ __global__ void k_gradient(const DevBlock* __restrict__ blks, const Tile* __rest
         R a2 = arg1 * arg1;
         R FunC1 = ttanh(a2 * a2);
         R aLgrd = ((R(1.) - FunC1) * R(0.61) + FunC1 * R(0.78)) * DLTxyz;
-        R B0 = R(2.) * Vort * dmax(Vort, Skl) / dmax((Vort * Vort + Skl * Skl) / R(2.), R(p.Alscale) * R(0.1));
+        R B0 = R(2.) * Vort * dmax(Vort, Skl) / dmax((Vort * Vort + Skl * Skl) * R(0.5), R(p.Alscale) * R(0.1));
         R g0 = ttanh(B0 * B0 * B0 * B0);
-        R sok = dmax(sqrt((Vort * Vort + Skl * Skl) / R(2.)), R(0.1) / R(1.0));
+        R sok = dmax(sqrt((Vort * Vort + Skl * Skl) * R(0.5)), R(0.1) / R(1.0));
         R alturb = sqrt((RmiuT + RMIUL) / Den / (Ref * sok * p15(R(0.09))));
         R A0 = R(1.) * dmax(((aLgrd / alturb / g0) - R(0.1)), R(0.0));
         rs<R>(b, S_FSCH)[c] = dmax(R(1.) * ttanh(A0 * A0 * A0), R(p.F_limiter1));
@@ -874,7 +873,7 @@ __device__ __forceinline__ void face_flux_body(const ParamsT<R>& p, int turb, co
     R sav = q.v(S_GRAD + d, 0);
     R f[5];
     if (p.Kind_Roe == 2) {          // rotated Roe: the contribution already carries |S|
-        const R Funscheme = (q.v(S_FSCH, -1) + q.v(S_FSCH, 0)) / R(2.);
+        const R Funscheme = (q.v(S_FSCH, -1) + q.v(S_FSCH, 0)) * R(0.5);
         roe_rotated<R>(p, qL[3], qR[3], qL[4], qR[4], qL[0], qR[0], qL[1], qR[1], qL[2], qR[2], sav1, sav2, sav3, sav,
                        rLo, rRo, Funscheme, f);
 #pragma unroll
@@ -1162,7 +1161,7 @@ __global__ void __launch_bounds__(CELL_TILE, sizeof(R) == 4 ? TG_PREP_MINB : TG_
             const R rvol = R(1.0) / rs<R>(b, S_VOL)[c];
             return rs<R>(b, S_D + L)[c] * rvol - R(bdf) * (R(0.5) / R(DT));
         } else {
-            return R((double)rs<R>(b, S_D + L)[c] / slot(b, S_VOL)[c] - bdf * 0.5 / DT);
+            return R(rs<R>(b, S_D + L)[c] / rs<R>(b, S_VOL)[c] - R(bdf) * R(0.5) / R(DT));
         }
     };
     if constexpr (MIXED) {
@@ -1171,11 +1170,11 @@ __global__ void __launch_bounds__(CELL_TILE, sizeof(R) == 4 ? TG_PREP_MINB : TG_
         cvs = stept / vol;
         fm = R(1.0) + (rs<R>(b, S_RDS)[c] + rs<R>(b, S_RDS + 1)[c] + rs<R>(b, S_RDS + 2)[c]) * cvs;
     } else {
-        const double Dtm = slot(b, S_DTM)[c], vol = slot(b, S_VOL)[c];
-        const double st = 2.0 * Dtm / (3.0 * Dtm / DT + 2.0);
-        const double cv = st / vol;
-        const double rsum = slot(b, S_RDS)[c] + slot(b, S_RDS + 1)[c] + slot(b, S_RDS + 2)[c];
-        stept = R(st); cvs = R(cv); fm = R(1.0 + rsum * cv);
+        const R Dtm = rs<R>(b, S_DTM)[c], vol = rs<R>(b, S_VOL)[c];
+        stept = R(2.0) * Dtm / (R(3.0) * Dtm / R(DT) + R(2.0));
+        cvs = stept / vol;
+        const R rsum = rs<R>(b, S_RDS)[c] + rs<R>(b, S_RDS + 1)[c] + rs<R>(b, S_RDS + 2)[c];
+        fm = R(1.0) + rsum * cvs;
     }
     // the diagonal terms into the record: FP64 path its four entries; mixed path the compact
     // record of this position (CompactRec: metric and radius per direction, velocity and total
@@ -1201,9 +1200,9 @@ __global__ void __launch_bounds__(CELL_TILE, sizeof(R) == 4 ? TG_PREP_MINB : TG_
     for (int L = 0; L < 5; ++L) DQ(L) = rhs(L);
     if constexpr (!MIXED) {
         if (pd.IF_Precondition) {     // the right-hand side preconditioned (TIME_LUSGS.F90:113-160)
-            double A[5] = {DQ(0), DQ(1), DQ(2), DQ(3), DQ(4)}, tpc[NPC];
-            precond_terms_at(pd, b, c, tpc);
-            precond_apply<double>(A, tpc);
+            R A[5] = {DQ(0), DQ(1), DQ(2), DQ(3), DQ(4)}, tpc[NPC];
+            precond_terms_at(p, b, c, tpc);
+            precond_apply<R>(A, tpc);
             for (int L = 0; L < 5; ++L) DQ(L) = A[L];
         }
     }
@@ -1396,13 +1395,13 @@ static __global__ void k_lusgs_jac_pc(const DevBlock* __restrict__ blks, const S
     if (nbp[sw_at(q, k, 6)] < 0) return;
     const SweepCell sc = cells[q];
     const DevBlock b = blks[sc.blk];
-    const Params p = cdev[b.cs].p;
+    const ParamsT<f64> p = cparams<f64>(cdev[b.cs]);
     const int c = cidx(b, sc.i, sc.j, sc.k);
     const int d = k % 3;
     const int st = d == 0 ? 1 : (d == 1 ? b.PI : b.PI * b.PJ);
-    double t[NPC];
+    f64 t[NPC];
     precond_terms_at(p, b, k < 3 ? c - st : c + st, t);
-    for (int m = 0; m < NPC; ++m) pc[sw_at(q, k * NPC + m, 6 * NPC)] = t[m];
+    for (int m = 0; m < NPC; ++m) pc[sw_at(q, k * NPC + m, 6 * NPC)] = t[m].v;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1428,6 +1427,9 @@ __device__ inline void sweep_map(int g, int lanes, int& e, int& L) {
     if (lanes & SWEEP_WPC) { e = (g / (32 * SWEEP_LANES)) * 32 + (g & 31); L = (g >> 5) % SWEEP_LANES; }
     else { e = g / SWEEP_LANES; L = g % SWEEP_LANES; }
 }
+
+__device__ __forceinline__ float ldcg(const float* p) { return __ldcg(p); }
+__device__ __forceinline__ f64 ldcg(const f64* p) { return f64(__ldcg(reinterpret_cast<const double*>(p))); }
 
 // Mixed-path (FP32) sweep step of one position, all seven components, from the compact records
 // (CompactRec).  Each neighbour's Jacobian row is rebuilt from its metric s, velocity v and total
@@ -1597,12 +1599,12 @@ __device__ inline void sweep_item(const int* __restrict__ nbp, const R* __restri
         for (int d = 0; d < 3; ++d) {
             const long long np = npv[d] >= 0 ? npv[d] : q;
 #pragma unroll
-            for (int m = 0; m < 5; ++m) nq[d][m] = __ldcg(dq + sw_at(np, m, DQ_STRIDE));
-            nt[d] = __ldcg(dq + sw_at(np, L < 5 ? 0 : L, DQ_STRIDE));
+            for (int m = 0; m < 5; ++m) nq[d][m] = ldcg(dq + sw_at(np, m, DQ_STRIDE));
+            nt[d] = ldcg(dq + sw_at(np, L < 5 ? 0 : L, DQ_STRIDE));
         }
     }
     R* D = dq + sw_at(q, L, DQ_STRIDE);
-    const R own = __ldcg(D);
+    const R own = ldcg(D);
     R acc[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -1613,7 +1615,7 @@ __device__ inline void sweep_item(const int* __restrict__ nbp, const R* __restri
         if (L < 5) {
             if (!hoist)
 #pragma unroll
-                for (int m = 0; m < 5; ++m) nq[d][m] = __ldcg(dq + sw_at(np, m, DQ_STRIDE));
+                for (int m = 0; m < 5; ++m) nq[d][m] = ldcg(dq + sw_at(np, m, DQ_STRIDE));
             const R AinRo = nq[d][0], AinRx = nq[d][1], AinRy = nq[d][2], AinRz = nq[d][3], AinRe = nq[d][4];
             R Dif;
             if (L == 0) {
@@ -1648,7 +1650,7 @@ __device__ inline void sweep_item(const int* __restrict__ nbp, const R* __restri
             val = R(0.5) * (Dif + sgn * (RDSt * Din));
         } else {
             const R VP = k[d][0];
-            const R Dq = hoist ? nt[d] : __ldcg(dq + sw_at(np, L, DQ_STRIDE));
+            const R Dq = hoist ? nt[d] : ldcg(dq + sw_at(np, L, DQ_STRIDE));
             val = R(0.5) * (Dq * VP + sgn * (RDSt * Dq));
         }
         acc[d] = has ? val : R(0.0);
@@ -1994,49 +1996,49 @@ __global__ void k_sweep_scatter(const DevBlock* __restrict__ blks, const Tile* _
 // F2-limited Cmu, the omega and k realizability limits and the eddy viscosity.  RmiuL is the
 // caller's laminar viscosity (the two routines evaluate Sutherland differently).
 // ---------------------------------------------------------------------------------------
-__device__ inline void sst_update(const Params& p, const DevBlock& b, int c, int d_fp32, double d6, double d7, double pRo,
-                                  double RmiuL) {
-    double* V5 = slot(b, S_V + 5);
-    double* V6 = slot(b, S_V + 6);
-    double ARTk = V5[c], ARTO = V6[c];
+__device__ inline void sst_update(const ParamsT<f64>& p, const DevBlock& b, int c, int d_fp32, f64 d6, f64 d7, f64 pRo,
+                                  f64 RmiuL) {
+    f64* V5 = rs<f64>(b, S_V + 5);
+    f64* V6 = rs<f64>(b, S_V + 6);
+    f64 ARTk = V5[c], ARTO = V6[c];
     if (d6 >= 0.0) ARTk = ARTk + d6;
-    else ARTk = ARTk * tmx::exp_(d6 / (ARTk + 1.e-10));
+    else ARTk = ARTk * texp<f64>(d6 / (ARTk + 1.e-10));
     ARTk = dmax(ARTk, 1.0e-10);
     if (d7 >= 0.0) ARTO = ARTO + d7;
-    else ARTO = ARTO * tmx::exp_(d7 / (ARTO + 1.e-10));
+    else ARTO = ARTO * texp<f64>(d7 / (ARTO + 1.e-10));
     ARTO = dmax(ARTO, 1.0e-10);
-    double DistN = slot(b, S_DST)[c];
-    auto G = [&](int q) { return d_fp32 ? (double)fslot(b, S_DQ + q)[c] : slot(b, S_DQ + q)[c]; };
-    double Dudx = G(0), Dudy = G(1), Dudz = G(2), Dvdx = G(3), Dvdy = G(4), Dvdz = G(5), Dwdx = G(6), Dwdy = G(7), Dwdz = G(8);
-    double Div = Dudx + Dvdy + Dwdz;
-    double prod = (2.0 * (Dudx * Dudx + Dvdy * Dvdy + Dwdz * Dwdz) + sq(Dudy + Dvdx) + sq(Dvdz + Dwdy) + sq(Dwdx + Dudz)
+    f64 DistN = rs<f64>(b, S_DST)[c];
+    auto G = [&](int q) { return d_fp32 ? f64((double)fslot(b, S_DQ + q)[c]) : rs<f64>(b, S_DQ + q)[c]; };
+    f64 Dudx = G(0), Dudy = G(1), Dudz = G(2), Dvdx = G(3), Dvdy = G(4), Dvdz = G(5), Dwdx = G(6), Dwdy = G(7), Dwdz = G(8);
+    f64 Div = Dudx + Dvdy + Dwdz;
+    f64 prod = (2.0 * (Dudx * Dudx + Dvdy * Dvdy + Dwdz * Dwdz) + sq(Dudy + Dvdx) + sq(Dvdz + Dwdy) + sq(Dwdx + Dudz)
                    - 2.0 / 3.0 * Div * Div);
     if (p.Kind_Model == 2) {    // Wilcox 2006 (TIME_Update_V.F90:821-858, TIME_RK_V_Update_New.F90:195-232)
-        double Sii = Dudx - (Dudx + Dvdy + Dwdz) / 3.;
-        double Sjj = Dvdy - (Dudx + Dvdy + Dwdz) / 3.;
-        double Skk = Dwdz - (Dudx + Dvdy + Dwdz) / 3.;
-        double Sij = (Dudy + Dvdx) / 2.0, Sik = (Dudz + Dwdx) / 2.0, Sjk = (Dvdz + Dwdy) / 2.0;
-        double Skl = sqrt(1.0 * Sii * Sii + 1.0 * Sjj * Sjj + 1.0 * Skk * Skk + 2.0 * Sij * Sij + 2.0 * Sik * Sik + 2.0 * Sjk * Sjk);
+        f64 Sii = Dudx - (Dudx + Dvdy + Dwdz) / 3.;
+        f64 Sjj = Dvdy - (Dudx + Dvdy + Dwdz) / 3.;
+        f64 Skk = Dwdz - (Dudx + Dvdy + Dwdz) / 3.;
+        f64 Sij = (Dudy + Dvdx) * 0.5, Sik = (Dudz + Dwdx) * 0.5, Sjk = (Dvdz + Dwdy) * 0.5;
+        f64 Skl = sqrt(1.0 * Sii * Sii + 1.0 * Sjj * Sjj + 1.0 * Skk * Skk + 2.0 * Sij * Sij + 2.0 * Sik * Sik + 2.0 * Sjk * Sjk);
         ARTO = dmax(ARTO, sqrt(pRo * fabs(prod) / (p.Prod_Lmt * p.Beta_star)) / p.Ref);
         ARTk = dmin(ARTk, 100000.0 * RmiuL * ARTO / pRo);
         V5[c] = ARTk;
         V6[c] = ARTO;
         ARTO = dmax(ARTO, 7. / 8. * pRo * sqrt(Skl * Skl * 2. / 0.09) / p.Ref);
-        slot(b, S_RMIU)[c] = ARTk / ARTO * pRo;
+        rs<f64>(b, S_RMIU)[c] = ARTk / ARTO * pRo;
         return;
     }
-    double arg2 = 2.0 * sqrt(ARTk / pRo) / p.Beta_star / (ARTO / pRo) / DistN / p.Ref;
+    f64 arg2 = 2.0 * sqrt(ARTk / pRo) / p.Beta_star / (ARTO / pRo) / DistN / p.Ref;
     arg2 = dmax(arg2, 500.0 * RmiuL / DistN / DistN / ARTO / p.Ref / p.Ref);
-    arg2 = tmx::tanh_(arg2 * arg2);
-    double Sii = Dudx, Sjj = Dvdy, Skk = Dwdz;
-    double Sij = (Dudy + Dvdx) / 2.0, Sik = (Dudz + Dwdx) / 2.0, Sjk = (Dvdz + Dwdy) / 2.0;
-    double Skl = sqrt(2.0 * (1.0 * Sii * Sii + 1.0 * Sjj * Sjj + 1.0 * Skk * Skk + 2.0 * Sij * Sij + 2.0 * Sik * Sik + 2.0 * Sjk * Sjk));
-    double Cmua = dmin(1.0, p.A1 * ARTO / pRo / ((Skl) * arg2 + 1.e-10) * p.Ref);
+    arg2 = ttanh<f64>(arg2 * arg2);
+    f64 Sii = Dudx, Sjj = Dvdy, Skk = Dwdz;
+    f64 Sij = (Dudy + Dvdx) * 0.5, Sik = (Dudz + Dwdx) * 0.5, Sjk = (Dvdz + Dwdy) * 0.5;
+    f64 Skl = sqrt(2.0 * (1.0 * Sii * Sii + 1.0 * Sjj * Sjj + 1.0 * Skk * Skk + 2.0 * Sij * Sij + 2.0 * Sik * Sik + 2.0 * Sjk * Sjk));
+    f64 Cmua = dmin(1.0, p.A1 * ARTO / pRo / ((Skl) * arg2 + 1.e-10) * p.Ref);
     ARTO = dmax(ARTO, sqrt(pRo * Cmua * fabs(prod) / (p.Prod_Lmt * p.Beta_star)) / p.Ref);
     ARTk = dmin(ARTk, 100000.0 * RmiuL * ARTO / pRo / Cmua);
     V5[c] = ARTk;
     V6[c] = ARTO;
-    slot(b, S_RMIU)[c] = Cmua * ARTk / ARTO * pRo;
+    rs<f64>(b, S_RMIU)[c] = Cmua * ARTk / ARTO * pRo;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -2046,7 +2048,7 @@ __global__ void k_update(const DevBlock* __restrict__ blks, const Tile* __restri
                          NormPart* __restrict__ parts, int d_fp32) {
     const Tile t = tiles[blockIdx.x];
     const DevBlock b = blks[t.blk];
-    const Params p = cdev[b.cs].p;
+    const ParamsT<f64> p = cparams<f64>(cdev[b.cs]);
     const int turb_upd = cdev[b.cs].turb_upd;
     int tid = threadIdx.x;
     double sa = 0, ma = -1, sk = 0, mk = 0, so = 0, mo = 0;
@@ -2056,57 +2058,57 @@ __global__ void k_update(const DevBlock* __restrict__ blks, const Tile* __restri
         int n = t.start + tid;
         int I = n % b.NI1 + 1, J = (n / b.NI1) % b.NJ1 + 1, K = n / (b.NI1 * b.NJ1) + 1;
         int c = cidx(b, I, J, K);
-        double* V[7];
-        for (int m = 0; m < 7; ++m) V[m] = slot(b, S_V + m);
-        double* PP = slot(b, S_PP);
-        double* T = slot(b, S_T);
-        double v1 = V[0][c];
+        f64* V[7];
+        for (int m = 0; m < 7; ++m) V[m] = rs<f64>(b, S_V + m);
+        f64* PP = rs<f64>(b, S_PP);
+        f64* T = rs<f64>(b, S_T);
+        f64 v1 = V[0][c];
         // DeltaQ from the sweeps: FP64, or FP32 in the mixed path
-        auto Dq = [&](int L) { return d_fp32 ? (double)fslot(b, S_D + L)[c] : slot(b, S_D + L)[c]; };
-        double d1 = Dq(0), d6 = Dq(5), d7 = Dq(6);
-        double DR = fabs(d1 / v1);
-        nanf = isnan(d1) ? 1 : 0;
-        sa = DR * DR; ma = DR; ia = n;
-        double DRk = fabs(d6 / v1), DRo = fabs(d7 / v1);
-        sk = DRk * DRk; mk = DRk; so = DRo * DRo; mo = DRo;
+        auto Dq = [&](int L) { return d_fp32 ? f64((double)fslot(b, S_D + L)[c]) : rs<f64>(b, S_D + L)[c]; };
+        f64 d1 = Dq(0), d6 = Dq(5), d7 = Dq(6);
+        f64 DR = fabs(d1 / v1);
+        nanf = isnan(d1.v) ? 1 : 0;
+        sa = (DR * DR).v; ma = DR.v; ia = n;
+        f64 DRk = fabs(d6 / v1), DRo = fabs(d7 / v1);
+        sk = (DRk * DRk).v; mk = DRk.v; so = (DRo * DRo).v; mo = DRo.v;
         // mean flow (non-preconditioned, TIME_Update_V.F90:621-689)
-        double AinRo = d1, AinRx = Dq(1), AinRy = Dq(2), AinRz = Dq(3);
-        double AinRe = Dq(4);
-        double pRo = v1;
-        double roinv = 1.0 / pRo;
-        double rr = p.omega0 * slot(b, S_RAD)[c];
+        f64 AinRo = d1, AinRx = Dq(1), AinRy = Dq(2), AinRz = Dq(3);
+        f64 AinRe = Dq(4);
+        f64 pRo = v1;
+        f64 roinv = 1.0 / pRo;
+        f64 rr = p.omega0 * rs<f64>(b, S_RAD)[c];
         if (p.IF_Precondition) {
             // preconditioned (TIME_Update_V.F90:580-607): conservative increments; the kinetic
             // energy takes the new momenta with the old 1/rho, and T the old pressure with the
             // new density
-            double pRx = V[1][c], pRy = V[2][c], pRz = V[3][c], pRe = V[4][c];
+            f64 pRx = V[1][c], pRy = V[2][c], pRz = V[3][c], pRe = V[4][c];
             pRo = pRo + AinRo;
             pRo = fabs(pRo);
             pRx = pRx + AinRx; pRy = pRy + AinRy; pRz = pRz + AinRz;
             pRe = pRe + AinRe;
             pRe = fabs(pRe);
-            double DV = 0.5 * (pRx * pRx + pRy * pRy + pRz * pRz) * roinv;
-            double pPP = (pRe - DV) * (1.4 - 1.0);
+            f64 DV = 0.5 * (pRx * pRx + pRy * pRy + pRz * pRz) * roinv;
+            f64 pPP = (pRe - DV) * (1.4 - 1.0);
             if (pPP <= 0.0) {
                 pPP = fabs(pPP);
                 pRe = pPP / (1.4 - 1.0) + DV;
             }
-            double pTT = p.RXM2 * PP[c] / pRo;
+            f64 pTT = p.RXM2 * PP[c] / pRo;
             V[0][c] = pRo; V[1][c] = pRx; V[2][c] = pRy; V[3][c] = pRz; V[4][c] = pRe;
             PP[c] = pPP;
             T[c] = pTT;
         } else {
-        double pVx = V[1][c] * roinv, pVy = V[2][c] * roinv, pVz = V[3][c] * roinv;
-        double AinX = (AinRx - pVx * AinRo) * roinv;
-        double AinY = (AinRy - pVy * AinRo) * roinv;
-        double AinZ = (AinRz - pVz * AinRo) * roinv;
-        double AinP = (1.4 - 1.0) * (AinRe - 0.5 * AinRo * (pVx * pVx + pVy * pVy + pVz * pVz) - pRo * (AinX * pVx + AinY * pVy + AinZ * pVz));
+        f64 pVx = V[1][c] * roinv, pVy = V[2][c] * roinv, pVz = V[3][c] * roinv;
+        f64 AinX = (AinRx - pVx * AinRo) * roinv;
+        f64 AinY = (AinRy - pVy * AinRo) * roinv;
+        f64 AinZ = (AinRz - pVz * AinRo) * roinv;
+        f64 AinP = (1.4 - 1.0) * (AinRe - 0.5 * AinRo * (pVx * pVx + pVy * pVy + pVz * pVz) - pRo * (AinX * pVx + AinY * pVy + AinZ * pVz));
         if (AinRo >= 0.) pRo = pRo + AinRo;
-        else pRo = pRo * tmx::exp_(AinRo / (pRo + 1.e-10));
+        else pRo = pRo * texp<f64>(AinRo / (pRo + 1.e-10));
         pRo = fabs(pRo);
-        double pp = PP[c];
+        f64 pp = PP[c];
         if (AinP >= 0.) pp = pp + AinP;
-        else pp = pp * tmx::exp_(AinP / (pp + 1.e-10));
+        else pp = pp * texp<f64>(AinP / (pp + 1.e-10));
         pp = fabs(pp);
         PP[c] = pp;
         T[c] = p.RXM2 * pp / pRo;
@@ -2115,14 +2117,14 @@ __global__ void k_update(const DevBlock* __restrict__ blks, const Tile* __restri
         V[1][c] = pRo * pVx;
         V[2][c] = pRo * pVy;
         V[3][c] = pRo * pVz;
-        double DV = 0.5 * (pVx * pVx + pVy * pVy + pVz * pVz);
+        f64 DV = 0.5 * (pVx * pVx + pVy * pVy + pVz * pVz);
         V[4][c] = pp / (1.4 - 1.0) + DV * pRo - 0.5 * sq(rr) * pRo;
         }
         if (turb_upd) {   // TIME_Update_V.F90:709-816
-            double VV = sq(V[1][c]) + sq(V[2][c]) + sq(V[3][c]);
-            double PPP = (1.4 - 1.0) * V[4][c] - 0.5 * (1.4 - 1.0) * (VV / pRo - sq(rr) * pRo);
-            double TT = p.RXM2 * PPP / pRo;
-            sst_update(p, b, c, d_fp32, d6, d7, pRo, mu_suth<double>(p, TT));
+            f64 VV = sq(V[1][c]) + sq(V[2][c]) + sq(V[3][c]);
+            f64 PPP = (1.4 - 1.0) * V[4][c] - 0.5 * (1.4 - 1.0) * (VV / pRo - sq(rr) * pRo);
+            f64 TT = p.RXM2 * PPP / pRo;
+            sst_update(p, b, c, d_fp32, d6, d7, pRo, mu_suth<f64>(p, TT));
         }
     }
     NormPart P;
@@ -2151,29 +2153,29 @@ __global__ void k_rk_update(const DevBlock* __restrict__ blks, const Tile* __res
         const int I = n % b.NI1 + 1, J = (n / b.NI1) % b.NJ1 + 1, K = n / (b.NI1 * b.NJ1) + 1;
         const int c = cidx(b, I, J, K);
         if (itr == 1)
-            for (int L = 0; L < 7; ++L) slot(b, S_WT2 + L)[c] = slot(b, S_V + L)[c];
-        auto Dq = [&](int L) { return d_fp32 ? (double)fslot(b, S_D + L)[c] : slot(b, S_D + L)[c]; };
-        const double d1 = Dq(0);
-        const double DR = fabs(d1 / slot(b, S_V)[c]);
-        nanf = isnan(d1) ? 1 : 0;
-        sa = DR * DR; ma = DR; ia = n;
-        const double dtm = slot(b, S_DTM)[c], vol = slot(b, S_VOL)[c];
-        double v[5];
+            for (int L = 0; L < 7; ++L) rs<f64>(b, S_WT2 + L)[c] = rs<f64>(b, S_V + L)[c];
+        auto Dq = [&](int L) { return d_fp32 ? f64((double)fslot(b, S_D + L)[c]) : rs<f64>(b, S_D + L)[c]; };
+        const f64 d1 = Dq(0);
+        const f64 DR = fabs(d1 / rs<f64>(b, S_V)[c]);
+        nanf = isnan(d1.v) ? 1 : 0;
+        sa = (DR * DR).v; ma = DR.v; ia = n;
+        const f64 dtm = rs<f64>(b, S_DTM)[c], vol = rs<f64>(b, S_VOL)[c];
+        f64 v[5];
         for (int L = 0; L < 5; ++L) {
-            const double d = Dq(L), w = slot(b, S_WT2 + L)[c];
-            double x = slot(b, S_V + L)[c];
+            const f64 d = Dq(L), w = rs<f64>(b, S_WT2 + L)[c];
+            f64 x = rs<f64>(b, S_V + L)[c];
             if (itr == 1) x = x + dtm * d / vol;
             else if (itr == 2) x = 0.75 * w + 0.25 * x + 0.25 * dtm * d / vol;
             else x = 1.0 / 3.0 * w + 2.0 / 3.0 * x + 2.0 / 3.0 * dtm * d / vol;
-            slot(b, S_V + L)[c] = x;
+            rs<f64>(b, S_V + L)[c] = x;
             v[L] = x;
         }
-        const double ri = 1.0 / v[0];
-        const double u = v[1] * ri, vv = v[2] * ri, w = v[3] * ri;
-        slot(b, S_RINV)[c] = ri;
-        slot(b, S_SVEL)[c] = u;
-        slot(b, S_SVEL + 1)[c] = vv;
-        slot(b, S_SVEL + 2)[c] = w;
+        const f64 ri = 1.0 / v[0];
+        const f64 u = v[1] * ri, vv = v[2] * ri, w = v[3] * ri;
+        rs<f64>(b, S_RINV)[c] = ri;
+        rs<f64>(b, S_SVEL)[c] = u;
+        rs<f64>(b, S_SVEL + 1)[c] = vv;
+        rs<f64>(b, S_SVEL + 2)[c] = w;
         if (d_fp32) {
             for (int L = 0; L < 5; ++L) fslot(b, S_V + L)[c] = (float)v[L];
             fslot(b, S_RINV)[c] = (float)ri;
@@ -2198,7 +2200,7 @@ __global__ void k_rk_vupdate(const DevBlock* __restrict__ blks, const Tile* __re
                              NormPart* __restrict__ parts, int d_fp32) {
     const Tile t = tiles[blockIdx.x];
     const DevBlock b = blks[t.blk];
-    const Params p = cdev[b.cs].p;
+    const ParamsT<f64> p = cparams<f64>(cdev[b.cs]);
     const int turb_upd = cdev[b.cs].turb_upd;
     const int tid = threadIdx.x;
     double sk = 0, mk = 0, so = 0, mo = 0;
@@ -2206,22 +2208,22 @@ __global__ void k_rk_vupdate(const DevBlock* __restrict__ blks, const Tile* __re
         const int n = t.start + tid;
         const int I = n % b.NI1 + 1, J = (n / b.NI1) % b.NJ1 + 1, K = n / (b.NI1 * b.NJ1) + 1;
         const int c = cidx(b, I, J, K);
-        const double v1 = slot(b, S_V)[c], v2 = slot(b, S_V + 1)[c], v3 = slot(b, S_V + 2)[c];
-        const double v4 = slot(b, S_V + 3)[c], v5 = slot(b, S_V + 4)[c];
-        double VV = v2 * v2 + v3 * v3 + v4 * v4;
-        const double pp = (1.4 - 1.0) * v5 - 0.5 * (1.4 - 1.0) * VV / v1;
-        slot(b, S_PP)[c] = pp;
-        slot(b, S_T)[c] = p.RXM2 * pp / v1;
-        auto Dq = [&](int L) { return d_fp32 ? (double)fslot(b, S_D + L)[c] : slot(b, S_D + L)[c]; };
-        const double d6 = Dq(5), d7 = Dq(6);
+        const f64 v1 = rs<f64>(b, S_V)[c], v2 = rs<f64>(b, S_V + 1)[c], v3 = rs<f64>(b, S_V + 2)[c];
+        const f64 v4 = rs<f64>(b, S_V + 3)[c], v5 = rs<f64>(b, S_V + 4)[c];
+        f64 VV = v2 * v2 + v3 * v3 + v4 * v4;
+        const f64 pp = (1.4 - 1.0) * v5 - 0.5 * (1.4 - 1.0) * VV / v1;
+        rs<f64>(b, S_PP)[c] = pp;
+        rs<f64>(b, S_T)[c] = p.RXM2 * pp / v1;
+        auto Dq = [&](int L) { return d_fp32 ? f64((double)fslot(b, S_D + L)[c]) : rs<f64>(b, S_D + L)[c]; };
+        const f64 d6 = Dq(5), d7 = Dq(6);
         if (turb_upd) {
             VV = sq(v2) + sq(v3) + sq(v4);
-            const double PPP = 0.4 * v5 - 0.2 * VV / v1;
-            const double TT = p.RXM2 * PPP / v1;
-            sst_update(p, b, c, d_fp32, d6, d7, v1, mu_suth_nocs<double>(p, TT));
+            const f64 PPP = 0.4 * v5 - 0.2 * VV / v1;
+            const f64 TT = p.RXM2 * PPP / v1;
+            sst_update(p, b, c, d_fp32, d6, d7, v1, mu_suth_nocs<f64>(p, TT));
         }
-        const double DRk = fabs(d6 / v1), DRo = fabs(d7 / v1);
-        sk = DRk * DRk; mk = DRk; so = DRo * DRo; mo = DRo;
+        const f64 DRk = fabs(d6 / v1), DRo = fabs(d7 / v1);
+        sk = (DRk * DRk).v; mk = DRk.v; so = (DRo * DRo).v; mo = DRo.v;
     }
     NormPart P = norm_identity();
     P.sk = sk; P.so = so; P.mk = mk; P.mo = mo;

@@ -12,11 +12,18 @@
 // Their accuracy against the platform libm is checked in the test-suite (a few ulp).
 #pragma once
 #include <math.h>
+#include "soft64.cuh"
 
 #ifdef __CUDACC__
 #define TM_HD __host__ __device__
 #else
 #define TM_HD
+#endif
+// the quotients: on the device the integer-pipe form of the same value (soft64.cuh)
+#ifdef __CUDA_ARCH__
+#define TM_DIV(a, b) sx::div(a, b)
+#else
+#define TM_DIV(a, b) ((a) / (b))
 #endif
 
 namespace tmx {
@@ -78,7 +85,7 @@ TM_HD inline double tanh_(double x) {
     if (ax > 22.0) t = 1.0;
     else {
         double e = expm1_(-2.0 * ax);
-        t = -e / (e + 2.0);
+        t = TM_DIV(-e, e + 2.0);
     }
     return copysign(t, x);
 }
@@ -90,7 +97,7 @@ TM_HD inline double log_(double x) {
     int e;
     double m = frexp(x, &e);
     if (m < SQRT_HALF) { m = m * 2.0; e = e - 1; }
-    double s = (m - 1.0) / (m + 1.0);
+    double s = TM_DIV(m - 1.0, m + 1.0);
     double s2 = s * s;
     double p = 1.0 / 25.0;
     p = p * s2 + 1.0 / 23.0;
@@ -121,9 +128,9 @@ TM_HD inline double atan_(double x) {
     const double TAN_PI_8 = 0.41421356237309503;
     double ax = fabs(x);
     bool inv = ax > 1.0;
-    double t = inv ? 1.0 / ax : ax;
+    double t = inv ? TM_DIV(1.0, ax) : ax;
     bool red = t > TAN_PI_8;
-    if (red) t = (t - 1.0) / (t + 1.0);
+    if (red) t = TM_DIV(t - 1.0, t + 1.0);
     double z = -(t * t);
     double p = 1.0 / 43.0;
     p = p * z + 1.0 / 41.0;
