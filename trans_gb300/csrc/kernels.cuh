@@ -785,14 +785,17 @@ __device__ __forceinline__ void face_flux_body(const ParamsT<R>& p, int turb, co
     }   // PART != 2
     if constexpr (PART == 1) return;
     // ---------------- reconstruction ----------------
+    // u, v, w, p, T.  FP64: one copy of the loop body.  Five copies with their integer-pipe quotients
+    // are ~200 KB of straight-line code, and the warps waited for instructions (MDCD face fluxes of
+    // the benchmark cascade 16.8 -> 16.0 ms per iteration)
     R qL[7], qR[7];
-    constexpr int qc[5] = {S_PRIM, S_PRIM + 1, S_PRIM + 2, S_PP, S_T};
+    constexpr int UNROLL = sizeof(R) == 8 ? 1 : 5;
     R gama = R(0.0);
     if (p.Kind_Spatial <= 2) {     // CONVECT_MUSCL (2) or CONVECT_MUSCL2 (1): the limiter differs
         const bool m2 = p.Kind_Spatial == 1;
-#pragma unroll
+#pragma unroll UNROLL
         for (int k = 0; k < 5; ++k) {
-            const int Q = qc[k];
+            const int Q = k < 3 ? S_PRIM + k : S_PP + (k - 3);
             R fm = fa(Q, -1), f0 = fa(Q, 0), fp = fa(Q, 1);
             R q1 = q.v(Q, -1), q0 = q.v(Q, 0);
             R DR = f0 - q1, DL = q1 - fm;
@@ -812,9 +815,9 @@ __device__ __forceinline__ void face_flux_body(const ParamsT<R>& p, int turb, co
         gama = R(p.gama_min) + sensor * (R(p.gama_max) - R(p.gama_min));
         // MDCDHYB: MUSCL states where the sensor reaches F_limiter2 (Space/CONVECT_MDCDHYB.F90:118-120, 175-177)
         const bool muscl = hyb && sensor >= R(p.F_limiter2);
-#pragma unroll
+#pragma unroll UNROLL
         for (int k = 0; k < 5; ++k) {
-            const int Q = qc[k];
+            const int Q = k < 3 ? S_PRIM + k : S_PP + (k - 3);
             R s6[6];
 #pragma unroll
             for (int o = 0; o < 6; ++o) s6[o] = q.v(Q, o - 3);
