@@ -468,7 +468,8 @@ def roofline(lib, c, kt, nsub, precision, sched):
         # path's two-plane launches): report the measured step against the floor of a dependent
         # launch chain of the same width (graph replay)
         pairs = sched.startswith("sweep=pairs")
-        roof["binding"] = "latency (one dependent step per " + ("two i+j+k hyperplanes" if pairs else "i+j+k hyperplane") + ")"
+        roof["binding"] = ("latency (one dependent step of every warp per i+j+k hyperplane)" if sched.startswith("sweep=march") else
+                           "latency (one dependent step per " + ("two i+j+k hyperplanes" if pairs else "i+j+k hyperplane") + ")")
         if sched.startswith("sweep=planes") or pairs:
             cells_per_plane = interior_cells(c) * nsub * 2 / dom_n      # dom_n counts both sweeps' launches
             # threads per launch: 8 per position in the FP64 path, 1 in the mixed path, 4 per

@@ -234,7 +234,7 @@ const char* trans_tuning(void* ctx) {
     const std::string tiles = c->sweep_mode == 3 ? std::to_string(c->tile_shape[0]) + "x" + std::to_string(c->tile_shape[1]) + "x"
                                                        + std::to_string(c->tile_shape[2]) + "/" : std::string();
     const std::string chain = c->pdl ? (c->pdl == 2 ? "-early" : "-chained") : "";
-    out = "sweep=" + std::string(c->sweep_mode == 5 ? "pairs" + chain
+    out = "sweep=" + std::string(c->sweep_mode == 6 ? std::string("march") : c->sweep_mode == 5 ? "pairs" + chain
                                  : c->sweep_mode >= 1 ? std::string(c->sweep_mode == 1 ? "coop " : c->sweep_mode == 2 ? "flow " : c->sweep_mode == 4 ? "clusters " : "tiles ")
                                                       + tiles + std::to_string(c->sweep_grid) + "x" + std::to_string(c->sweep_block)
                                  : c->sweep_mode == 0 ? (c->pdl ? (c->pdl == 2 ? "planes-early" : "planes-chained") : "planes") : "untuned")

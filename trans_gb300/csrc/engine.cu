@@ -188,7 +188,7 @@ int ctx_init(Ctx* c, int precision, long long budget) {
     // polls (for tests of the timeout path: a small n makes the waits run out)
     const char* sp = std::getenv("TRANS_SWEEP_SPIN");
     if (sp) c->spin_limit = (unsigned)std::max(0L, std::strtol(sp, nullptr, 10));
-    // sweep schedule: TRANS_SWEEP=planes | coop | flow | tiles | clusters | pairs forces one (for tests);
+    // sweep schedule: TRANS_SWEEP=planes | coop | flow | tiles | clusters | pairs | march forces one (for tests);
     // default: tuned
     const char* m = std::getenv("TRANS_SWEEP");
     std::string ms = m ? m : "";
@@ -199,6 +199,12 @@ int ctx_init(Ctx* c, int precision, long long budget) {
         c->sweep_mode = 4; c->sweep_grid = 8; c->sweep_block = 256;
         const char* pfs = std::getenv("TRANS_SWEEP_PF");
         c->sweep_pf = pfs ? std::max(0, std::atoi(pfs)) : 0;
+    }
+    // march: marching warps (mixed path; the FP64 path takes planes)
+    if (ms == "march" && !c->mixed) ms = "planes";
+    if (ms == "march") {
+        c->sweep_forced = true;
+        c->sweep_mode = 6;
     }
     // pairs: two hyperplanes per launch (mixed path; the FP64 path takes planes)
     if (ms == "pairs" && !c->mixed) ms = "planes";
@@ -232,6 +238,9 @@ void free_worklists(Ctx* c) {
     dfree(c->d_rmaps);
     dfree(c->d_bc); dfree(c->d_outlet); dfree(c->d_lines); dfree(c->d_sweep); dfree(c->d_plane_off); dfree(c->d_pb_off);
     dfree(c->d_nbp); dfree(c->d_flags); dfree(c->d_rec); dfree(c->d_dqs); dfree(c->d_dq2); dfree(c->d_orph); dfree(c->d_dq_save);
+    dfree(c->d_mtiles); dfree(c->d_medgeJ); dfree(c->d_medgeK); dfree(c->d_mctl);
+    c->n_mtiles = 0;
+    c->march = false;
     c->pair_lo.clear(); c->pair_up.clear(); dfree(c->d_parts); dfree(c->d_pc);
     dfree(c->d_cdev); dfree(c->d_stage); dfree(c->d_tile_first); dfree(c->d_norms);
     dfree(c->d_tiles); dfree(c->d_tflags); dfree(c->d_qpos); dfree(c->d_bc_first); dfree(c->d_intg);

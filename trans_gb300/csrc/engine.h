@@ -113,6 +113,13 @@ struct Ctx {
     struct SweepPair { int p_first, p_count, o_off, o_count; };
     std::vector<SweepPair> pair_lo, pair_up;
     int* d_orph = nullptr;
+    // marching warps (sweep_mode 6, mixed path, its default): the sweep arrays are stored in their order;
+    // tiles, edge buffers and counters
+    bool march = false;
+    MarchTile* d_mtiles = nullptr;
+    int n_mtiles = 0;
+    void *d_medgeJ = nullptr, *d_medgeK = nullptr;
+    MarchCtl* d_mctl = nullptr;
     double* d_pc = nullptr;              // PrecondDW coefficients of the sweep neighbours (IF_Precondition = 1)
     NormPart* d_parts = nullptr;
     std::vector<NormPart> h_parts;
@@ -139,8 +146,8 @@ struct Ctx {
     // 0 = one launch per hyperplane (graph), 1 = one cooperative launch with grid barriers,
     // 2 = dataflow over ready flags, 3 = tiled wavefront, 4 = one thread-block cluster per
     // block with cluster barriers between hyperplanes (mixed path; sweep_grid = CTAs per
-    // cluster), 5 = two hyperplanes per launch (mixed path, graph); -1 = pick the fastest on
-    // first use
+    // cluster), 5 = two hyperplanes per launch (mixed path, graph), 6 = marching warps (mixed path,
+    // where its arrays fit); -1 = pick the fastest of the others on first use
     // (all bit-identical)
     int sweep_mode = -1, sweep_grid = 0, sweep_block = 0;
     int tile_shape[3] = {0, 0, 0};       // tiles of the tiled wavefront (built for this shape)
@@ -173,6 +180,11 @@ struct Ctx {
 };
 
 int fail(Ctx* c, int code, const std::string& msg);
+// a sweep whose bounded wait gave up (the schedules that report there: the cooperative ones and the
+// marching warps)
+inline bool sweep_timed_out(const Ctx* c) {
+    return ((c->sweep_mode >= 1 && c->sweep_mode <= 3) || c->sweep_mode == 6) && c->h_sync->err;
+}
 const char* stateless_error();          // message of the last failed context-free call on this thread
 
 #define CK(call)                                                                                  \

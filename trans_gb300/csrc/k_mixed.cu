@@ -5,6 +5,7 @@
 #include "flux_inst.cuh"
 #include "kernels_mixed.cuh"
 #include "resid_tma.cuh"
+#include "sweep_march.cuh"
 
 namespace tg {
 cudaError_t prepare_resid_tma() {
@@ -58,6 +59,19 @@ void launch_resid_tma(int dir, cudaStream_t s, const DevBlock* blks, const Resid
     if (dir == 1) k_resid_tma<1><<<nt, 32 * RT_R1, rt_smem_bytes(1), s>>>(blks, tiles, cdev, m, err, limit);
     else if (dir == 2) k_resid_tma<2><<<nt, RT_FACES, rt_smem_bytes(2), s>>>(blks, tiles, cdev, m, err, limit);
     else k_resid_tma<3><<<nt, RT_FACES, rt_smem_bytes(3), s>>>(blks, tiles, cdev, m, err, limit);
+}
+template <int TURB>
+static void march(cudaStream_t s, const SweepView& v, const MarchTile* tiles, int ntiles, ulonglong2* bufJ, ulonglong2* bufK,
+                  MarchCtl* ctl, SweepSync* sy, unsigned limit) {
+    k_sweep_march<true, TURB><<<ntiles, 96, 0, s>>>(tiles, ntiles, (const float*)v.rec, (float*)v.dq, bufJ, bufK, ctl, sy, limit);
+    k_sweep_march<false, TURB><<<ntiles, 96, 0, s>>>(tiles, ntiles, (const float*)v.rec, (float*)v.dq, bufJ, bufK, ctl, sy, limit);
+}
+cudaError_t launch_sweep_march(cudaStream_t s, const SweepView& v, const MarchTile* tiles, int ntiles, void* bufJ, void* bufK,
+                               MarchCtl* ctl, SweepSync* sy, int turb, unsigned limit) {
+    if (ntiles <= 0) return cudaSuccess;
+    auto f = (turb & 3) == 0 ? march<0> : (turb & 3) == 1 ? march<1> : march<2>;
+    f(s, v, tiles, ntiles, (ulonglong2*)bufJ, (ulonglong2*)bufK, ctl, sy, limit);
+    return cudaGetLastError();
 }
 void launch_specrad_mixed(cudaStream_t s, const DevBlock* blks, const Tile* tiles, int nt, const CaseDev* cdev) {
     if (nt > 0) k_specrad_mixed<<<nt, CELL_TILE, 0, s>>>(blks, tiles, cdev);

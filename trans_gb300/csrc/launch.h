@@ -79,6 +79,12 @@ cudaError_t launch_sweep_cluster(cudaStream_t s, const SweepView& v, const int* 
                                  int pf);
 int sweep_cluster_fits(int cs, int bs);
 
+// the mixed path's sweeps as marching warps (k_mixed.cu, sweep_march.cuh): lower, then upper sweep
+struct MarchTile;
+struct MarchCtl;
+cudaError_t launch_sweep_march(cudaStream_t s, const SweepView& v, const MarchTile* tiles, int ntiles, void* bufJ,
+                               void* bufK, MarchCtl* ctl, SweepSync* sy, int turb, unsigned limit);
+
 // flux, source and sweep kernels, instantiated per arithmetic type
 struct FluxLaunchers {
     void (*gradient)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*);

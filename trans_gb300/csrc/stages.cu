@@ -294,6 +294,16 @@ int sweep_once(Ctx* c, int mode, int grid, int block, bool capture = false) {
         c->launches++;
         return TRANS_OK;
     }
+    if (mode == 6) {
+        if (!c->march) return fail(c, TRANS_E_ARG, "marching sweeps are a mixed-path schedule");
+        // (graph replays keep the flag cleared here or by the run that reported it)
+        if (!capture) CK(cudaMemsetAsync(c->d_sync, 0, sizeof(SweepSync), s));
+        CK(launch_sweep_march(s, c->sv, c->d_mtiles, c->n_mtiles, c->d_medgeJ, c->d_medgeK, c->d_mctl, c->d_sync,
+                              c->sweep_lanes, c->spin_limit));
+        if (!capture) CK(cudaMemcpyAsync(c->h_sync, c->d_sync, sizeof(SweepSync), cudaMemcpyDeviceToHost, s));
+        c->launches += 2;
+        return TRANS_OK;
+    }
     if (mode == 4) {
         CK(launch_sweep_cluster(s, c->sv, c->d_pb_off, nh, (int)c->blk.size(), c->sweep_lanes, grid, block, c->sweep_pf));
         c->launches++;
@@ -657,7 +667,7 @@ int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot) {
                 } else {
                     for (int h = 0; h < nh; ++h) nl += (c->plane_off[h + 1] > c->plane_off[h]) ? 2 : 0;
                 }
-                KScope t(c, K_SWEEP, (c->sweep_mode >= 1 && c->sweep_mode != 5) ? 1 : nl);
+                KScope t(c, K_SWEEP, c->sweep_mode == 6 ? 2 : (c->sweep_mode >= 1 && c->sweep_mode != 5) ? 1 : nl);
                 if (capture) rc = sweep_once(c, c->sweep_mode, c->sweep_grid, c->sweep_block, true);
                 else rc = run_sweeps(c);
                 if (rc) return rc;
@@ -681,7 +691,7 @@ int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot) {
             CK(cudaMemcpyAsync(c->h_norms, c->d_norms, sizeof(BlockNorms) * nblk, cudaMemcpyDeviceToHost, s));
             CK(cudaMemcpyAsync(c->h_kerr, c->d_kerr, sizeof(int), cudaMemcpyDeviceToHost, s));
             CK(cudaStreamSynchronize(s));
-            if (c->sweep_mode >= 1 && c->sweep_mode <= 3 && c->h_sync->err) return fail(c, TRANS_E_TIMEOUT, "LU-SGS sweep wait timed out");
+            if (sweep_timed_out(c)) return fail(c, TRANS_E_TIMEOUT, "LU-SGS sweep wait timed out");
             if (*c->h_kerr) return fail(c, TRANS_E_TIMEOUT, "residual tile staging wait timed out");
             if ((rc = collect_norms(c, c->h_norms))) return rc;
             break;
@@ -835,7 +845,10 @@ int run_iterations(Ctx* c, int n) {
         }
         for (int q = 1; q < m; ++q) advance();  // KI of the last replayed iteration
         done += m;
-        if (c->sweep_mode >= 1 && c->sweep_mode <= 3 && c->h_sync->err) return fail(c, TRANS_E_TIMEOUT, "LU-SGS sweep wait timed out");
+        if (sweep_timed_out(c)) {
+            CK(cudaMemsetAsync(c->d_sync, 0, sizeof(SweepSync), c->stream));
+            return fail(c, TRANS_E_TIMEOUT, "LU-SGS sweep wait timed out");
+        }
         if (*c->h_kerr) return fail(c, TRANS_E_TIMEOUT, "residual tile staging wait timed out");
         if (nan) return fail(c, TRANS_E_NAN, "NaN in the density increment");
     }

@@ -218,6 +218,79 @@ bool build_resid_tma(Ctx* c) {
     return prepare_resid_tma() == cudaSuccess;
 }
 
+// The marching sweeps' tiles (MarchTile, types.cuh), in an order in which a tile's j- and k-neighbours on
+// the lower side come first (by tile diagonal, then block), and the sweep arrays stored in their
+// order.  Leaves c->march false where the places are beyond int indexes or the edge buffers do not
+// fit: the context then keeps the hyperplane order and its schedules.
+int build_march(Ctx* c) {
+    const int nblk = (int)c->blk.size();
+    std::vector<int> ntj(nblk), ntk(nblk);
+    struct Key { int d, n, tj, tk; };
+    std::vector<Key> keys;
+    for (int n = 0; n < nblk; ++n) {
+        ntj[n] = (c->blk[n].NJ1 + MARCH_J - 1) / MARCH_J;
+        ntk[n] = (c->blk[n].NK1 + MARCH_K - 1) / MARCH_K;
+        for (int tk = 0; tk < ntk[n]; ++tk)
+            for (int tj = 0; tj < ntj[n]; ++tj) keys.push_back(Key{tj + tk, n, tj, tk});
+    }
+    std::stable_sort(keys.begin(), keys.end(), [](const Key& a, const Key& b) { return a.d < b.d; });
+    std::vector<std::vector<int>> first(nblk);         // first step of tile (tj, tk)
+    for (int n = 0; n < nblk; ++n) first[n].assign((size_t)ntj[n] * ntk[n], -1);
+    long long s0 = 0;
+    for (const Key& k : keys) {
+        first[k.n][k.tj + (size_t)ntj[k.n] * k.tk] = (int)s0;
+        s0 += c->blk[k.n].NI1 + MARCH_J + MARCH_K - 2;
+        if (s0 > 0x7fffffffLL / 32) return TRANS_OK;
+    }
+    std::vector<MarchTile> tiles;
+    for (const Key& k : keys) {
+        const DevBlock& b = c->blk[k.n];
+        auto at = [&](int tj, int tk) {
+            return tj < 0 || tk < 0 || tj >= ntj[k.n] || tk >= ntk[k.n] ? -1 : first[k.n][tj + (size_t)ntj[k.n] * tk];
+        };
+        tiles.push_back(MarchTile{b.NI1, std::min(MARCH_J, b.NJ1 - k.tj * MARCH_J), std::min(MARCH_K, b.NK1 - k.tk * MARCH_K),
+                                  at(k.tj, k.tk), {at(k.tj - 1, k.tk), at(k.tj + 1, k.tk)}, {at(k.tj, k.tk - 1), at(k.tj, k.tk + 1)}});
+    }
+    const size_t word = 4 * sizeof(ulonglong2);        // 8 floats, each with its tag
+    const size_t nj = (size_t)s0 * MARCH_K * word, nk = (size_t)s0 * MARCH_J * word, places = (size_t)s0 * 32;
+    const size_t nrec = places * NCREC * sizeof(float), ndq = places * DQ_STRIDE * sizeof(float);
+    auto room = [](void* p, size_t bytes) { return cudaMalloc((void**)p, bytes) == cudaSuccess; };
+    if (!room(&c->d_medgeJ, nj) || !room(&c->d_medgeK, nk) || !room(&c->d_rec, nrec) || !room(&c->d_dqs, ndq)) {
+        cudaGetLastError();
+        for (void** p : {&c->d_medgeJ, &c->d_medgeK, &c->d_rec, &c->d_dqs}) {
+            if (*p) cudaFree(*p);
+            *p = nullptr;
+        }
+        return TRANS_OK;
+    }
+    int rc;
+    if ((rc = upload_vec(c, tiles.data(), sizeof(MarchTile) * tiles.size(), (void**)&c->d_mtiles))) return rc;
+    c->n_mtiles = (int)tiles.size();
+    CK(cudaMalloc(&c->d_mctl, sizeof(MarchCtl)));
+    CK(cudaMemsetAsync(c->d_medgeJ, 0, nj, c->stream));         // tag 0 is never used
+    CK(cudaMemsetAsync(c->d_medgeK, 0, nk, c->stream));
+    CK(cudaMemsetAsync(c->d_rec, 0, nrec, c->stream));          // the places outside the blocks stay finite
+    CK(cudaMemsetAsync(c->d_dqs, 0, ndq, c->stream));
+    CK(cudaMemsetAsync(c->d_mctl, 0, sizeof(MarchCtl), c->stream));
+    CK(cudaMemsetAsync(c->d_sync, 0, sizeof(SweepSync), c->stream));
+    std::vector<int> qpos(c->cell_tiles.size() * (size_t)CELL_TILE, -1);
+    for (size_t t = 0; t < c->cell_tiles.size(); ++t) {
+        const Tile& tl = c->cell_tiles[t];
+        const DevBlock& b = c->blk[tl.blk];
+        for (int r = 0; r < tl.count; ++r) {
+            const int n = tl.start + r, i = n % b.NI1, j = (n / b.NI1) % b.NJ1, k = n / (b.NI1 * b.NJ1);
+            const int a = j % MARCH_J, bb = k % MARCH_K;
+            const int step = first[tl.blk][j / MARCH_J + (size_t)ntj[tl.blk] * (k / MARCH_K)] + i + a + bb;
+            qpos[t * CELL_TILE + r] = step * 32 + bb * MARCH_J + a;
+        }
+    }
+    if ((rc = upload_vec(c, qpos.data(), sizeof(int) * qpos.size(), (void**)&c->d_qpos))) return rc;
+    c->sv = SweepView{};
+    c->sv.rec = c->d_rec; c->sv.dq = c->d_dqs; c->sv.n = (long long)places;
+    c->march = true;
+    return TRANS_OK;
+}
+
 }  // namespace
 
 int rebuild(Ctx* c) {
@@ -278,91 +351,96 @@ int rebuild(Ctx* c) {
     if ((rc = upload_vec(c, c->bc.data(), sizeof(BCEntry) * c->bc.size(), (void**)&c->d_bc))) return rc;
     if ((rc = upload_vec(c, c->outlet.data(), sizeof(BCEntry) * c->outlet.size(), (void**)&c->d_outlet))) return rc;
     if ((rc = upload_vec(c, c->lines.data(), sizeof(OutletLine) * c->lines.size(), (void**)&c->d_lines))) return rc;
-    // hyperplane order of the LU-SGS sweeps over all blocks of all cases: h = i+j+k = 3 ..
-    int hmax = 3;
-    for (auto& b : c->blk) hmax = std::max(hmax, b.NI1 + b.NJ1 + b.NK1);
-    c->plane_off.assign(1, 0);
-    std::vector<int> pb_off;
-    for (int h = 3; h <= hmax; ++h) {
-        for (int n = 0; n < nblk; ++n) {
-            const DevBlock& b = c->blk[n];
+    c->march = false;
+    if (c->mixed && (!c->sweep_forced || c->sweep_mode == 6) && (rc = build_march(c))) return rc;
+    if (c->sweep_forced && c->sweep_mode == 6 && !c->march) return fail(c, TRANS_E_ARG, "the marching sweeps do not fit");
+    if (!c->march) {
+        // hyperplane order of the LU-SGS sweeps over all blocks of all cases: h = i+j+k = 3 ..
+        int hmax = 3;
+        for (auto& b : c->blk) hmax = std::max(hmax, b.NI1 + b.NJ1 + b.NK1);
+        c->plane_off.assign(1, 0);
+        std::vector<int> pb_off;
+        for (int h = 3; h <= hmax; ++h) {
+            for (int n = 0; n < nblk; ++n) {
+                const DevBlock& b = c->blk[n];
+                pb_off.push_back((int)c->sweep.size());
+                for (int k = 1; k <= b.NK1; ++k)
+                    for (int j = 1; j <= b.NJ1; ++j) {
+                        int i = h - j - k;
+                        if (i >= 1 && i <= b.NI1) c->sweep.push_back(SweepCell{n, i, j, k});
+                    }
+            }
             pb_off.push_back((int)c->sweep.size());
-            for (int k = 1; k <= b.NK1; ++k)
-                for (int j = 1; j <= b.NJ1; ++j) {
-                    int i = h - j - k;
-                    if (i >= 1 && i <= b.NI1) c->sweep.push_back(SweepCell{n, i, j, k});
-                }
+            c->plane_off.push_back((int)c->sweep.size());
         }
-        pb_off.push_back((int)c->sweep.size());
-        c->plane_off.push_back((int)c->sweep.size());
-    }
-    if ((rc = upload_vec(c, pb_off.data(), sizeof(int) * pb_off.size(), (void**)&c->d_pb_off))) return rc;
-    if ((rc = upload_vec(c, c->sweep.data(), sizeof(SweepCell) * c->sweep.size(), (void**)&c->d_sweep))) return rc;
-    if ((rc = upload_vec(c, c->plane_off.data(), sizeof(int) * c->plane_off.size(), (void**)&c->d_plane_off))) return rc;
-    {   // neighbour positions in sweep order: lower i,j,k (0..2) and upper (3..5), -1 = none
-        const long long N = (long long)c->sweep.size();
-        const long long Np = (N + 31) / 32 * 32;
-        std::vector<std::vector<int>> pos(nblk);
-        for (int n = 0; n < nblk; ++n) pos[n].assign((size_t)c->blk[n].nint, -1);
-        for (long long q = 0; q < N; ++q) {
-            const SweepCell& sc = c->sweep[q];
-            const DevBlock& b = c->blk[sc.blk];
-            pos[sc.blk][(size_t)(sc.i - 1) + (size_t)b.NI1 * ((sc.j - 1) + (size_t)b.NJ1 * (sc.k - 1))] = (int)q;
-        }
-        std::vector<int> nbp((size_t)6 * Np, -1);
-        for (long long q = 0; q < N; ++q) {
-            const SweepCell& sc = c->sweep[q];
-            const DevBlock& b = c->blk[sc.blk];
-            const int ijk[3] = {sc.i, sc.j, sc.k}, hi[3] = {b.NI1, b.NJ1, b.NK1};
-            for (int side = 0; side < 2; ++side)
-                for (int d = 0; d < 3; ++d) {
-                    int x[3] = {ijk[0], ijk[1], ijk[2]};
-                    x[d] += side == 0 ? -1 : 1;
-                    if (x[d] < 1 || x[d] > hi[d]) continue;
-                    nbp[sw_at(q, 3 * side + d, 6)] =
-                        pos[sc.blk][(size_t)(x[0] - 1) + (size_t)b.NI1 * ((x[1] - 1) + (size_t)b.NJ1 * (x[2] - 1))];
-                }
-        }
-        if ((rc = upload_vec(c, nbp.data(), sizeof(int) * nbp.size(), (void**)&c->d_nbp))) return rc;
-        // sweep position of every slot of every cell tile (tiles hold consecutive interior cells)
-        std::vector<int> qpos(c->cell_tiles.size() * (size_t)CELL_TILE, -1);
-        for (size_t t = 0; t < c->cell_tiles.size(); ++t) {
-            const Tile& tl = c->cell_tiles[t];
-            for (int r = 0; r < tl.count; ++r) qpos[t * CELL_TILE + r] = pos[tl.blk][(size_t)tl.start + r];
-        }
-        if ((rc = upload_vec(c, qpos.data(), sizeof(int) * qpos.size(), (void**)&c->d_qpos))) return rc;
-        CK(cudaMalloc(&c->d_rec, (size_t)c->fl->rec_width * Np * c->fl->elem));
-        CK(cudaMalloc(&c->d_dqs, (size_t)DQ_STRIDE * Np * c->fl->elem));
-        if (c->fl->sweep_pair) {
-            // two-plane schedule: the second DeltaQ array, and per launch the first plane's
-            // positions that no neighbour on the second plane computes (block corners)
-            CK(cudaMalloc(&c->d_dq2, (size_t)DQ_STRIDE * Np * c->fl->elem));
-            const int nh = (int)c->plane_off.size() - 1;
-            std::vector<int> orph;
-            auto add = [&](std::vector<Ctx::SweepPair>& out, int h, int h1, int side) {
-                Ctx::SweepPair sp{0, 0, (int)orph.size(), 0};
-                if (h1 >= 0 && h1 < nh) { sp.p_first = c->plane_off[h1]; sp.p_count = c->plane_off[h1 + 1] - c->plane_off[h1]; }
-                for (int q = c->plane_off[h]; q < c->plane_off[h + 1]; ++q) {
-                    bool reached = false;
-                    for (int d = 0; d < 3; ++d) reached |= nbp[sw_at(q, side + d, 6)] >= 0;
-                    if (!reached || sp.p_count == 0) orph.push_back(q);
-                }
-                sp.o_count = (int)orph.size() - sp.o_off;
-                out.push_back(sp);
-            };
-            c->pair_lo.clear();
-            c->pair_up.clear();
-            for (int h = 0; h < nh; h += 2) add(c->pair_lo, h, h + 1, 3);        // reached from its upper neighbours
-            for (int h = nh - 1; h >= 0; h -= 2) add(c->pair_up, h, h - 1, 0);   // from its lower neighbours
-            if (orph.empty()) orph.push_back(0);
-            if ((rc = upload_vec(c, orph.data(), sizeof(int) * orph.size(), (void**)&c->d_orph))) return rc;
-        }
-        CK(cudaMalloc(&c->d_flags, (size_t)2 * Np * sizeof(int)));
-        c->sv.cells = c->d_sweep; c->sv.nbp = c->d_nbp; c->sv.rec = c->d_rec; c->sv.dq = c->d_dqs; c->sv.n = N;
-        c->sv.pc = nullptr;
-        if (c->cases[0]->p.IF_Precondition == 1) {      // the neighbours' PrecondDW coefficients (FP64 path)
-            CK(cudaMalloc(&c->d_pc, (size_t)6 * NPC * Np * sizeof(double)));
-            c->sv.pc = c->d_pc;
+        if ((rc = upload_vec(c, pb_off.data(), sizeof(int) * pb_off.size(), (void**)&c->d_pb_off))) return rc;
+        if ((rc = upload_vec(c, c->sweep.data(), sizeof(SweepCell) * c->sweep.size(), (void**)&c->d_sweep))) return rc;
+        if ((rc = upload_vec(c, c->plane_off.data(), sizeof(int) * c->plane_off.size(), (void**)&c->d_plane_off))) return rc;
+        {   // neighbour positions in sweep order: lower i,j,k (0..2) and upper (3..5), -1 = none
+            const long long N = (long long)c->sweep.size();
+            const long long Np = (N + 31) / 32 * 32;
+            std::vector<std::vector<int>> pos(nblk);
+            for (int n = 0; n < nblk; ++n) pos[n].assign((size_t)c->blk[n].nint, -1);
+            for (long long q = 0; q < N; ++q) {
+                const SweepCell& sc = c->sweep[q];
+                const DevBlock& b = c->blk[sc.blk];
+                pos[sc.blk][(size_t)(sc.i - 1) + (size_t)b.NI1 * ((sc.j - 1) + (size_t)b.NJ1 * (sc.k - 1))] = (int)q;
+            }
+            std::vector<int> nbp((size_t)6 * Np, -1);
+            for (long long q = 0; q < N; ++q) {
+                const SweepCell& sc = c->sweep[q];
+                const DevBlock& b = c->blk[sc.blk];
+                const int ijk[3] = {sc.i, sc.j, sc.k}, hi[3] = {b.NI1, b.NJ1, b.NK1};
+                for (int side = 0; side < 2; ++side)
+                    for (int d = 0; d < 3; ++d) {
+                        int x[3] = {ijk[0], ijk[1], ijk[2]};
+                        x[d] += side == 0 ? -1 : 1;
+                        if (x[d] < 1 || x[d] > hi[d]) continue;
+                        nbp[sw_at(q, 3 * side + d, 6)] =
+                            pos[sc.blk][(size_t)(x[0] - 1) + (size_t)b.NI1 * ((x[1] - 1) + (size_t)b.NJ1 * (x[2] - 1))];
+                    }
+            }
+            if ((rc = upload_vec(c, nbp.data(), sizeof(int) * nbp.size(), (void**)&c->d_nbp))) return rc;
+            // sweep position of every slot of every cell tile (tiles hold consecutive interior cells)
+            std::vector<int> qpos(c->cell_tiles.size() * (size_t)CELL_TILE, -1);
+            for (size_t t = 0; t < c->cell_tiles.size(); ++t) {
+                const Tile& tl = c->cell_tiles[t];
+                for (int r = 0; r < tl.count; ++r) qpos[t * CELL_TILE + r] = pos[tl.blk][(size_t)tl.start + r];
+            }
+            if ((rc = upload_vec(c, qpos.data(), sizeof(int) * qpos.size(), (void**)&c->d_qpos))) return rc;
+            CK(cudaMalloc(&c->d_rec, (size_t)c->fl->rec_width * Np * c->fl->elem));
+            CK(cudaMalloc(&c->d_dqs, (size_t)DQ_STRIDE * Np * c->fl->elem));
+            if (c->fl->sweep_pair) {
+                // two-plane schedule: the second DeltaQ array, and per launch the first plane's
+                // positions that no neighbour on the second plane computes (block corners)
+                CK(cudaMalloc(&c->d_dq2, (size_t)DQ_STRIDE * Np * c->fl->elem));
+                const int nh = (int)c->plane_off.size() - 1;
+                std::vector<int> orph;
+                auto add = [&](std::vector<Ctx::SweepPair>& out, int h, int h1, int side) {
+                    Ctx::SweepPair sp{0, 0, (int)orph.size(), 0};
+                    if (h1 >= 0 && h1 < nh) { sp.p_first = c->plane_off[h1]; sp.p_count = c->plane_off[h1 + 1] - c->plane_off[h1]; }
+                    for (int q = c->plane_off[h]; q < c->plane_off[h + 1]; ++q) {
+                        bool reached = false;
+                        for (int d = 0; d < 3; ++d) reached |= nbp[sw_at(q, side + d, 6)] >= 0;
+                        if (!reached || sp.p_count == 0) orph.push_back(q);
+                    }
+                    sp.o_count = (int)orph.size() - sp.o_off;
+                    out.push_back(sp);
+                };
+                c->pair_lo.clear();
+                c->pair_up.clear();
+                for (int h = 0; h < nh; h += 2) add(c->pair_lo, h, h + 1, 3);        // reached from its upper neighbours
+                for (int h = nh - 1; h >= 0; h -= 2) add(c->pair_up, h, h - 1, 0);   // from its lower neighbours
+                if (orph.empty()) orph.push_back(0);
+                if ((rc = upload_vec(c, orph.data(), sizeof(int) * orph.size(), (void**)&c->d_orph))) return rc;
+            }
+            CK(cudaMalloc(&c->d_flags, (size_t)2 * Np * sizeof(int)));
+            c->sv.cells = c->d_sweep; c->sv.nbp = c->d_nbp; c->sv.rec = c->d_rec; c->sv.dq = c->d_dqs; c->sv.n = N;
+            c->sv.pc = nullptr;
+            if (c->cases[0]->p.IF_Precondition == 1) {      // the neighbours' PrecondDW coefficients (FP64 path)
+                CK(cudaMalloc(&c->d_pc, (size_t)6 * NPC * Np * sizeof(double)));
+                c->sv.pc = c->d_pc;
+            }
         }
     }
     {   // staging buffer for the largest Fortran field (DQdxyz: 18 components, lower bound -1)
@@ -388,7 +466,8 @@ int rebuild(Ctx* c) {
     // it was tuned (a serving loop adds and removes cases every few iterations, and a tuning run
     // times ~40 candidate sweeps); the schedule kept is re-captured for the new work lists
     const long long npos = (long long)c->sweep.size();
-    if (!c->sweep_forced && (c->tuned_positions <= 0 || npos > 2 * c->tuned_positions || 2 * npos < c->tuned_positions))
+    if (c->march) c->sweep_mode = 6;
+    else if (!c->sweep_forced && (c->sweep_mode == 6 || c->tuned_positions <= 0 || npos > 2 * c->tuned_positions || 2 * npos < c->tuned_positions))
         c->sweep_mode = -1;
     c->built = true;
     return TRANS_OK;
