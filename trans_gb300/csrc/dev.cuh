@@ -106,8 +106,8 @@ struct MirrorList {       // slot ranges [first, first+count) copied FP64 -> FP3
     int n, to_fp64, first[6], count[6];
 };
 
-struct Tile {             // a run of consecutive interior cells (or faces) of one block
-    int blk, start, count, pad_;
+struct Tile {             // a run of consecutive interior cells (or faces of direction dir, 1..3) of one block
+    int blk, start, count, dir;
 };
 
 // one page-locked Fortran-layout array of a field transfer and its slots (k_fields_xfer)

@@ -234,7 +234,8 @@ int ctx_init(Ctx* c, int precision, long long budget) {
 
 void free_worklists(Ctx* c) {
     dfree(c->d_blk); dfree(c->d_off); dfree(c->d_cell); dfree(c->d_ghost);
-    for (int d = 0; d < 3; ++d) { dfree(c->d_face[d]); dfree(c->d_rtiles[d]); c->n_rtiles[d] = 0; }
+    dfree(c->d_face);
+    for (int d = 0; d < 3; ++d) { dfree(c->d_rtiles[d]); c->n_rtiles[d] = 0; }
     dfree(c->d_rmaps);
     dfree(c->d_bc); dfree(c->d_outlet); dfree(c->d_lines); dfree(c->d_sweep); dfree(c->d_plane_off); dfree(c->d_pb_off);
     dfree(c->d_nbp); dfree(c->d_flags); dfree(c->d_rec); dfree(c->d_dqs); dfree(c->d_dq2); dfree(c->d_orph); dfree(c->d_dq_save);

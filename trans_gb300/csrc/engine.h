@@ -67,8 +67,8 @@ struct Ctx {
     DevBlock* d_blk = nullptr;
     long long* d_off = nullptr;          // padded-cell offsets of the blocks (for flat kernels)
     long long total_cells = 0;
-    std::vector<Tile> cell_tiles, face_tiles[3], ghost_tiles;
-    Tile *d_cell = nullptr, *d_face[3] = {nullptr, nullptr, nullptr}, *d_ghost = nullptr;
+    std::vector<Tile> cell_tiles, face_tiles, ghost_tiles;      // face tiles: of the three directions in turn
+    Tile *d_cell = nullptr, *d_face = nullptr, *d_ghost = nullptr;
     std::vector<int> cell_tile_blk;      // block of each cell tile (norm reduction)
     // mixed path: the residual from TMA-staged tiles (one tile list per face direction, NRMAP
     // tensor maps per block over its FP32 slots) when 1; 0 (the default) uses k_face_flux +

@@ -16,12 +16,11 @@ void shg(cudaStream_t s, const DevBlock* b, const Tile* t, int nt) {
 void bcg(cudaStream_t s, const DevBlock* b, const BCEntry* e, int n) {
     if (n > 0) k_bc_grad<TG_R><<<(n + 127) / 128, 128, 0, s>>>(b, e, n);
 }
-template <int DIR>
 void ff(cudaStream_t s, const DevBlock* b, const Tile* t, int nt, const CaseDev* cd) {
     if (nt <= 0) return;
     // viscous, then convective fluxes (two register budgets)
-    k_face_flux<TG_R, DIR, 1><<<nt, FACE_TILE, 0, s>>>(b, t, cd);
-    k_face_flux<TG_R, DIR, 2><<<nt, FACE_TILE, 0, s>>>(b, t, cd);
+    k_face_flux<TG_R, 1><<<nt, FACE_TILE, 0, s>>>(b, t, cd);
+    k_face_flux<TG_R, 2><<<nt, FACE_TILE, 0, s>>>(b, t, cd);
 }
 void ga(cudaStream_t s, const DevBlock* b, const Tile* t, int nt, const CaseDev* cd) {
     if (nt > 0) k_gather<TG_R><<<nt, CELL_TILE, 0, s>>>(b, t, cd);
@@ -174,7 +173,7 @@ void scat(cudaStream_t s, const DevBlock* b, const Tile* tiles, int nt, const in
 }  // namespace
 
 const FluxLaunchers& TG_NAME() {
-    static const FluxLaunchers L = {grd, shg, bcg, {ff<1>, ff<2>, ff<3>}, ga, fc, hu, prep, jac, swl, swu, swa, swa_occ, swf, swf_occ,
+    static const FluxLaunchers L = {grd, shg, bcg, ff, ga, fc, hu, prep, jac, swl, swu, swa, swa_occ, swf, swf_occ,
                                     swt, swt_occ, scat, sizeof(TG_R) == 4 ? swpair : nullptr, sizeof(TG_R),
                                     sizeof(TG_R) == 4 ? (int)NCREC : (int)NREC};
     return L;

@@ -671,10 +671,10 @@ struct FaceGlobal {
 };
 
 // PART 0: every flux; 1: the viscous and k-omega diffusion fluxes only; 2: the convective ones
-template <typename R, int DIR, int PART = 0, class A>
-__device__ __forceinline__ void face_flux_body(const ParamsT<R>& p, int turb, const A& q, R* F) {
-    constexpr int d = DIR - 1;
-    constexpr int AL = S_ALAGM + d, AIN = S_AINV + d, SDD = S_SD + 3 * d;
+template <typename R, int PART = 0, class A>
+__device__ __forceinline__ void face_flux_body(const int DIR, const ParamsT<R>& p, int turb, const A& q, R* F) {
+    const int d = DIR - 1;
+    const int AL = S_ALAGM + d, AIN = S_AINV + d, SDD = S_SD + 3 * d;
     // face average of a slot at the face o steps from this one (SPACEINTERP_GetSurfCenterVars)
     auto fa = [&](int slot, int o) { return (q.v(AL, o) * q.v(slot, o - 1) + q.v(AL, o - 1) * q.v(slot, o)) * q.v(AIN, o); };
     if constexpr (PART != 2) {
@@ -920,12 +920,17 @@ __device__ __forceinline__ void face_flux_body(const ParamsT<R>& p, int turb, co
 // FX words, so that each gets its own register budget (the same arithmetic, so the FP64
 // fluxes stay bit-identical): as one kernel the FP32 fluxes needed 96 registers (five CTAs per
 // SM) and were issue-latency bound, split 80 and 64 (six and eight); the FP64 ones 250 (two),
-// split at most 168 and 142 (three each)
-template <typename R, int DIR, int PART = 0>
+// split at most 168 and 142 (three each).  A launch covers the faces of all three directions (the
+// tile's): a launch per direction ended in a partly filled wave three times, and a small block's
+// three launches ran one after the other (us per iteration, three launches -> one of each part:
+// 1,920-cell channel FP64 257 -> 86, 352,256-cell cascade FP64 3,019 -> 2,884 and mixed 132 -> 97,
+// 1,966,080-cell cascade FP64 15,670 -> 15,617 and mixed 629 -> 617)
+template <typename R, int PART = 0>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (PART == 1 ? TG_FACE_MINB_VISC : TG_FACE_MINB) : (PART == 0 ? 1 : 3)) k_face_flux(const DevBlock* __restrict__ blks, const Tile* __restrict__ tiles,
                                                           const CaseDev* __restrict__ cdev) {
     const Tile t = tiles[blockIdx.x];
     if ((int)threadIdx.x >= t.count) return;
+    const int DIR = t.dir;
     const DevBlock b = blks[t.blk];
     const ParamsT<R> p = cparams<R>(cdev[b.cs]);
     const int turb = cdev[b.cs].turb;
@@ -936,7 +941,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (PART == 1 ? TG_FACE_MIN
     const int c = cidx(b, i, j, k);
     const FaceGlobal<R> q{b, c, s};
     R F[NFX];
-    face_flux_body<R, DIR, PART>(p, turb, q, F);
+    face_flux_body<R, PART>(DIR, p, turb, q, F);
     const size_t nc = (size_t)b.ncell;
     R* FX = rs<R>(b, S_FX + NFX * (DIR - 1));
     if constexpr (PART != 2) {

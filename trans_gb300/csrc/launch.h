@@ -90,7 +90,7 @@ struct FluxLaunchers {
     void (*gradient)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*);
     void (*shock_ghost)(cudaStream_t, const DevBlock*, const Tile*, int);
     void (*bc_grad)(cudaStream_t, const DevBlock*, const BCEntry*, int);
-    void (*face_flux[3])(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*);
+    void (*face_flux)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*);
     void (*gather)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*);
     void (*sst_fc1)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*);
     // cross-rank 1-to-1 segment: words (host-built table, device staging) into the ghost layers

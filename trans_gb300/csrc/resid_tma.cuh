@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(DIR == 1 ? 32 * RT_R1 : RT_FACES, 2)
         for (int m = 0; m < NFX; ++m) F[m] = 0.f;
         if (l <= RT_X1 && ia >= 3 && ia <= b.NI + 2 && ja <= b.NJ + 1 && ka <= b.NK + 1) {
             const FaceTile<DIR> q{sm, b, c, 1, r * RT_W1 + l + 4};
-            face_flux_body<float, DIR>(p, turb, q, F);
+            face_flux_body<float>(DIR, p, turb, q, F);
         }
         float Fp[NFX];          // the plus-side face of this lane's cell: the next lane's face
 #pragma unroll
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(DIR == 1 ? 32 * RT_R1 : RT_FACES, 2)
 #pragma unroll
             for (int m = 0; m < NFX; ++m) F[m] = 0.f;
             const FaceTile<DIR> q{sm, b, c, s, x + RT_X * f};
-            face_flux_body<float, DIR>(p, turb, q, F);
+            face_flux_body<float>(DIR, p, turb, q, F);
 #pragma unroll
             for (int m = 0; m < NFX; ++m) Fb[m * RT_FACES + tid] = F[m];
         }

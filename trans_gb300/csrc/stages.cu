@@ -528,7 +528,7 @@ int tune_resid(Ctx* c) {
                 launch_resid_tma(d + 1, s, c->d_blk, c->d_rtiles[d], c->n_rtiles[d], c->d_cdev, c->d_rmaps, c->d_kerr,
                                  c->resid_spin);
         } else {
-            for (int d = 0; d < 3; ++d) c->fl->face_flux[d](s, c->d_blk, c->d_face[d], (int)c->face_tiles[d].size(), c->d_cdev);
+            c->fl->face_flux(s, c->d_blk, c->d_face, (int)c->face_tiles.size(), c->d_cdev);
             c->fl->gather(s, c->d_blk, c->d_cell, nct, c->d_cdev);
         }
     };
@@ -631,13 +631,13 @@ int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot) {
                 c->launches += 3;
                 break;
             }
-            for (int d = 0; d < 3; ++d) {
-                // the viscous and the convective fluxes of a direction are two launches
+            {
+                // the viscous and the convective fluxes of every direction are a launch each
                 KScope t(c, K_FACE, 2);
-                c->fl->face_flux[d](s, c->d_blk, c->d_face[d], (int)c->face_tiles[d].size(), c->d_cdev);
+                c->fl->face_flux(s, c->d_blk, c->d_face, (int)c->face_tiles.size(), c->d_cdev);
             }
             { KScope t(c, K_GATHER); c->fl->gather(s, c->d_blk, c->d_cell, nct, c->d_cdev); }
-            c->launches += 7;
+            c->launches += 3;
             break;
         case TRANS_STAGE_LUSGS: {
             if (!capture && (rc = upload_cdev(c))) return rc;

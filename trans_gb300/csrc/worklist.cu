@@ -142,11 +142,11 @@ int build_bc(Ctx* c, const CaseRec* cs) {
     return TRANS_OK;
 }
 
-void make_tiles(int nblk, const std::vector<long long>& counts, int tile, std::vector<Tile>& out, std::vector<int>* owner) {
+void make_tiles(int nblk, const std::vector<long long>& counts, int tile, std::vector<Tile>& out, std::vector<int>* owner, int dir = 0) {
     for (int b = 0; b < nblk; ++b)
         for (long long s = 0; s < counts[b]; s += tile) {
             Tile t;
-            t.blk = b; t.start = (int)s; t.count = (int)std::min<long long>(tile, counts[b] - s); t.pad_ = 0;
+            t.blk = b; t.start = (int)s; t.count = (int)std::min<long long>(tile, counts[b] - s); t.dir = dir;
             out.push_back(t);
             if (owner) owner->push_back(b);
         }
@@ -297,7 +297,7 @@ int rebuild(Ctx* c) {
     CK(cudaStreamSynchronize(c->stream));
     free_worklists(c);
     c->blk.clear(); c->cell_tiles.clear(); c->cell_tile_blk.clear(); c->ghost_tiles.clear();
-    for (int d = 0; d < 3; ++d) c->face_tiles[d].clear();
+    c->face_tiles.clear();
     c->bc.clear(); c->bc_first.clear(); c->outlet.clear(); c->lines.clear(); c->sweep.clear(); c->plane_off.clear();
     c->cdev_last.clear();
     if (c->cases.empty()) return TRANS_OK;
@@ -332,11 +332,10 @@ int rebuild(Ctx* c) {
         gcnt[n] = 6LL * ((long long)b.NJ1 * b.NK1 + (long long)b.NI1 * b.NK1 + (long long)b.NI1 * b.NJ1);
     }
     make_tiles(nblk, cnt, CELL_TILE, c->cell_tiles, &c->cell_tile_blk);
-    for (int d = 0; d < 3; ++d) make_tiles(nblk, fcnt[d], FACE_TILE, c->face_tiles[d], nullptr);
+    for (int d = 0; d < 3; ++d) make_tiles(nblk, fcnt[d], FACE_TILE, c->face_tiles, nullptr, d + 1);
     make_tiles(nblk, gcnt, CELL_TILE, c->ghost_tiles, nullptr);
     if ((rc = upload_vec(c, c->cell_tiles.data(), sizeof(Tile) * c->cell_tiles.size(), (void**)&c->d_cell))) return rc;
-    for (int d = 0; d < 3; ++d)
-        if ((rc = upload_vec(c, c->face_tiles[d].data(), sizeof(Tile) * c->face_tiles[d].size(), (void**)&c->d_face[d]))) return rc;
+    if ((rc = upload_vec(c, c->face_tiles.data(), sizeof(Tile) * c->face_tiles.size(), (void**)&c->d_face))) return rc;
     if ((rc = upload_vec(c, c->ghost_tiles.data(), sizeof(Tile) * c->ghost_tiles.size(), (void**)&c->d_ghost))) return rc;
     if (c->mixed && c->resid_tma != 0 && !build_resid_tma(c)) c->resid_tma = 0;
     // boundary tables
