@@ -81,6 +81,19 @@ __host__ __device__ inline size_t sw_at(long long q, int m, int width) {
     return (size_t)q * (size_t)width + (size_t)m;
 }
 
+// FP64 marching sweeps (sweep_march64.cuh): the record of a cell -- per direction its Jacobian terms
+// of the mean flow, the mean-flow diagonal, the radii, stept, cvs, the k-omega diagonal and
+// contravariant speeds -- and its DeltaQ; entry m of storage place q, the 32 places of a step side by
+// side.  The mean flow reads entries 0 .. M64_MEAN_ROWS - 1, k and omega those from M64_TURB_ROW0 on.
+enum March64Rec { M64_TERMS = JC_VPT, M64_FM = 3 * M64_TERMS, M64_RDS = M64_FM + 1, M64_STEPT = M64_RDS + 3, M64_CVS = M64_STEPT + 1,
+                  M64_FT = M64_CVS + 1, M64_VPT = M64_FT + 1, M64_WIDTH = M64_VPT + 3,
+                  M64_MEAN_ROWS = M64_FT, M64_TURB_ROW0 = M64_RDS };
+__host__ __device__ inline int m64_diag(int m) {      // of the hyperplane records' REC_STEPT .. REC_FT
+    return m == REC_STEPT ? M64_STEPT : m == REC_CVS ? M64_CVS : m == REC_FM ? M64_FM : M64_FT;
+}
+__host__ __device__ inline size_t m64_rec(long long q, int m) { return ((size_t)(q >> 5) * M64_WIDTH + m) * 32 + (q & 31); }
+__host__ __device__ inline size_t m64_dq(long long q, int L) { return ((size_t)(q >> 5) * DQ_STRIDE + L) * 32 + (q & 31); }
+
 // face-flux components (per face and direction)
 enum FX { FX_VX = 0, FX_VY = 1, FX_VZ = 2, FX_VE = 3, FX_TK = 4, FX_TO = 5,
           FX_C0 = 6, FX_CK = 11, FX_CO = 12, NFX = 13 };

@@ -200,8 +200,7 @@ int ctx_init(Ctx* c, int precision, long long budget) {
         const char* pfs = std::getenv("TRANS_SWEEP_PF");
         c->sweep_pf = pfs ? std::max(0, std::atoi(pfs)) : 0;
     }
-    // march: marching warps (mixed path; the FP64 path takes planes)
-    if (ms == "march" && !c->mixed) ms = "planes";
+    // march: marching warps
     if (ms == "march") {
         c->sweep_forced = true;
         c->sweep_mode = 6;
@@ -239,8 +238,8 @@ void free_worklists(Ctx* c) {
     dfree(c->d_rmaps);
     dfree(c->d_bc); dfree(c->d_outlet); dfree(c->d_lines); dfree(c->d_sweep); dfree(c->d_plane_off); dfree(c->d_pb_off);
     dfree(c->d_nbp); dfree(c->d_flags); dfree(c->d_rec); dfree(c->d_dqs); dfree(c->d_dq2); dfree(c->d_orph); dfree(c->d_dq_save);
-    dfree(c->d_mtiles); dfree(c->d_medgeJ); dfree(c->d_medgeK); dfree(c->d_mctl);
-    c->n_mtiles = 0;
+    dfree(c->d_mtiles); dfree(c->d_mruns); dfree(c->d_medgeJ); dfree(c->d_medgeK); dfree(c->d_mctl);
+    c->n_mtiles = c->n_mruns = 0;
     c->march = false;
     c->pair_lo.clear(); c->pair_up.clear(); dfree(c->d_parts); dfree(c->d_pc);
     dfree(c->d_cdev); dfree(c->d_stage); dfree(c->d_tile_first); dfree(c->d_norms);

@@ -113,11 +113,13 @@ struct Ctx {
     struct SweepPair { int p_first, p_count, o_off, o_count; };
     std::vector<SweepPair> pair_lo, pair_up;
     int* d_orph = nullptr;
-    // marching warps (sweep_mode 6, mixed path, its default): the sweep arrays are stored in their order;
-    // tiles, edge buffers and counters
+    // marching warps (sweep_mode 6, the default where their arrays fit; not with preconditioning): the sweep
+    // arrays are stored in their order; tiles, edge buffers, counters, and the FP64 records' runs of steps
     bool march = false;
     MarchTile* d_mtiles = nullptr;
     int n_mtiles = 0;
+    int2* d_mruns = nullptr;
+    int n_mruns = 0;
     void *d_medgeJ = nullptr, *d_medgeK = nullptr;
     MarchCtl* d_mctl = nullptr;
     double* d_pc = nullptr;              // PrecondDW coefficients of the sweep neighbours (IF_Precondition = 1)
@@ -146,8 +148,8 @@ struct Ctx {
     // 0 = one launch per hyperplane (graph), 1 = one cooperative launch with grid barriers,
     // 2 = dataflow over ready flags, 3 = tiled wavefront, 4 = one thread-block cluster per
     // block with cluster barriers between hyperplanes (mixed path; sweep_grid = CTAs per
-    // cluster), 5 = two hyperplanes per launch (mixed path, graph), 6 = marching warps (mixed path,
-    // where its arrays fit); -1 = pick the fastest of the others on first use
+    // cluster), 5 = two hyperplanes per launch (mixed path, graph), 6 = marching warps (the
+    // default where their arrays fit, without preconditioning); -1 = pick the fastest of the others on first use
     // (all bit-identical)
     int sweep_mode = -1, sweep_grid = 0, sweep_block = 0;
     int tile_shape[3] = {0, 0, 0};       // tiles of the tiled wavefront (built for this shape)

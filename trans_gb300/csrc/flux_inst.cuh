@@ -31,8 +31,8 @@ void hu(cudaStream_t s, const DevBlock& b, const int* tab, int n, int sweep, dou
 void fc(cudaStream_t s, const DevBlock* b, const Tile* t, int nt, const CaseDev* cd) {
     if (nt > 0) k_sst_fc1<TG_R><<<nt, CELL_TILE, 0, s>>>(b, t, cd);
 }
-void prep(cudaStream_t s, const DevBlock* b, const Tile* tiles, int nt, const int* qpos, const SweepView& v, const CaseDev* cd) {
-    if (nt > 0) k_lusgs_prep<TG_R><<<nt, CELL_TILE, 0, s>>>(b, tiles, qpos, (TG_R*)v.rec, (TG_R*)v.dq, cd);
+void prep(cudaStream_t s, const DevBlock* b, const Tile* tiles, int nt, const int* qpos, const SweepView& v, const CaseDev* cd, int march) {
+    if (nt > 0) k_lusgs_prep<TG_R><<<nt, CELL_TILE, 0, s>>>(b, tiles, qpos, (TG_R*)v.rec, (TG_R*)v.dq, cd, march);
 }
 // the FP64 path's neighbour Jacobian terms; the mixed path rebuilds them in the sweep from the
 // compact records k_lusgs_prep writes, so it has no such pass
@@ -167,8 +167,8 @@ void swpair(cudaStream_t s, const SweepView& v, void* y, bool lower, int p_first
                                o_count, turb & 3, chained, pf_first, pf_count);
     }
 }
-void scat(cudaStream_t s, const DevBlock* b, const Tile* tiles, int nt, const int* qpos, const SweepView& v, int l0) {
-    if (nt > 0 && v.n > 0) k_sweep_scatter<TG_R><<<nt, CELL_TILE, 0, s>>>(b, tiles, qpos, (const TG_R*)v.dq, l0);
+void scat(cudaStream_t s, const DevBlock* b, const Tile* tiles, int nt, const int* qpos, const SweepView& v, int l0, int march) {
+    if (nt > 0 && v.n > 0) k_sweep_scatter<TG_R><<<nt, CELL_TILE, 0, s>>>(b, tiles, qpos, (const TG_R*)v.dq, l0, march);
 }
 }  // namespace
 

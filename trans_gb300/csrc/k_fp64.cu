@@ -4,6 +4,7 @@
 #define TG_NAME flux_launchers_f64
 #define TG_COMMON_KERNELS
 #include "flux_inst.cuh"
+#include "sweep_march64.cuh"
 
 namespace tg {
 void launch_specrad(cudaStream_t s, const DevBlock* blks, const Tile* tiles, int nt, const CaseDev* cdev) {
@@ -46,6 +47,27 @@ void launch_geom_static(cudaStream_t s, const DevBlock* blks, int nblk, long lon
 }  // namespace tg
 
 namespace tg {
+template <int TURB>
+static cudaError_t march64(cudaStream_t s, const SweepView& v, const MarchTile* tiles, int ntiles, ulonglong2* bufJ, ulonglong2* bufK,
+                           MarchCtl* ctl, SweepSync* sy, unsigned limit) {
+    const int n = march64_ctas(ntiles, TURB);
+    const size_t sm = march64_bytes(TURB);
+    cudaError_t e = cudaFuncSetAttribute(k_march64<true, TURB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_march64<false, TURB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    k_march64<true, TURB><<<n, 160, sm, s>>>(tiles, ntiles, (const f64*)v.rec, (f64*)v.dq, bufJ, bufK, ctl, sy, limit);
+    k_march64<false, TURB><<<n, 160, sm, s>>>(tiles, ntiles, (const f64*)v.rec, (f64*)v.dq, bufJ, bufK, ctl, sy, limit);
+    return cudaGetLastError();
+}
+cudaError_t launch_sweep_march64(cudaStream_t s, const SweepView& v, const MarchTile* tiles, int ntiles, void* bufJ, void* bufK,
+                                 MarchCtl* ctl, SweepSync* sy, int turb, unsigned limit) {
+    if (ntiles <= 0) return cudaSuccess;
+    auto f = (turb & 3) == 0 ? march64<0> : (turb & 3) == 1 ? march64<1> : march64<2>;
+    return f(s, v, tiles, ntiles, (ulonglong2*)bufJ, (ulonglong2*)bufK, ctl, sy, limit);
+}
+void launch_march64_jac(cudaStream_t s, const DevBlock* blks, const MarchTile* tiles, const int2* runs, int nruns, void* rec) {
+    if (nruns > 0) k_march64_jac<<<(nruns + 3) / 4, 128, 0, s>>>(blks, tiles, runs, nruns, (f64*)rec);
+}
 void launch_halo_pack(cudaStream_t s, const DevBlock& b, const int* cells, int n, int sweep, int dq_fp32, double* out) {
     if (n > 0) k_halo_pack<<<(n + 127) / 128, 128, 0, s>>>(b, cells, n, sweep, dq_fp32, out);
 }

@@ -1142,7 +1142,7 @@ __device__ inline R rc_fr1(const ParamsT<R>& p, const DevBlock& b, int I, int J,
 #endif
 template <typename R>
 __global__ void __launch_bounds__(CELL_TILE, sizeof(R) == 4 ? TG_PREP_MINB : TG_PREP_MINB_F64) k_lusgs_prep(const DevBlock* __restrict__ blks, const Tile* __restrict__ tiles, const int* __restrict__ qpos,
-                             R* __restrict__ rec, R* __restrict__ dq, const CaseDev* __restrict__ cdev) {
+                             R* __restrict__ rec, R* __restrict__ dq, const CaseDev* __restrict__ cdev, int march) {
     const Tile t = tiles[blockIdx.x];
     if ((int)threadIdx.x >= t.count) return;
     const DevBlock b = blks[t.blk];
@@ -1153,8 +1153,9 @@ __global__ void __launch_bounds__(CELL_TILE, sizeof(R) == 4 ? TG_PREP_MINB : TG_
     const int I = nlex % b.NI1 + 1, J = (nlex / b.NI1) % b.NJ1 + 1, K = nlex / (b.NI1 * b.NJ1) + 1;
     const long long q = qpos[(size_t)blockIdx.x * CELL_TILE + threadIdx.x];
     const int c = cidx(b, I, J, K);
-    auto REC = [&](int m) -> R& { return rec[sw_at(q, m, NREC)]; };
-    auto DQ = [&](int L) -> R& { return dq[sw_at(q, L, DQ_STRIDE)]; };
+    // FP64: in hyperplane order, or that of the marching sweeps (march)
+    auto REC = [&](int m) -> R& { return rec[march ? m64_rec(q, m64_diag(m)) : sw_at(q, m, NREC)]; };
+    auto DQ = [&](int L) -> R& { return dq[sizeof(R) == 8 && march ? m64_dq(q, L) : sw_at(q, L, DQ_STRIDE)]; };
     // BDF2 right-hand side and the mean-flow diagonal (TIME_LUSGS.F90:73-108).  FP64 path: the
     // reference's operations.  Mixed path: the time-level difference 3V - 4Wt0 + Wt1 in FP64
     // (it cancels), everything else in FP32 with one reciprocal of the volume.  (This kernel is
@@ -1981,7 +1982,7 @@ __global__ void k_sweep_tiles(const int* __restrict__ nbp, const R* __restrict__
 // the Runge-Kutta path sweeps and returns only k and omega, l0 = 5)
 template <typename R>
 __global__ void k_sweep_scatter(const DevBlock* __restrict__ blks, const Tile* __restrict__ tiles, const int* __restrict__ qpos,
-                                const R* __restrict__ dq, int l0) {
+                                const R* __restrict__ dq, int l0, int march) {
     const Tile t = tiles[blockIdx.x];
     if ((int)threadIdx.x >= t.count) return;
     const DevBlock b = blks[t.blk];
@@ -1991,7 +1992,7 @@ __global__ void k_sweep_scatter(const DevBlock* __restrict__ blks, const Tile* _
     const long long q = qpos[(size_t)blockIdx.x * CELL_TILE + threadIdx.x];
     R d[7];
 #pragma unroll
-    for (int L = 0; L < 7; ++L) d[L] = L >= l0 ? dq[sw_at(q, L, DQ_STRIDE)] : R(0);
+    for (int L = 0; L < 7; ++L) d[L] = L >= l0 ? dq[sizeof(R) == 8 && march ? m64_dq(q, L) : sw_at(q, L, DQ_STRIDE)] : R(0);
 #pragma unroll
     for (int L = 0; L < 7; ++L)
         if (L >= l0) rs<R>(b, S_D + L)[c] = d[L];

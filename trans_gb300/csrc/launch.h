@@ -85,6 +85,15 @@ struct MarchCtl;
 cudaError_t launch_sweep_march(cudaStream_t s, const SweepView& v, const MarchTile* tiles, int ntiles, void* bufJ,
                                void* bufK, MarchCtl* ctl, SweepSync* sy, int turb, unsigned limit);
 
+// the FP64 path's (k_fp64.cu, sweep_march64.cuh), and the Jacobian terms of its records: runs of
+// M64_JAC_STEPS steps of a tile
+cudaError_t launch_sweep_march64(cudaStream_t s, const SweepView& v, const MarchTile* tiles, int ntiles, void* bufJ, void* bufK,
+                                 MarchCtl* ctl, SweepSync* sy, int turb, unsigned limit);
+void launch_march64_jac(cudaStream_t s, const DevBlock* blks, const MarchTile* tiles, const int2* runs, int nruns, void* rec);
+constexpr int M64_JAC_STEPS = 2;
+constexpr int M64_EDGES = 7;               // edge words of a step and lane, one per component (FP32: MARCH_EDGES)
+constexpr int MARCH_EDGES = 4;
+
 // flux, source and sweep kernels, instantiated per arithmetic type
 struct FluxLaunchers {
     void (*gradient)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*);
@@ -97,8 +106,9 @@ struct FluxLaunchers {
     void (*halo_unpack)(cudaStream_t, const DevBlock&, const int* tab, int n, int sweep, double cost, double sint,
                         const double* in);
     // LU-SGS right-hand sides + neighbour Jacobian terms into the sweep-order arrays
-    // (cell order over the cell tiles; qpos = sweep position of each tile slot)
-    void (*prep)(cudaStream_t, const DevBlock*, const Tile*, int nt, const int* qpos, const SweepView&, const CaseDev*);
+    // (cell order over the cell tiles; qpos = sweep position of each tile slot; march: the arrays are
+    // stored in the order of the marching sweeps)
+    void (*prep)(cudaStream_t, const DevBlock*, const Tile*, int nt, const int* qpos, const SweepView&, const CaseDev*, int march);
     void (*jac)(cudaStream_t, const DevBlock*, const SweepView&, const CaseDev*);   // neighbours' Jacobian terms (sweep order)
     // lanes: components swept (bits 0-1: 0 mean flow, 1 all, 2 k-omega) | SWEEP_WPC thread mapping
     // (pf_first, pf_count: a later hyperplane prefetched into L2, count 0 = none; chained: 0 plain
@@ -122,7 +132,7 @@ struct FluxLaunchers {
                                int grid, int block, unsigned limit);
     int (*sweep_tiles_occupancy)(int block);
     // DeltaQ l0..6 back to cell order, one thread per interior cell of the cell tiles
-    void (*scatter)(cudaStream_t, const DevBlock*, const Tile*, int nt, const int* qpos, const SweepView&, int l0);
+    void (*scatter)(cudaStream_t, const DevBlock*, const Tile*, int nt, const int* qpos, const SweepView&, int l0, int march);
     // two hyperplanes per launch (mixed path only; null in FP64): the lower sweep reads v.dq and
     // writes y, the upper reads y and writes v.dq; p_first/p_count: the second plane, orph/o_count:
     // the first plane's positions with no neighbour on the second

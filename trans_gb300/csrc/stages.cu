@@ -295,11 +295,11 @@ int sweep_once(Ctx* c, int mode, int grid, int block, bool capture = false) {
         return TRANS_OK;
     }
     if (mode == 6) {
-        if (!c->march) return fail(c, TRANS_E_ARG, "marching sweeps are a mixed-path schedule");
+        if (!c->march) return fail(c, TRANS_E_ARG, "the sweep arrays are not in the marching order");
         // (graph replays keep the flag cleared here or by the run that reported it)
         if (!capture) CK(cudaMemsetAsync(c->d_sync, 0, sizeof(SweepSync), s));
-        CK(launch_sweep_march(s, c->sv, c->d_mtiles, c->n_mtiles, c->d_medgeJ, c->d_medgeK, c->d_mctl, c->d_sync,
-                              c->sweep_lanes, c->spin_limit));
+        auto launch = c->mixed ? launch_sweep_march : launch_sweep_march64;
+        CK(launch(s, c->sv, c->d_mtiles, c->n_mtiles, c->d_medgeJ, c->d_medgeK, c->d_mctl, c->d_sync, c->sweep_lanes, c->spin_limit));
         if (!capture) CK(cudaMemcpyAsync(c->h_sync, c->d_sync, sizeof(SweepSync), cudaMemcpyDeviceToHost, s));
         c->launches += 2;
         return TRANS_OK;
@@ -655,8 +655,9 @@ int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot) {
             }
             {
                 KScope t(c, K_PREP);
-                c->fl->prep(s, c->d_blk, c->d_cell, nct, c->d_qpos, c->sv, c->d_cdev);
-                c->fl->jac(s, c->d_blk, c->sv, c->d_cdev);
+                c->fl->prep(s, c->d_blk, c->d_cell, nct, c->d_qpos, c->sv, c->d_cdev, c->march);
+                if (!c->march) c->fl->jac(s, c->d_blk, c->sv, c->d_cdev);
+                else if (!c->mixed) launch_march64_jac(s, c->d_blk, c->d_mtiles, c->d_mruns, c->n_mruns, c->sv.rec);
             }
             c->launches += 2;
             {
@@ -672,7 +673,7 @@ int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot) {
                 else rc = run_sweeps(c);
                 if (rc) return rc;
             }
-            { KScope t(c, K_SCATTER); c->fl->scatter(s, c->d_blk, c->d_cell, nct, c->d_qpos, c->sv, c->sweep_lanes == 2 ? 5 : 0); }
+            { KScope t(c, K_SCATTER); c->fl->scatter(s, c->d_blk, c->d_cell, nct, c->d_qpos, c->sv, c->sweep_lanes == 2 ? 5 : 0, c->march); }
             c->launches++;
             break;
         }

@@ -26,18 +26,10 @@
 // warp records the error and the tile goes on without the words.
 #pragma once
 #include "kernels.cuh"
+#include "march_words.cuh"
 
 namespace tg {
 
-__device__ __forceinline__ ulonglong2 march_ld(const ulonglong2* p) {
-    ulonglong2 v;
-    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ void march_st(ulonglong2* p, float x, float y, unsigned tag) {
-    const unsigned long long t = (unsigned long long)tag << 32;
-    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(t | __float_as_uint(x)), "l"(t | __float_as_uint(y)));
-}
 __device__ __forceinline__ void march_copy16(void* smem, const void* g) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g) : "memory");
 }

@@ -44,14 +44,14 @@ struct TileView {
     const int* dep;
 };
 
-// Marching sweeps (mixed path, sweep_march.cuh): a tile of MARCH_J x MARCH_K lines of a block (nj x nk
+// Marching sweeps (sweep_march.cuh, sweep_march64.cuh): a tile of MARCH_J x MARCH_K lines of a block (nj x nk
 // of them inside it), one warp, walked along i.  The records and DeltaQ are stored in its order, 32
 // places a step (lane a + MARCH_J b of step i - 1 + a + b), from step s0 on; the edge buffers are
 // numbered by the same steps.  sJ, sK: the first steps of the tiles it takes edge words from in the
 // lower (0) and upper (1) sweep, -1 = none.
 constexpr int MARCH_J = 8, MARCH_K = 4;      // MARCH_J * MARCH_K = 32 lanes
 constexpr int MARCH_STAGES = 8;              // shared-memory stages of 3.6 KB
-struct MarchTile { int NI1, nj, nk, s0, sJ[2], sK[2]; };
+struct MarchTile { int NI1, nj, nk, s0, sJ[2], sK[2], blk, j0, k0; };
 struct MarchCtl { unsigned epoch, ticket[2], done[2]; };
 
 struct NormPart {         // per-tile partial residual norms (Time/TIME_Update_V.F90:106-294)

@@ -249,11 +249,12 @@ int build_march(Ctx* c) {
             return tj < 0 || tk < 0 || tj >= ntj[k.n] || tk >= ntk[k.n] ? -1 : first[k.n][tj + (size_t)ntj[k.n] * tk];
         };
         tiles.push_back(MarchTile{b.NI1, std::min(MARCH_J, b.NJ1 - k.tj * MARCH_J), std::min(MARCH_K, b.NK1 - k.tk * MARCH_K),
-                                  at(k.tj, k.tk), {at(k.tj - 1, k.tk), at(k.tj + 1, k.tk)}, {at(k.tj, k.tk - 1), at(k.tj, k.tk + 1)}});
+                                  at(k.tj, k.tk), {at(k.tj - 1, k.tk), at(k.tj + 1, k.tk)}, {at(k.tj, k.tk - 1), at(k.tj, k.tk + 1)},
+                                  k.n, k.tj * MARCH_J + 1, k.tk * MARCH_K + 1});
     }
-    const size_t word = 4 * sizeof(ulonglong2);        // 8 floats, each with its tag
+    const size_t word = (c->mixed ? MARCH_EDGES : M64_EDGES) * sizeof(ulonglong2);     // 8 floats or 7 doubles, every 32 bits with the tag
     const size_t nj = (size_t)s0 * MARCH_K * word, nk = (size_t)s0 * MARCH_J * word, places = (size_t)s0 * 32;
-    const size_t nrec = places * NCREC * sizeof(float), ndq = places * DQ_STRIDE * sizeof(float);
+    const size_t nrec = places * (c->mixed ? (size_t)NCREC : (size_t)M64_WIDTH) * c->fl->elem, ndq = places * DQ_STRIDE * c->fl->elem;
     auto room = [](void* p, size_t bytes) { return cudaMalloc((void**)p, bytes) == cudaSuccess; };
     if (!room(&c->d_medgeJ, nj) || !room(&c->d_medgeK, nk) || !room(&c->d_rec, nrec) || !room(&c->d_dqs, ndq)) {
         cudaGetLastError();
@@ -266,6 +267,13 @@ int build_march(Ctx* c) {
     int rc;
     if ((rc = upload_vec(c, tiles.data(), sizeof(MarchTile) * tiles.size(), (void**)&c->d_mtiles))) return rc;
     c->n_mtiles = (int)tiles.size();
+    if (!c->mixed) {
+        std::vector<int2> runs;
+        for (int t = 0; t < c->n_mtiles; ++t)
+            for (int s = 0; s < tiles[t].NI1 + MARCH_J + MARCH_K - 2; s += M64_JAC_STEPS) runs.push_back(make_int2(t, s));
+        if ((rc = upload_vec(c, runs.data(), sizeof(int2) * runs.size(), (void**)&c->d_mruns))) return rc;
+        c->n_mruns = (int)runs.size();
+    }
     CK(cudaMalloc(&c->d_mctl, sizeof(MarchCtl)));
     CK(cudaMemsetAsync(c->d_medgeJ, 0, nj, c->stream));         // tag 0 is never used
     CK(cudaMemsetAsync(c->d_medgeK, 0, nk, c->stream));
@@ -351,7 +359,7 @@ int rebuild(Ctx* c) {
     if ((rc = upload_vec(c, c->outlet.data(), sizeof(BCEntry) * c->outlet.size(), (void**)&c->d_outlet))) return rc;
     if ((rc = upload_vec(c, c->lines.data(), sizeof(OutletLine) * c->lines.size(), (void**)&c->d_lines))) return rc;
     c->march = false;
-    if (c->mixed && (!c->sweep_forced || c->sweep_mode == 6) && (rc = build_march(c))) return rc;
+    if (c->cases[0]->p.IF_Precondition != 1 && (!c->sweep_forced || c->sweep_mode == 6) && (rc = build_march(c))) return rc;
     if (c->sweep_forced && c->sweep_mode == 6 && !c->march) return fail(c, TRANS_E_ARG, "the marching sweeps do not fit");
     if (!c->march) {
         // hyperplane order of the LU-SGS sweeps over all blocks of all cases: h = i+j+k = 3 ..
