@@ -17,9 +17,9 @@
 //
 // Bound by the FP64 pipe and the chain of a step: 46 FP64 instructions (1.5 us) and two divisions on
 // the integer pipe on the way from one step to the next, 2.2 us a step of a tile by itself.  Both
-// sweeps with the records' preparation, hyperplane launches before and now: 16x12x10 cells 355 and
-// 283 us, 64x48x20 1,213 and 798 us, 98,304 cells 2,400 and 1,932 us, 490,560 cells 8,047 and 5,185 us;
-// k and omega alone (Runge-Kutta, annulus, three stages) 2,162 and 1,268 us.
+// sweeps with the records' preparation, hyperplane launches before and now: 24x16x5 cells 355 and
+// 283 us, 96x48x8 1,213 and 798 us, a cascade of 352,256 cells 2,400 and 1,932 us, of 1,966,080 cells
+// 8,047 and 5,185 us; k and omega alone (Runge-Kutta, annulus 70x38x26, three stages) 2,162 and 1,268 us.
 #pragma once
 #include "kernels.cuh"
 #include "launch.h"
@@ -77,7 +77,7 @@ struct March64Walk {
 };
 
 // Bulk copies of a step's inputs into a stage, complete on a transaction barrier; the wait for a phase
-// is bounded.  Four stages leave two mean-flow CTAs on an SM: at 490,560 cells 3.42 ms for both sweeps,
+// is bounded.  Four stages leave two mean-flow CTAs on an SM: at 1,966,080 cells 3.42 ms for both sweeps,
 // against 3.71 with three stages and CTAs and 4.03 with two stages and four (the CTAs of one SM
 // are on one diagonal, and the steps of each take longer); no difference at the smaller sizes.
 constexpr int M64_STAGES = 4;
@@ -338,7 +338,7 @@ k_march64(const MarchTile* __restrict__ tiles, int ntiles, const f64* __restrict
 }
 
 // The cells' Jacobian terms and radii into the records, one warp per M64_JAC_STEPS steps of a tile: a step
-// is 156 FP64 instructions, so warps of eight steps left the smallest blocks waiting (with prep, 16x12x10
+// is 156 FP64 instructions, so warps of eight steps left the smallest blocks waiting (with prep, 24x16x5
 // cells: 108 us, and 53 with two); consecutive steps of a lane read consecutive cells of its line
 static __global__ void __launch_bounds__(128) k_march64_jac(const DevBlock* __restrict__ blks, const MarchTile* __restrict__ tiles,
                                                             const int2* __restrict__ runs, int nruns, f64* __restrict__ rec) {
