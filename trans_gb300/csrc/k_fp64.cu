@@ -11,7 +11,7 @@ void launch_specrad(cudaStream_t s, const DevBlock* blks, const Tile* tiles, int
     if (nt > 0) k_specrad<<<nt, CELL_TILE, 0, s>>>(blks, tiles, cdev);
 }
 void launch_bc_state(cudaStream_t s, const DevBlock* blks, const BCEntry* ent, int n, const CaseDev* cdev) {
-    if (n > 0) k_bc_state<<<(n + 127) / 128, 128, 0, s>>>(blks, ent, n, cdev);
+    if (n > 0) k_bc_state<<<(n + 31) / 32, 32, 0, s>>>(blks, ent, n, cdev);
 }
 void launch_bc_outlet(cudaStream_t s, const DevBlock* blks, const BCEntry* ent, const OutletLine* lines, int nl,
                       const CaseDev* cdev) {
