@@ -1,4 +1,4 @@
-"""The integer-pipe double division and square root of the FP64 path (trans_gb300/csrc/soft64.cuh)
+"""The integer-pipe double division, square root and comparisons of the FP64 path (trans_gb300/csrc/soft64.cuh)
 against IEEE arithmetic, compiled for the host: the correctly rounded result bit for bit over
 every kind of operand pair where the digit recurrence or the rounding could go wrong.  (The
 device forms are held to the hardware's by trans_check_conversions, tests/test_gpu_cvt.py.)"""
@@ -41,6 +41,10 @@ int main(int, char** v) {
         const double x = of_bits(a), y = of_bits(b), z = fabs(x);
         if (!same(sx::div(x, y), x / y)) ++bad;
         if (!same(sx::sqrt(z), ::sqrt(z))) ++bad;
+        const double w[3] = {y, x, -x};                                                  // comparisons
+        for (double u : w)
+            if (sx::less(x, u) != (x < u) || sx::less(u, x) != (u < x) || sx::less_equal(x, u) != (x <= u) ||
+                sx::less_equal(u, x) != (u <= x) || sx::equal(x, u) != (x == u)) ++bad;
     }
     printf("%ld\n", bad);
     return 0;

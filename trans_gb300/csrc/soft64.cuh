@@ -1,4 +1,4 @@
-// soft64.cuh -- IEEE double division and square root on the integer and FP32 pipes.
+// soft64.cuh -- IEEE double division, square root and comparisons on the integer and FP32 pipes.
 //
 // GB300 issues one FP64 warp instruction per SM sub-partition every ~64 cycles (2 lanes per SM
 // and clock) and a compiled double division or square root is ten of them or more, so the FP64
@@ -138,6 +138,17 @@ SX_FN double div(double a, double b) {
     return of_bits(sign | (((uint64_t)e << 52) + ((N + 1) >> 1)));
 }
 
+// comparisons (an FP64 instruction each): the bit patterns as integers in the order of the values (both
+// zeros 0), false with a NaN; face fluxes of 1,966,080 cells 15.62 -> 15.40 ms, an iteration 25.03 -> 24.71
+SX_FN bool is_nan(double a) { return (bits_of(a) << 1) > 0xffe0000000000000ull; }
+SX_FN int64_t order_of(double a) {
+    const int64_t u = (int64_t)bits_of(a);
+    return u < 0 ? (int64_t)(0x8000000000000000ull - (uint64_t)u) : u;
+}
+SX_FN bool less(double a, double b) { return order_of(a) < order_of(b) && !is_nan(a) && !is_nan(b); }
+SX_FN bool less_equal(double a, double b) { return order_of(a) <= order_of(b) && !is_nan(a) && !is_nan(b); }
+SX_FN bool equal(double a, double b) { return order_of(a) == order_of(b) && !is_nan(a) && !is_nan(b); }
+
 SX_RARE double sqrt_rare(double a) { return ::sqrt(a); }
 
 SX_FN double sqrt(double a) {
@@ -187,12 +198,12 @@ SX_FN f64 operator*(f64 a, f64 b) { return f64(a.v * b.v); }
 SX_FN f64 operator/(f64 a, f64 b) {
     return f64(sx::div(a.v, b.v));
 }
-SX_FN bool operator<(f64 a, f64 b) { return a.v < b.v; }
-SX_FN bool operator>(f64 a, f64 b) { return a.v > b.v; }
-SX_FN bool operator<=(f64 a, f64 b) { return a.v <= b.v; }
-SX_FN bool operator>=(f64 a, f64 b) { return a.v >= b.v; }
-SX_FN bool operator==(f64 a, f64 b) { return a.v == b.v; }
-SX_FN bool operator!=(f64 a, f64 b) { return a.v != b.v; }
+SX_FN bool operator<(f64 a, f64 b) { return sx::less(a.v, b.v); }
+SX_FN bool operator>(f64 a, f64 b) { return sx::less(b.v, a.v); }
+SX_FN bool operator<=(f64 a, f64 b) { return sx::less_equal(a.v, b.v); }
+SX_FN bool operator>=(f64 a, f64 b) { return sx::less_equal(b.v, a.v); }
+SX_FN bool operator==(f64 a, f64 b) { return sx::equal(a.v, b.v); }
+SX_FN bool operator!=(f64 a, f64 b) { return !sx::equal(a.v, b.v); }
 using ::sqrt;
 using ::fabs;
 SX_FN f64 sqrt(f64 a) { return f64(sx::sqrt(a.v)); }
