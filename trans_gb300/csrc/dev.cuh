@@ -105,7 +105,15 @@ struct DevBlock {
     int cs;               // case slot: index of the block's case in the CaseDev array
     double* base;
     float* fbase;         // FP32 copies of the slots read by the FP32 kernels (mixed mode only)
+    double* aux;          // shared terms of the FP64 face fluxes (AuxTerm), or null
 };
+
+// Terms that several faces share, one value per padded cell c (k_face_terms): AX_FA + 7 (dir-1) + v, the
+// face average of u, v, w, T, k, omega, p over the cell's minus face; AX_PR + 7 k + m, products of the
+// reconstructed variable k (u, v, w, p, T) with a constant (MdcdProduct); AX_DD + 10 (dir-1) + 2 k + e,
+// squared second differences of the variable, from the cell onwards and backwards to it.
+enum AuxTerm { AX_FA = 0, AX_PR = 21, AX_DD = 56, AX_MUSCL = AX_PR, AX_MDCD = 86 };   // entries per cell of the two schemes
+enum MdcdProduct { MP_H, MP_G, MP_13, MP_76, MP_116, MP_16, MP_56, NMP };           // 3/2, 5/2, 1/3, 7/6, 11/6, 1/6, 5/6
 
 constexpr int CELL_TILE = 256;   // interior cells per cell tile (and threads per CTA of the cell kernels)
 constexpr int SWEEP_LANES = 8;   // threads per cell in the LU-SGS sweeps (one per DeltaQ component)
@@ -434,41 +442,54 @@ template <> __device__ inline void mdcd_pair<float>(const float* s6, float gama,
 // The indicators are non-negative, so their maximum is an integer maximum of the bit patterns.
 // 130 FP64 instructions and 16 quotients per variable and face, against ~170 for the
 // expressions as written (face fluxes of the benchmark cascade 18.0 -> 16.8 ms per iteration).
-template <> __device__ __forceinline__ void mdcd_pair<f64>(const f64* s, f64 gama, f64& ql, f64& qr) {
-    const f64 beta = f64(1.0408329997330663);      // sqrt(13 / 12)
+// The products, and the squared second differences, are terms of a cell that serve up to six
+// faces; where k_face_terms has left them in memory, 88 instructions are left.
+//
+// pr(m, o): product m of stencil value o (0..5); dd(o), de(o): (beta s_o - 2 beta s_(o+1)) + beta s_(o+2)
+// squared, and the same from s_(o+2) backwards.
+constexpr double MDCD_BETA = 1.0408329997330663;      // sqrt(13 / 12)
+__device__ constexpr double mdcd_factor(int m) {
+    return m == MP_H ? 1.5 : m == MP_G ? 2.5 : m == MP_13 ? 2. / 6. : m == MP_76 ? 7. / 6. : m == MP_116 ? 11. / 6. : m == MP_16 ? 1. / 6. : 5. / 6.;
+}
+__device__ __forceinline__ f64 mdcd_dd(f64 b0, f64 b1, f64 b2) { return sq(fma2(-2.0, b1, b0) + b2); }
+template <class P, class D, class E>
+__device__ __forceinline__ void mdcd_states(const f64* s, f64 gama, const P& pr, const D& dd, const E& de, f64& ql, f64& qr) {
     const f64 epsm = f64(1.0e-6);
     const f64 aw0 = f64(1.5) * (f64(0.0463783) + gama);
     const f64 aw1 = f64(0.5 - 1.5 * 0.0463783) + f64(4.5) * gama;
     const f64 aw2 = f64(0.5 - 1.5 * 0.0463783) - f64(4.5) * gama;
     const f64 aw3 = f64(1.5) * (f64(0.0463783) - gama);
-    const f64 c26 = f64(2. / 6.), c76 = f64(7. / 6.), c116 = f64(11. / 6.), c16 = f64(1. / 6.), c56 = f64(5. / 6.);
-    f64 b[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) b[k] = beta * s[k];
-    const f64 h0 = f64(1.5) * s[0], h2 = f64(1.5) * s[2], h3 = f64(1.5) * s[3], h5 = f64(1.5) * s[5];
-    const f64 g2 = f64(2.5) * s[2], g3 = f64(2.5) * s[3];
-    const f64 p0 = c26 * s[0], p1 = c76 * s[1], p2 = c116 * s[2], p3 = c116 * s[3], p4 = c76 * s[4], p5 = c26 * s[5];
-    const f64 e1 = c16 * s[1], e2 = c56 * s[2], e3 = c56 * s[3], e4 = c16 * s[4], t2 = c26 * s[2], t3 = c26 * s[3];
+    const f64 h0 = pr(MP_H, 0), h2 = pr(MP_H, 2), h3 = pr(MP_H, 3), h5 = pr(MP_H, 5);
+    const f64 g2 = pr(MP_G, 2), g3 = pr(MP_G, 3);
+    const f64 p0 = pr(MP_13, 0), p1 = pr(MP_76, 1), p2 = pr(MP_116, 2), p3 = pr(MP_116, 3), p4 = pr(MP_76, 4), p5 = pr(MP_13, 5);
+    const f64 e1 = pr(MP_16, 1), e2 = pr(MP_56, 2), e3 = pr(MP_56, 3), e4 = pr(MP_16, 4), t2 = pr(MP_13, 2), t3 = pr(MP_13, 3);
     // one state from the stencil values in its own order
-    auto state = [&](f64 s0, f64 s1, f64 s3, f64 s4, f64 b0, f64 b1, f64 b2, f64 b3, f64 b4, f64 b5,
+    auto state = [&](f64 s0, f64 s1, f64 s3, f64 s4, f64 d1, f64 d2, f64 d3, f64 d4,
                      f64 m2, f64 m5, f64 n3, f64 r0, f64 r1, f64 r2, f64 r3) {
         const f64 F1 = fma2(0.5, fma2(-4.0, s1, s0), m2);
         const f64 F2 = s3 - s1;
         const f64 F3 = fma2(-0.5, s4, fma2(2.0, s3, -m2));
         const f64 F4 = fma2(-4.0, s4, n3) + m5;
-        const f64 I1 = sq(F1) + sq(fma2(-2.0, b1, b0) + b2);
-        const f64 I2 = fma2(0.25, sq(F2), sq(fma2(-2.0, b2, b1) + b3));
-        const f64 I3 = sq(F3) + sq(fma2(-2.0, b3, b2) + b4);
-        f64 I4 = sq(F4) + sq(fma2(-2.0, b4, b3) + b5);
+        const f64 I1 = sq(F1) + d1;
+        const f64 I2 = fma2(0.25, sq(F2), d2);
+        const f64 I3 = sq(F3) + d3;
+        f64 I4 = sq(F4) + d4;
         I4 = umax(umax(umax(I1, I2), I3), I4);
         const f64 a1 = aw0 / sq(epsm + I1), a2 = aw1 / sq(epsm + I2), a3 = aw2 / sq(epsm + I3), a4 = aw3 / sq(epsm + I4);
         const f64 S = a1 + a2 + a3 + a4;
         return a1 / S * r0 + a2 / S * r1 + a3 / S * r2 + a4 / S * r3;
     };
-    ql = state(s[0], s[1], s[3], s[4], b[0], b[1], b[2], b[3], b[4], b[5], h2, h5, g3,
+    ql = state(s[0], s[1], s[3], s[4], dd(0), dd(1), dd(2), dd(3), h2, h5, g3,
                p0 - p1 + p2, -e1 + e2 + t3, t2 + e3 - e4, p3 - p4 + p5);
-    qr = state(s[5], s[4], s[2], s[1], b[5], b[4], b[3], b[2], b[1], b[0], h3, h0, g2,
+    qr = state(s[5], s[4], s[2], s[1], de(3), de(2), de(1), de(0), h3, h0, g2,
                p5 - p4 + p3, -e4 + e3 + t2, t3 + e2 - e1, p2 - p1 + p0);
+}
+template <> __device__ __forceinline__ void mdcd_pair<f64>(const f64* s, f64 gama, f64& ql, f64& qr) {
+    f64 b[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) b[k] = f64(MDCD_BETA) * s[k];
+    mdcd_states(s, gama, [&](int m, int o) { return f64(mdcd_factor(m)) * s[o]; },
+                [&](int o) { return mdcd_dd(b[o], b[o + 1], b[o + 2]); }, [&](int o) { return mdcd_dd(b[o + 2], b[o + 1], b[o]); }, ql, qr);
 }
 
 // Roe_Common of the rotated scheme (Space/CONVECT_Roe_Rotated.F90:597-752), non-preconditioned:

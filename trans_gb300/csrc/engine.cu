@@ -238,7 +238,7 @@ void free_worklists(Ctx* c) {
     dfree(c->d_rmaps);
     dfree(c->d_bc); dfree(c->d_outlet); dfree(c->d_lines); dfree(c->d_sweep); dfree(c->d_plane_off); dfree(c->d_pb_off);
     dfree(c->d_nbp); dfree(c->d_flags); dfree(c->d_rec); dfree(c->d_dqs); dfree(c->d_dq2); dfree(c->d_orph); dfree(c->d_dq_save);
-    dfree(c->d_mtiles); dfree(c->d_mruns); dfree(c->d_medgeJ); dfree(c->d_medgeK); dfree(c->d_mctl);
+    dfree(c->d_aux); dfree(c->d_mtiles); dfree(c->d_mruns); dfree(c->d_medgeJ); dfree(c->d_medgeK); dfree(c->d_mctl);
     c->n_mtiles = c->n_mruns = 0;
     c->march = false;
     c->pair_lo.clear(); c->pair_up.clear(); dfree(c->d_parts); dfree(c->d_pc);

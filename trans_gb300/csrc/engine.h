@@ -113,6 +113,9 @@ struct Ctx {
     struct SweepPair { int p_first, p_count, o_off, o_count; };
     std::vector<SweepPair> pair_lo, pair_up;
     int* d_orph = nullptr;
+    // the terms that faces of the FP64 path share (AuxTerm), where they fit: device memory and budget
+    // are left for everything else first
+    double* d_aux = nullptr;
     // marching warps (sweep_mode 6, the default where their arrays fit; not with preconditioning): the sweep
     // arrays are stored in their order; tiles, edge buffers, counters, and the FP64 records' runs of steps
     bool march = false;

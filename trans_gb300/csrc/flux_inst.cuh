@@ -7,8 +7,15 @@
 
 namespace tg {
 namespace {
-void grd(cudaStream_t s, const DevBlock* b, const Tile* t, int nt, const CaseDev* cd) {
-    if (nt > 0) k_gradient<TG_R><<<nt, CELL_TILE, 0, s>>>(b, t, cd);
+void grd(cudaStream_t s, const DevBlock* b, const Tile* t, int nt, const CaseDev* cd, bool terms) {
+    if (nt <= 0) return;
+    if constexpr (sizeof(TG_R) == 8) {
+        if (terms) {
+            k_gradient<TG_R, true><<<nt, CELL_TILE, 0, s>>>(b, t, cd);
+            return;
+        }
+    }
+    k_gradient<TG_R><<<nt, CELL_TILE, 0, s>>>(b, t, cd);
 }
 void shg(cudaStream_t s, const DevBlock* b, const Tile* t, int nt) {
     if (nt > 0) k_shock_ghost<TG_R><<<nt, CELL_TILE, 0, s>>>(b, t);
@@ -16,9 +23,16 @@ void shg(cudaStream_t s, const DevBlock* b, const Tile* t, int nt) {
 void bcg(cudaStream_t s, const DevBlock* b, const BCEntry* e, int n) {
     if (n > 0) k_bc_grad<TG_R><<<(n + 127) / 128, 128, 0, s>>>(b, e, n);
 }
-void ff(cudaStream_t s, const DevBlock* b, const Tile* t, int nt, const CaseDev* cd) {
+void ff(cudaStream_t s, const DevBlock* b, const Tile* t, int nt, const CaseDev* cd, bool terms) {
     if (nt <= 0) return;
     // viscous, then convective fluxes (two register budgets)
+    if constexpr (sizeof(TG_R) == 8) {
+        if (terms) {
+            k_face_flux<TG_R, 1, FaceTerms><<<nt, FACE_TILE, 0, s>>>(b, t, cd);
+            k_face_flux<TG_R, 2, FaceTerms><<<nt, FACE_TILE, 0, s>>>(b, t, cd);
+            return;
+        }
+    }
     k_face_flux<TG_R, 1><<<nt, FACE_TILE, 0, s>>>(b, t, cd);
     k_face_flux<TG_R, 2><<<nt, FACE_TILE, 0, s>>>(b, t, cd);
 }

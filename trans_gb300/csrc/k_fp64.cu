@@ -7,6 +7,10 @@
 #include "sweep_march64.cuh"
 
 namespace tg {
+void launch_face_terms(cudaStream_t s, const DevBlock* blks, int nblk, long long total, const long long* off, const CaseDev* cdev,
+                       int mdcd) {
+    if (total > 0) k_face_terms<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(blks, nblk, total, off, cdev, mdcd);
+}
 void launch_specrad(cudaStream_t s, const DevBlock* blks, const Tile* tiles, int nt, const CaseDev* cdev) {
     if (nt > 0) k_specrad<<<nt, CELL_TILE, 0, s>>>(blks, tiles, cdev);
 }

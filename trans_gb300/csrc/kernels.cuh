@@ -454,6 +454,64 @@ __global__ void k_prims(const DevBlock* __restrict__ blks, int nblk, long long t
     rs<f64>(b, S_SVEL + 2)[c] = rs<f64>(b, S_V + 3)[c] * ri;
 }
 
+// The terms that several faces of the FP64 path share (AuxTerm), one thread per padded cell: the face
+// averages, read by the gradient and twice or three times per face by the fluxes, and the MDCD
+// reconstruction's products and squared second differences, each formed by up to six faces before.
+// The same operations on the same operands, so the same bits.  mdcd: with the latter.  A direction's terms
+// belong to the cells that are interior in the other two; face averages from face 0 to N + 2.
+// Bound by the FP64 pipe, like its readers: 72 and 160 instructions a cell against 576 and 720 in the
+// gradient and the faces.  Gradient and face fluxes with this kernel, before and now: the 1,966,080-cell
+// cascade (MDCD) 17.0 and 13.9 ms, 352,256 cells 3.16 and 2.62, the annulus 70x38x26 (three stages) 2.23
+// and 1.93, the channel 96x48x8 (MUSCL) 0.275 and 0.255; 24x16x5 cells no difference.
+__global__ void __launch_bounds__(256) k_face_terms(const DevBlock* __restrict__ blks, int nblk, long long total,
+                                                    const long long* __restrict__ off, const CaseDev* __restrict__ cdev, int mdcd) {
+    const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= total) return;
+    int lo = 0, hi = nblk - 1;
+    while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (off[mid] <= g) lo = mid; else hi = mid - 1; }
+    const DevBlock b = blks[lo];
+    const int c = (int)(g - off[lo]);
+    // (padded columns past NI + 2 hold no cell)
+    const int at[3] = {c % b.PI - 2, c / b.PI % b.PJ - 2, c / (b.PI * b.PJ) - 2}, N[3] = {b.NI, b.NJ, b.NK}, st[3] = {1, b.PI, b.PI * b.PJ};
+    bool in[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) in[d] = at[d] >= 1 && at[d] < N[d];
+    const bool line[3] = {in[1] && in[2], in[0] && in[2], in[0] && in[1]};
+    if (!(line[0] || line[1] || line[2]) || at[0] > N[0] + 2) return;
+    const size_t nc = (size_t)b.ncell;
+    f64* aux = reinterpret_cast<f64*>(b.aux);
+    const int scheme = cdev[b.cs].p.Kind_Spatial, turb = cdev[b.cs].turb;
+    const int qs[7] = {S_PRIM, S_PRIM + 1, S_PRIM + 2, S_T, S_PRIM + 3, S_PRIM + 4, S_PP};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        if (!line[d] || at[d] < 0 || at[d] > N[d] + 1) continue;
+        const int s = st[d];
+        const f64 al = rs<f64>(b, S_ALAGM + d)[c], am = rs<f64>(b, S_ALAGM + d)[c - s], ai = rs<f64>(b, S_AINV + d)[c];
+#pragma unroll
+        for (int v = 0; v < 7; ++v) {
+            if (v == 6 ? scheme > 2 : v > 3 && !turb) continue;       // p: only the MUSCL schemes
+            const f64* q = rs<f64>(b, qs[v]);
+            aux[(AX_FA + 7 * d + v) * nc + c] = (al * q[c - s] + am * q[c]) * ai;
+        }
+    }
+    if (!mdcd || scheme <= 2) return;
+#pragma unroll 1
+    for (int k = 0; k < 5; ++k) {
+        const f64* q = rs<f64>(b, k < 3 ? S_PRIM + k : S_PP + (k - 3));
+        const f64 s0 = q[c], b0 = f64(MDCD_BETA) * s0;
+#pragma unroll
+        for (int m = 0; m < NMP; ++m) aux[(AX_PR + NMP * k + m) * nc + c] = f64(mdcd_factor(m)) * s0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            if (!line[d] || at[d] > N[d]) continue;
+            const f64 b1 = f64(MDCD_BETA) * q[c + st[d]], b2 = f64(MDCD_BETA) * q[c + 2 * st[d]];
+            f64* o = aux + (AX_DD + 10 * d + 2 * k) * nc + c;
+            o[0] = mdcd_dd(b0, b1, b2);
+            o[nc] = mdcd_dd(b2, b1, b0);
+        }
+    }
+}
+
 // FP32 copies of FP64 slot ranges over every padded cell (mixed path)
 __global__ void k_mirror(const DevBlock* __restrict__ blks, int nblk, long long total, const long long* __restrict__ off,
                          MirrorList ml) {
@@ -477,7 +535,7 @@ __global__ void k_mirror(const DevBlock* __restrict__ blks, int nblk, long long 
 // ---------------------------------------------------------------------------------------
 // Space/DIFF_DqDxyz.F90:25-74, 232-265, 300-381 (gradients and shock sensor, interior cells)
 // ---------------------------------------------------------------------------------------
-template <typename R>
+template <typename R, bool TERMS = false>
 __global__ void k_gradient(const DevBlock* __restrict__ blks, const Tile* __restrict__ tiles, const CaseDev* __restrict__ cdev) {
     const Tile t = tiles[blockIdx.x];
     if ((int)threadIdx.x >= t.count) return;
@@ -502,8 +560,14 @@ __global__ void k_gradient(const DevBlock* __restrict__ blks, const Tile* __rest
         for (int d = 0; d < 3; ++d) {
             const R* al = rs<R>(b, S_ALAGM + d);
             const R* ai = rs<R>(b, S_AINV + d);
-            fw[d] = favg(qs[q], al, ai, c, st[d]);
-            fe[d] = favg(qs[q], al, ai, c + st[d], st[d]);
+            if constexpr (TERMS) {
+                const R* f = reinterpret_cast<const R*>(b.aux) + (size_t)(AX_FA + 7 * d + q) * b.ncell;
+                fw[d] = f[c];
+                fe[d] = f[c + st[d]];
+            } else {
+                fw[d] = favg(qs[q], al, ai, c, st[d]);
+                fe[d] = favg(qs[q], al, ai, c + st[d], st[d]);
+            }
         }
         for (int m = 0; m < 3; ++m) {
             const R* S1 = SD + (size_t)(0 * 3 + m) * b.ncell;
@@ -676,9 +740,18 @@ __global__ void k_bc_grad(const DevBlock* __restrict__ blks, const BCEntry* __re
 // ---------------------------------------------------------------------------------------
 template <typename R>
 struct FaceGlobal {
+    static constexpr bool TERMS = false;
     const DevBlock& b;
     int c, s;
     __device__ R v(int slot, int o) const { return R(rs<R>(b, slot)[c + o * s]); }
+};
+// the same with the terms that faces share (k_face_terms): q.aux(m, o), term m of that cell
+struct FaceTerms {
+    static constexpr bool TERMS = true;
+    const DevBlock& b;
+    int c, s;
+    __device__ f64 v(int slot, int o) const { return rs<f64>(b, slot)[c + o * s]; }
+    __device__ f64 aux(int m, int o) const { return reinterpret_cast<const f64*>(b.aux)[(size_t)m * b.ncell + c + o * s]; }
 };
 
 // PART 0: every flux; 1: the viscous and k-omega diffusion fluxes only; 2: the convective ones
@@ -687,7 +760,15 @@ __device__ __forceinline__ void face_flux_body(const int DIR, const ParamsT<R>& 
     const int d = DIR - 1;
     const int AL = S_ALAGM + d, AIN = S_AINV + d, SDD = S_SD + 3 * d;
     // face average of a slot at the face o steps from this one (SPACEINTERP_GetSurfCenterVars)
-    auto fa = [&](int slot, int o) { return (q.v(AL, o) * q.v(slot, o - 1) + q.v(AL, o - 1) * q.v(slot, o)) * q.v(AIN, o); };
+    auto fa_here = [&](int slot, int o) { return (q.v(AL, o) * q.v(slot, o - 1) + q.v(AL, o - 1) * q.v(slot, o)) * q.v(AIN, o); };
+    auto fa = [&](int slot, int o) -> R {
+        if constexpr (A::TERMS) {
+            const int v = slot == S_T ? 3 : slot == S_PP ? 6 : slot < S_PRIM + 3 ? slot - S_PRIM : slot - S_PRIM + 1;
+            return q.aux(AX_FA + 7 * d + v, o);
+        } else {
+            return fa_here(slot, o);
+        }
+    };
     if constexpr (PART != 2) {
     // ---------------- viscous flux (DIFFUSION_Centered) ----------------
     const bool wall = q.v(S_WALL + d, 0) != R(0.0);
@@ -835,6 +916,10 @@ __device__ __forceinline__ void face_flux_body(const int DIR, const ParamsT<R>& 
             if (muscl) {
                 qL[k] = s6[2] + R(0.5) * alimiter(s6[3] - s6[2], s6[2] - s6[1]);
                 qR[k] = s6[3] - R(0.5) * alimiter(s6[3] - s6[2], s6[4] - s6[3]);
+            } else if constexpr (A::TERMS) {
+                const int pk = AX_PR + NMP * k, dk = AX_DD + 10 * d + 2 * k;
+                mdcd_states(s6, gama, [&](int m, int o) { return q.aux(pk + m, o - 3); }, [&](int o) { return q.aux(dk, o - 3); },
+                            [&](int o) { return q.aux(dk + 1, o - 3); }, qL[k], qR[k]);
             } else {
                 mdcd_pair(s6, gama, qL[k], qR[k]);
             }
@@ -864,7 +949,7 @@ __device__ __forceinline__ void face_flux_body(const int DIR, const ParamsT<R>& 
         R rl, rr;
         if (p.Kind_Spatial <= 2) {
             const bool m2 = p.Kind_Spatial == 1;
-            R fm = fa(S_RAD, -1), f0 = fa(S_RAD, 0), fp = fa(S_RAD, 1);
+            R fm = fa_here(S_RAD, -1), f0 = fa_here(S_RAD, 0), fp = fa_here(S_RAD, 1);
             R q1 = q.v(S_RAD, -1), q0 = q.v(S_RAD, 0);
             R DR = f0 - q1, DL = q1 - fm;
             rl = q1 + (m2 ? muscl2_limiter(DR, DL) : alimiter(DR, DL));
@@ -876,7 +961,7 @@ __device__ __forceinline__ void face_flux_body(const int DIR, const ParamsT<R>& 
             for (int o = 0; o < 6; ++o) s6[o] = q.v(S_RAD, o - 3);
             mdcd_pair(s6, gama, rl, rr);
         } else {
-            rl = fa(S_RAD, 0);
+            rl = fa_here(S_RAD, 0);
             rr = rl;
         }
         rLo = rl * R(p.omega0);
@@ -896,7 +981,7 @@ __device__ __forceinline__ void face_flux_body(const int DIR, const ParamsT<R>& 
         if (p.Kind_Roe == 1) {
             // preconditioning reads VL(d,8), the face-averaged eddy viscosity (0 while turbulence
             // is off), and Alagm(d) of the face's cell (Space/CONVECT_Roe_Original.F90:86-87)
-            const R RmiuTf = (p.IF_Precondition && turb) ? fa(S_RMIU, 0) : R(0.0);
+            const R RmiuTf = (p.IF_Precondition && turb) ? fa_here(S_RMIU, 0) : R(0.0);
             roe_flux<R>(p, qL[3], qR[3], qL[4], qR[4], qL[0], qR[0], qL[1], qR[1], qL[2], qR[2], sav1, sav2, sav3, sav, rLo, rRo,
                         f, RmiuTf, q.v(AL, 0));
         } else
@@ -936,7 +1021,7 @@ __device__ __forceinline__ void face_flux_body(const int DIR, const ParamsT<R>& 
 // three launches ran one after the other (us per iteration, three launches -> one of each part:
 // 1,920-cell channel FP64 257 -> 86, 352,256-cell cascade FP64 3,019 -> 2,884 and mixed 132 -> 97,
 // 1,966,080-cell cascade FP64 15,670 -> 15,617 and mixed 629 -> 617)
-template <typename R, int PART = 0>
+template <typename R, int PART = 0, class A = FaceGlobal<R>>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (PART == 1 ? TG_FACE_MINB_VISC : TG_FACE_MINB) : (PART == 0 ? 1 : 3)) k_face_flux(const DevBlock* __restrict__ blks, const Tile* __restrict__ tiles,
                                                           const CaseDev* __restrict__ cdev) {
     const Tile t = tiles[blockIdx.x];
@@ -950,7 +1035,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (PART == 1 ? TG_FACE_MIN
     int i = n % ni + 1, j = (n / ni) % nj + 1, k = n / (ni * nj) + 1;
     const int s = DIR == 1 ? 1 : (DIR == 2 ? b.PI : b.PI * b.PJ);
     const int c = cidx(b, i, j, k);
-    const FaceGlobal<R> q{b, c, s};
+    const A q{b, c, s};
     R F[NFX];
     face_flux_body<R, PART>(DIR, p, turb, q, F);
     const size_t nc = (size_t)b.ncell;

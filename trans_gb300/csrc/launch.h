@@ -19,6 +19,8 @@ void launch_bc_state(cudaStream_t s, const DevBlock* blks, const BCEntry* ent, i
 void launch_bc_outlet(cudaStream_t s, const DevBlock* blks, const BCEntry* ent, const OutletLine* lines, int nl,
                       const CaseDev* cdev);
 void launch_prims(cudaStream_t s, const DevBlock* blks, int nblk, long long total, const long long* off);
+void launch_face_terms(cudaStream_t s, const DevBlock* blks, int nblk, long long total, const long long* off, const CaseDev* cdev,
+                       int mdcd);
 void launch_update(cudaStream_t s, const DevBlock* blks, const Tile* tiles, int nt, const CaseDev* cdev, NormPart* parts,
                    int d_fp32);
 void launch_block_norms(cudaStream_t s, const DevBlock* blks, int nblk, const NormPart* parts, const int* tile_first,
@@ -96,10 +98,11 @@ constexpr int MARCH_EDGES = 4;
 
 // flux, source and sweep kernels, instantiated per arithmetic type
 struct FluxLaunchers {
-    void (*gradient)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*);
+    // terms: the FP64 kernels read the terms that launch_face_terms left (AuxTerm)
+    void (*gradient)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*, bool terms);
     void (*shock_ghost)(cudaStream_t, const DevBlock*, const Tile*, int);
     void (*bc_grad)(cudaStream_t, const DevBlock*, const BCEntry*, int);
-    void (*face_flux)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*);
+    void (*face_flux)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*, bool terms);
     void (*gather)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*);
     void (*sst_fc1)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*);
     // cross-rank 1-to-1 segment: words (host-built table, device staging) into the ghost layers

@@ -69,6 +69,7 @@ __host__ __device__ constexpr int rt_offset(int field) {       // first float of
 // offset outside the staged range, is read from the slot arrays
 template <int DIR>
 struct FaceTile {
+    static constexpr bool TERMS = false;
     const float* sm;
     const DevBlock& b;
     int c, s, pos;

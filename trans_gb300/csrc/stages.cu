@@ -528,7 +528,7 @@ int tune_resid(Ctx* c) {
                 launch_resid_tma(d + 1, s, c->d_blk, c->d_rtiles[d], c->n_rtiles[d], c->d_cdev, c->d_rmaps, c->d_kerr,
                                  c->resid_spin);
         } else {
-            c->fl->face_flux(s, c->d_blk, c->d_face, (int)c->face_tiles.size(), c->d_cdev);
+            c->fl->face_flux(s, c->d_blk, c->d_face, (int)c->face_tiles.size(), c->d_cdev, false);
             c->fl->gather(s, c->d_blk, c->d_cell, nct, c->d_cdev);
         }
     };
@@ -572,7 +572,8 @@ namespace {
 
 // One stage.  capture: inside a CUDA-graph capture (no host synchronisation, no parameter
 // upload, the norms go to history slot `slot`).
-int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot) {
+// seq: the stage is one of a whole iteration's, with nothing between it and the stages before
+int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot, bool seq) {
     if (c->cases.empty()) return fail(c, TRANS_E_ARG, "no case");
     int rc;
     if (!capture) {
@@ -610,7 +611,13 @@ int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot) {
                 KScope t(c, K_PRIMS);
                 launch_prims(s, c->d_blk, (int)c->blk.size(), c->total_cells, c->d_off);
             }
-            { KScope t(c, K_GRADIENT); c->fl->gradient(s, c->d_blk, c->d_cell, nct, c->d_cdev); }
+            // the face averages, and with an iteration to follow the fluxes' other shared terms
+            if (c->d_aux) {
+                KScope t(c, K_FACE);
+                launch_face_terms(s, c->d_blk, (int)c->blk.size(), c->total_cells, c->d_off, c->d_cdev, seq);
+                c->launches++;
+            }
+            { KScope t(c, K_GRADIENT); c->fl->gradient(s, c->d_blk, c->d_cell, nct, c->d_cdev, c->d_aux != nullptr); }
             { KScope t(c, K_SHOCK_GHOST); c->fl->shock_ghost(s, c->d_blk, c->d_ghost, (int)c->ghost_tiles.size()); }
             c->launches += 3;
             break;
@@ -633,8 +640,13 @@ int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot) {
             }
             {
                 // the viscous and the convective fluxes of every direction are a launch each
-                KScope t(c, K_FACE, 2);
-                c->fl->face_flux(s, c->d_blk, c->d_face, (int)c->face_tiles.size(), c->d_cdev);
+                const bool terms = c->d_aux != nullptr;
+                KScope t(c, K_FACE, terms && !seq ? 3 : 2);
+                if (terms && !seq) {           // the caller may have changed the state since the gradient stage
+                    launch_face_terms(s, c->d_blk, (int)c->blk.size(), c->total_cells, c->d_off, c->d_cdev, 1);
+                    c->launches++;
+                }
+                c->fl->face_flux(s, c->d_blk, c->d_face, (int)c->face_tiles.size(), c->d_cdev, terms);
             }
             { KScope t(c, K_GATHER); c->fl->gather(s, c->d_blk, c->d_cell, nct, c->d_cdev); }
             c->launches += 3;
@@ -714,7 +726,7 @@ int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot) {
 
 }  // namespace
 
-int run_stage(Ctx* c, int stage, int itr) { return stage_exec(c, stage, itr, false, 0); }
+int run_stage(Ctx* c, int stage, int itr) { return stage_exec(c, stage, itr, false, 0, false); }
 
 // One outer iteration (main.F90:54-171 + :192-197) of every case at its current KI.
 int run_iteration(Ctx* c) {
@@ -724,7 +736,7 @@ int run_iteration(Ctx* c) {
     int rc = TRANS_OK;
     for (int it = 1; it <= nsub && rc == TRANS_OK; ++it)
         for (int st = TRANS_STAGE_SPECRAD; st <= TRANS_STAGE_UPDATE && rc == TRANS_OK; ++st)
-            rc = run_stage(c, st, it);
+            rc = stage_exec(c, st, it, false, 0, true);
     if (rc == TRANS_OK) rc = run_stage(c, TRANS_STAGE_UPDATE_U, nsub);
     if (rc != TRANS_OK && rc != TRANS_E_NAN) return rc;
     for (CaseRec* cs : c->cases) {               // a NaN iteration still has its norms
@@ -770,8 +782,8 @@ int capture_iterations(Ctx* c, int n) {
     for (int q = 0; q < n && rc == TRANS_OK; ++q) {
         for (int it = 1; it <= nsub && rc == TRANS_OK; ++it)
             for (int st = TRANS_STAGE_SPECRAD; st <= TRANS_STAGE_UPDATE && rc == TRANS_OK; ++st)
-                rc = stage_exec(c, st, it, true, q);
-        if (rc == TRANS_OK) rc = stage_exec(c, TRANS_STAGE_UPDATE_U, nsub, true, q);
+                rc = stage_exec(c, st, it, true, q, true);
+        if (rc == TRANS_OK) rc = stage_exec(c, TRANS_STAGE_UPDATE_U, nsub, true, q, true);
     }
     if (rc == TRANS_OK) {
         cudaMemcpyAsync(c->h_norms, c->d_norms, sizeof(BlockNorms) * (size_t)nblk * n, cudaMemcpyDeviceToHost, s);

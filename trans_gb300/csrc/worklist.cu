@@ -299,6 +299,30 @@ int build_march(Ctx* c) {
     return TRANS_OK;
 }
 
+// Memory for the FP64 face fluxes' shared terms, after everything else of the context has its own:
+// within the budget that is left, and within a quarter of the free device memory (the fluxes form the
+// terms themselves without it)
+int build_terms(Ctx* c) {
+    if (c->mixed) return TRANS_OK;
+    auto entries = [&](const DevBlock& b) { return c->cases[b.cs]->p.Kind_Spatial > 2 ? AX_MDCD : AX_MUSCL; };
+    size_t n = 0, free_b = 0, total_b = 0;
+    for (const DevBlock& b : c->blk) n += (size_t)b.ncell * entries(b);
+    const size_t bytes = n * sizeof(double);
+    if (c->budget > 0 && c->in_use + (long long)bytes > c->budget) return TRANS_OK;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 4 || cudaMalloc(&c->d_aux, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        c->d_aux = nullptr;
+        return TRANS_OK;
+    }
+    size_t at = 0;
+    for (DevBlock& b : c->blk) {
+        b.aux = c->d_aux + at;
+        at += (size_t)b.ncell * entries(b);
+    }
+    CK(cudaMemcpyAsync(c->d_blk, c->blk.data(), sizeof(DevBlock) * c->blk.size(), cudaMemcpyHostToDevice, c->stream));
+    return TRANS_OK;
+}
+
 }  // namespace
 
 int rebuild(Ctx* c) {
@@ -476,6 +500,7 @@ int rebuild(Ctx* c) {
     if (c->march) c->sweep_mode = 6;
     else if (!c->sweep_forced && (c->sweep_mode == 6 || c->tuned_positions <= 0 || npos > 2 * c->tuned_positions || 2 * npos < c->tuned_positions))
         c->sweep_mode = -1;
+    if ((rc = build_terms(c))) return rc;
     c->built = true;
     return TRANS_OK;
 }
