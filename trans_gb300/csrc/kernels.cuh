@@ -1062,6 +1062,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (PART == 1 ? TG_FACE_MIN
 // D of every interior cell in the reference's accumulation order (main.F90:92-133):
 //   D = 0 - Fv(i) + Fv(i+1) - Fv(j) + Fv(j+1) - Fv(k) + Fv(k+1) - Fc(i) + Fc(i+1) - ...
 // ---------------------------------------------------------------------------------------
+// (the sums unrolled, so that their loads go out together: mixed, 352,256 cells 28 -> 22 us, 1,966,080
+// cells 98 -> 88)
 template <typename R>
 __global__ void k_gather(const DevBlock* __restrict__ blks, const Tile* __restrict__ tiles, const CaseDev* __restrict__ cdev) {
     const Tile t = tiles[blockIdx.x];
@@ -1074,39 +1076,38 @@ __global__ void k_gather(const DevBlock* __restrict__ blks, const Tile* __restri
     const int st[3] = {1, b.PI, b.PI * b.PJ};
     const size_t nc = (size_t)b.ncell;
     const R* FX = rs<R>(b, S_FX);
-    auto fx = [&](int d, int m, int cc) { return R(FX[(size_t)(NFX * d + m) * nc + cc]); };
-    {   // rho: no viscous flux
-        R acc = R(0.0);
-        for (int d = 0; d < 3; ++d) { acc = acc - fx(d, FX_C0, c); acc = acc + fx(d, FX_C0, c + st[d]); }
-        rs<R>(b, S_D)[c] = acc;
-    }
-    // rotating-frame source of DIFFUSION_Centered (:812-822), after its viscous terms: Coriolis
-    // and centrifugal force on y and z momentum times the cell volume.  With omega(1) = 0 it adds
-    // a signed zero, which leaves a sum that started at +0 unchanged, so it is skipped.
     const R om = cparams<R>(cdev[b.cs]).omega0;
-    for (int L = 1; L < 5; ++L) {
+#pragma unroll
+    for (int L = 0; L < 7; ++L) {
         R acc = R(0.0);
-        for (int d = 0; d < 3; ++d) { acc = acc - fx(d, FX_VX + L - 1, c); acc = acc + fx(d, FX_VX + L - 1, c + st[d]); }
-        if ((L == 2 || L == 3) && om != R(0.0)) {
-            const R* V = rs<R>(b, S_V);
-            const R V1 = R(V[c]);
-            const R ss = L == 2 ? R(2.0) * om * R(V[3 * nc + c]) + om * R(rs<R>(b, S_YC)[c]) * om * V1
-                                : R(-2.0) * om * R(V[2 * nc + c]) + om * R(rs<R>(b, S_ZC)[c]) * om * V1;
-            acc = acc + ss * R(rs<R>(b, S_VOL)[c]);
+        auto add = [&](int m) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const R* f = FX + (size_t)(NFX * d + m) * nc;
+                acc = acc - R(f[c]);
+                acc = acc + R(f[c + st[d]]);
+            }
+        };
+        if (L == 0) {           // rho: no viscous flux
+            add(FX_C0);
+        } else if (L < 5) {
+            add(FX_VX + L - 1);
+            // rotating-frame source of DIFFUSION_Centered (:812-822), after its viscous terms: Coriolis
+            // and centrifugal force on y and z momentum times the cell volume.  With omega(1) = 0 it adds
+            // a signed zero, which leaves a sum that started at +0 unchanged, so it is skipped.
+            if ((L == 2 || L == 3) && om != R(0.0)) {
+                const R* V = rs<R>(b, S_V);
+                const R V1 = R(V[c]);
+                const R ss = L == 2 ? R(2.0) * om * R(V[3 * nc + c]) + om * R(rs<R>(b, S_YC)[c]) * om * V1
+                                    : R(-2.0) * om * R(V[2 * nc + c]) + om * R(rs<R>(b, S_ZC)[c]) * om * V1;
+                acc = acc + ss * R(rs<R>(b, S_VOL)[c]);
+            }
+            add(FX_C0 + L);
+        } else if (turb) {
+            add(FX_TK + L - 5);
+            add(FX_CK + L - 5);
         }
-        for (int d = 0; d < 3; ++d) { acc = acc - fx(d, FX_C0 + L, c); acc = acc + fx(d, FX_C0 + L, c + st[d]); }
         rs<R>(b, S_D + L)[c] = acc;
-    }
-    if (turb) {
-        for (int q = 0; q < 2; ++q) {
-            R acc = R(0.0);
-            for (int d = 0; d < 3; ++d) { acc = acc - fx(d, FX_TK + q, c); acc = acc + fx(d, FX_TK + q, c + st[d]); }
-            for (int d = 0; d < 3; ++d) { acc = acc - fx(d, FX_CK + q, c); acc = acc + fx(d, FX_CK + q, c + st[d]); }
-            rs<R>(b, S_D + 5 + q)[c] = acc;
-        }
-    } else {
-        rs<R>(b, S_D + 5)[c] = R(0.0);
-        rs<R>(b, S_D + 6)[c] = R(0.0);
     }
 }
 
@@ -1231,11 +1232,15 @@ __device__ inline R rc_fr1(const ParamsT<R>& p, const DevBlock& b, int I, int J,
 
 // (FP32: two resident CTAs of 256 threads per SM, i.e. at most 128 registers)
 #ifndef TG_PREP_MINB
-#define TG_PREP_MINB 3      // resident CTAs per SM of the FP32 preparation (84 registers, 80-byte spill)
+#define TG_PREP_MINB 3      // resident CTAs per SM of the FP32 preparation (128 registers; 3 CTAs: 82 against 70 us at 352,256 cells)
 #endif
 #ifndef TG_PREP_MINB_F64
-#define TG_PREP_MINB_F64 2  // ... and of the FP64 one (128 registers, 84-byte spill; 254 at one CTA per SM)
+#define TG_PREP_MINB_F64 2  // ... and of the FP64 one (128 registers, 100-byte spill; at one CTA 2,377 against 2,020 us at 1,966,080)
 #endif
+// Bound by load latency at its registers; the FP32 right-hand sides leave in two 16-byte words of a cell
+// (in the marching order neighbouring cells lie 1 KB apart, so each 4-byte word was a sector of its own):
+// 352,256 cells 59 -> 51 us, 1,966,080 cells 268 -> 225, a batch of five cascades 381 -> 312.  Summing the
+// face fluxes here, without k_gather, took 342 us where the two take 313.
 template <typename R>
 __global__ void __launch_bounds__(CELL_TILE, sizeof(R) == 4 ? TG_PREP_MINB : TG_PREP_MINB_F64) k_lusgs_prep(const DevBlock* __restrict__ blks, const Tile* __restrict__ tiles, const int* __restrict__ qpos,
                              R* __restrict__ rec, R* __restrict__ dq, const CaseDev* __restrict__ cdev, int march) {
@@ -1251,7 +1256,16 @@ __global__ void __launch_bounds__(CELL_TILE, sizeof(R) == 4 ? TG_PREP_MINB : TG_
     const int c = cidx(b, I, J, K);
     // FP64: in hyperplane order, or that of the marching sweeps (march)
     auto REC = [&](int m) -> R& { return rec[march ? m64_rec(q, m64_diag(m)) : sw_at(q, m, NREC)]; };
-    auto DQ = [&](int L) -> R& { return dq[sizeof(R) == 8 && march ? m64_dq(q, L) : sw_at(q, L, DQ_STRIDE)]; };
+    R DQ[7];                                       // the right-hand sides, stored by put(first, last)
+    auto put = [&](int l0, int l1) {
+        if constexpr (sizeof(R) == 4) {            // four at a time: 0-3, and 4-6 with the unused eighth
+            float4* d = reinterpret_cast<float4*>(dq) + (size_t)q * (DQ_STRIDE / 4);
+            if (l0 == 0) d[0] = make_float4(DQ[0], DQ[1], DQ[2], DQ[3]);
+            else d[1] = make_float4(DQ[4], DQ[5], DQ[6], 0.0f);
+        } else {
+            for (int L = l0; L < l1; ++L) dq[march ? m64_dq(q, L) : sw_at(q, L, DQ_STRIDE)] = DQ[L];
+        }
+    };
     // BDF2 right-hand side and the mean-flow diagonal (TIME_LUSGS.F90:73-108).  FP64 path: the
     // reference's operations.  Mixed path: the time-level difference 3V - 4Wt0 + Wt1 in FP64
     // (it cancels), everything else in FP32 with one reciprocal of the volume.  (This kernel is
@@ -1285,6 +1299,7 @@ __global__ void __launch_bounds__(CELL_TILE, sizeof(R) == 4 ? TG_PREP_MINB : TG_
     // record of this position (CompactRec: metric and radius per direction, velocity and total
     // enthalpy, stept, cvs and the reciprocals of the two diagonals)
     auto finish = [&](R ft) {
+        put(MIXED ? 4 : 5, 7);
         if constexpr (MIXED) {
             float4* R4 = reinterpret_cast<float4*>(rec) + (size_t)q * (NCREC / 4);
 #pragma unroll
@@ -1302,22 +1317,24 @@ __global__ void __launch_bounds__(CELL_TILE, sizeof(R) == 4 ? TG_PREP_MINB : TG_
             REC(REC_FT) = ft;
         }
     };
-    for (int L = 0; L < 5; ++L) DQ(L) = rhs(L);
+#pragma unroll
+    for (int L = 0; L < 5; ++L) DQ[L] = rhs(L);
     if constexpr (!MIXED) {
         if (pd.IF_Precondition) {     // the right-hand side preconditioned (TIME_LUSGS.F90:113-160)
-            R A[5] = {DQ(0), DQ(1), DQ(2), DQ(3), DQ(4)}, tpc[NPC];
+            R tpc[NPC];
             precond_terms_at(p, b, c, tpc);
-            precond_apply<R>(A, tpc);
-            for (int L = 0; L < 5; ++L) DQ(L) = A[L];
+            precond_apply<R>(DQ, tpc);
         }
     }
+    put(0, 5);
     if (!turb) {            // the k-omega lanes of the sweeps then produce zeros
-        DQ(5) = rs<R>(b, S_D + 5)[c];
-        DQ(6) = rs<R>(b, S_D + 6)[c];
+        DQ[5] = rs<R>(b, S_D + 5)[c];
+        DQ[6] = rs<R>(b, S_D + 6)[c];
         finish(R(1.0));
         return;
     }
-    for (int L = 5; L < 7; ++L) DQ(L) = rhs(L);
+#pragma unroll
+    for (int L = 5; L < 7; ++L) DQ[L] = rhs(L);
     auto G = [&](int q) { return rs<R>(b, S_DQ + q)[c]; };
     R dudx = G(0), dudy = G(1), dudz = G(2), dvdx = G(3), dvdy = G(4), dvdz = G(5), dwdx = G(6), dwdy = G(7), dwdz = G(8);
     R dtkdx = G(12), dtkdy = G(13), dtkdz = G(14), dtodx = G(15), dtody = G(16), dtodz = G(17);
@@ -1334,7 +1351,7 @@ __global__ void __launch_bounds__(CELL_TILE, sizeof(R) == 4 ? TG_PREP_MINB : TG_
     if (p.Kind_Model == 2) {    // Wilcox 2006 k-omega (TURBTWO_TIME_LUSGS_SST.F90:418-547)
         const R c23 = R(2.0 / 3.0);
         R SourceN1 = -(c23 * dmax(Div, R(0.0))) - Bs * ARTO / ARo * Ref;
-        DQ(5) = DQ(5) + ((tprod - c23 * dmin(Div, R(0.0)) * ARTk) + SourceN1 * ARTk);
+        DQ[5] = DQ[5] + ((tprod - c23 * dmin(Div, R(0.0)) * ARTk) + SourceN1 * ARTk);
         const R CnegTk = fabs(SourceN1);
         tprod = dmin(prod, Votg) / Ref;
         const R h = R(0.5);
@@ -1358,7 +1375,7 @@ __global__ void __launch_bounds__(CELL_TILE, sizeof(R) == 4 ? TG_PREP_MINB : TG_
         R Source = SourceP + SourceN1 * ARTO;
         R dltCD = cdif <= R(0.) ? R(0.) : R(0.125);
         Source = Source + dltCD * ARo * ARo / ARTO / Ref * cdif;
-        DQ(6) = DQ(6) + Source;
+        DQ[6] = DQ[6] + Source;
         finish(R(fm) + (CnegTk + R(2.0) * fabs(SourceN1)) * R(stept));
         return;
     }
@@ -1431,7 +1448,7 @@ __global__ void __launch_bounds__(CELL_TILE, sizeof(R) == 4 ? TG_PREP_MINB : TG_
         CnegTk = fabs(-(c23 * dmax(Div, R(0.0))) - R(1.5) * sqrt(ARTk / ARo) / alIDDES);
         if (p.If_fix_Transition && rs<R>(b, S_XC)[c] < p.Trans_location) Source = R(0.0);
     }
-    DQ(5) = DQ(5) + Source;
+    DQ[5] = DQ[5] + Source;
     tprod = dmin(prod, Votg) / Ref;
     R GamaAB = R(p.Gama1) * arg1 + R(p.Gama2) * (R(1.0) - arg1);
     R BetaAB = R(p.Beta1) * arg1 + R(p.Beta2) * (R(1.0) - arg1);
@@ -1448,7 +1465,7 @@ __global__ void __launch_bounds__(CELL_TILE, sizeof(R) == 4 ? TG_PREP_MINB : TG_
     R SourceCross = R(2.0) * (R(1) - arg1) * ARo * Sigo2 / (ARTO / ARo) * cdif / Ref;
     SourceCross = sgn1(SourceCross) * dmin(fabs(SourceCross), fabs(SourceP) * R(0.5));
     Source = Source + SourceCross;
-    DQ(6) = DQ(6) + Source;
+    DQ[6] = DQ[6] + Source;
     CnegTO = R(2.0) * fabs(SourceN1);
     finish(R(fm) + (CnegTk + CnegTO) * R(stept));
 }
@@ -2086,9 +2103,16 @@ __global__ void k_sweep_scatter(const DevBlock* __restrict__ blks, const Tile* _
     const int I = n % b.NI1 + 1, J = (n / b.NI1) % b.NJ1 + 1, K = n / (b.NI1 * b.NJ1) + 1;
     const int c = cidx(b, I, J, K);
     const long long q = qpos[(size_t)blockIdx.x * CELL_TILE + threadIdx.x];
-    R d[7];
+    R d[8];
+    if constexpr (sizeof(R) == 4) {                // two 16-byte words of a place: 39 us at 1,966,080 cells, 63 word by word
+        const float4* w = reinterpret_cast<const float4*>(dq) + (size_t)q * (DQ_STRIDE / 4);
+        const float4 x = w[0], y = w[1];
+        d[0] = x.x; d[1] = x.y; d[2] = x.z; d[3] = x.w;
+        d[4] = y.x; d[5] = y.y; d[6] = y.z;
+    } else {
 #pragma unroll
-    for (int L = 0; L < 7; ++L) d[L] = L >= l0 ? dq[sizeof(R) == 8 && march ? m64_dq(q, L) : sw_at(q, L, DQ_STRIDE)] : R(0);
+        for (int L = 0; L < 7; ++L) d[L] = L >= l0 ? dq[march ? m64_dq(q, L) : sw_at(q, L, DQ_STRIDE)] : R(0);
+    }
 #pragma unroll
     for (int L = 0; L < 7; ++L)
         if (L >= l0) rs<R>(b, S_D + L)[c] = d[L];
