@@ -17,33 +17,49 @@ namespace tg {
 // |D/V| and the NaN flag.  A CTA reduces them by warp shuffles -- lane l takes lane l+w for
 // w = 16, 8, 4, 2, 1 -- then warp 0 over the warps' results, a fixed order.  The maximum of
 // |D1/V1| keeps the later cell on ties (IF(DUa<=DR), :135).
+//
+// Bound by the FP64 pipe, where an instruction costs a warp 63 cycles however few lanes need it:
+// maxima and ties are integer comparisons, and the three sums share the lanes that the tree frees (6
+// additions a warp instead of 15, and no comparison of 20).  Update with its norms, before and now:
+// 24x16x5 cells FP64 51 and 45 us, 1,966,080 cells FP64 1,407 and 1,319; 96x48x8 cells mixed 22.5 and
+// 18.5, 1,966,080 cells mixed 147 and 141.
 // ---------------------------------------------------------------------------------------
 __device__ inline NormPart norm_identity() {
     NormPart a;
     a.sa = 0; a.ma = -1; a.sk = 0; a.mk = 0; a.so = 0; a.mo = 0; a.ia = -1; a.nan = 0; a.pad_ = 0;
     return a;
 }
-__device__ inline void norm_join(NormPart& a, const NormPart& b) {
-    a.sa += b.sa; a.sk += b.sk; a.so += b.so;
-    if (b.ma > a.ma || (b.ma == a.ma && b.ia > a.ia)) { a.ma = b.ma; a.ia = b.ia; }
-    a.mk = dmax(a.mk, b.mk); a.mo = dmax(a.mo, b.mo);
+// the maxima and the flag of b into a
+__device__ inline void norm_join_max(NormPart& a, const NormPart& b) {
+    if (sx::less(a.ma, b.ma) || (sx::equal(b.ma, a.ma) && b.ia > a.ia)) { a.ma = b.ma; a.ia = b.ia; }
+    if (sx::less(a.mk, b.mk)) a.mk = b.mk;
+    if (sx::less(a.mo, b.mo)) a.mo = b.mo;
     a.nan |= b.nan;
 }
-__device__ inline NormPart norm_shfl_down(const NormPart& a, int w) {
-    const unsigned full = 0xffffffffu;
-    NormPart b;
-    b.sa = __shfl_down_sync(full, a.sa, w); b.ma = __shfl_down_sync(full, a.ma, w);
-    b.sk = __shfl_down_sync(full, a.sk, w); b.mk = __shfl_down_sync(full, a.mk, w);
-    b.so = __shfl_down_sync(full, a.so, w); b.mo = __shfl_down_sync(full, a.mo, w);
-    b.ia = __shfl_down_sync(full, a.ia, w); b.nan = __shfl_down_sync(full, a.nan, w);
-    b.pad_ = 0;
-    return b;
-}
+// the warp's reduction, valid in lane 0
 __device__ inline NormPart norm_reduce_warp(NormPart a) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
     for (int w = 16; w > 0; w >>= 1) {
-        const NormPart o = norm_shfl_down(a, w);
-        if ((int)(threadIdx.x & 31) + w < 32) norm_join(a, o);
+        NormPart b;
+        b.ma = __shfl_down_sync(full, a.ma, w);
+        b.mk = __shfl_down_sync(full, a.mk, w);
+        b.mo = __shfl_down_sync(full, a.mo, w);
+        b.ia = __shfl_down_sync(full, a.ia, w);
+        b.nan = __shfl_down_sync(full, a.nan, w);
+        if (lane + w < 32) norm_join_max(a, b);
     }
+    // sums of lanes l and l + 16: sa in lanes 0-15, sk in 16-31; so in both halves
+    const bool hi = lane & 16, odd = lane & 8;
+    const double p = (hi ? a.sk : a.sa) + __shfl_xor_sync(full, hi ? a.sa : a.sk, 16);
+    const double q = a.so + __shfl_xor_sync(full, a.so, 16);
+    // of l and l + 8: sa in lanes 0-7, so in 8-15, sk in 16-23
+    double r = (odd ? q : p) + __shfl_xor_sync(full, odd ? p : q, 8);
+    for (int w = 4; w > 0; w >>= 1) r += __shfl_xor_sync(full, r, w);
+    a.sa = __shfl_sync(full, r, 0);
+    a.so = __shfl_sync(full, r, 8);
+    a.sk = __shfl_sync(full, r, 16);
     return a;
 }
 // the CTA's reduction, valid in thread 0 (blockDim a multiple of 32); every thread calls it
@@ -2196,7 +2212,7 @@ __global__ void k_update(const DevBlock* __restrict__ blks, const Tile* __restri
         auto Dq = [&](int L) { return d_fp32 ? f64((double)fslot(b, S_D + L)[c]) : rs<f64>(b, S_D + L)[c]; };
         f64 d1 = Dq(0), d6 = Dq(5), d7 = Dq(6);
         f64 DR = fabs(d1 / v1);
-        nanf = isnan(d1.v) ? 1 : 0;
+        nanf = sx::is_nan(d1.v) ? 1 : 0;
         sa = (DR * DR).v; ma = DR.v; ia = n;
         f64 DRk = fabs(d6 / v1), DRo = fabs(d7 / v1);
         sk = (DRk * DRk).v; mk = DRk.v; so = (DRo * DRo).v; mo = DRo.v;
@@ -2286,7 +2302,7 @@ __global__ void k_rk_update(const DevBlock* __restrict__ blks, const Tile* __res
         auto Dq = [&](int L) { return d_fp32 ? f64((double)fslot(b, S_D + L)[c]) : rs<f64>(b, S_D + L)[c]; };
         const f64 d1 = Dq(0);
         const f64 DR = fabs(d1 / rs<f64>(b, S_V)[c]);
-        nanf = isnan(d1.v) ? 1 : 0;
+        nanf = sx::is_nan(d1.v) ? 1 : 0;
         sa = (DR * DR).v; ma = DR.v; ia = n;
         const f64 dtm = rs<f64>(b, S_DTM)[c], vol = rs<f64>(b, S_VOL)[c];
         f64 v[5];
@@ -2369,25 +2385,24 @@ __global__ void k_rk_vupdate(const DevBlock* __restrict__ blks, const Tile* __re
 __global__ void k_block_norms(const DevBlock* __restrict__ blks, const NormPart* __restrict__ parts,
                               const int* __restrict__ tile_first, BlockNorms* __restrict__ out) {
     const int bi = blockIdx.x, tid = threadIdx.x;
-    double sa = 0, sk = 0, so = 0, ma = -1, mk = 0, mo = 0;
-    long long ia = 0;
-    int nan = 0;
-    for (int t = tile_first[bi] + tid; t < tile_first[bi + 1]; t += blockDim.x) {
-        const NormPart P = parts[t];
-        sa += P.sa; sk += P.sk; so += P.so;
-        if (P.ma > ma || (P.ma == ma && P.ia > ia)) { ma = P.ma; ia = P.ia; }
-        mk = dmax(mk, P.mk); mo = dmax(mo, P.mo);
-        nan |= P.nan;
-    }
     NormPart P;
-    P.sa = sa; P.ma = ma; P.sk = sk; P.mk = mk; P.so = so; P.mo = mo; P.ia = ia; P.nan = nan; P.pad_ = 0;
+    P.sa = 0; P.ma = -1; P.sk = 0; P.mk = 0; P.so = 0; P.mo = 0; P.ia = 0; P.nan = 0; P.pad_ = 0;
+#pragma unroll 4
+    for (int t = tile_first[bi] + tid; t < tile_first[bi + 1]; t += blockDim.x) {
+        const NormPart A = parts[t];
+        P.sa += A.sa; P.sk += A.sk; P.so += A.so;
+        norm_join_max(P, A);
+    }
     P = norm_reduce_cta(P);
+    if (tid >= 32) return;
+    const DevBlock B = blks[bi];
+    // the three roots side by side, a lane each (every lane of the first warp has the sums)
+    const f64 sum = tid == 0 ? P.sa : tid == 1 ? P.sk : P.so;
+    const double rms = sqrt(sum / f64(B.NI1) / f64(B.NJ1) / f64(B.NK1)).v;
+    const double rms_k = __shfl_sync(0xffffffffu, rms, 1), rms_o = __shfl_sync(0xffffffffu, rms, 2);
     if (tid == 0) {
-        const DevBlock B = blks[bi];
         BlockNorms N;
-        N.DRSa = sqrt(P.sa / B.NI1 / B.NJ1 / B.NK1);
-        N.DRSk = sqrt(P.sk / B.NI1 / B.NJ1 / B.NK1);
-        N.DRSo = sqrt(P.so / B.NI1 / B.NJ1 / B.NK1);
+        N.DRSa = rms; N.DRSk = rms_k; N.DRSo = rms_o;
         N.DUa = P.ma; N.DUk = P.mk; N.DUo = P.mo;
         const long long i0 = P.ia;
         N.Ima = (int)(i0 % B.NI1) + 1; N.Jma = (int)((i0 / B.NI1) % B.NJ1) + 1; N.Kma = (int)(i0 / ((long long)B.NI1 * B.NJ1)) + 1;
