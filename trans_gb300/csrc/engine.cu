@@ -144,6 +144,8 @@ int ctx_init(Ctx* c, int precision, long long budget) {
     c->fl = c->mixed ? &flux_launchers_f32() : &flux_launchers_f64();
     c->budget = budget;
     CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
+    for (cudaStream_t& s : c->side) CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    for (cudaEvent_t* e : {&c->ev_fork, &c->ev_radii, &c->ev_jac, &c->ev_side1}) CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     CK(cudaMalloc(&c->d_sync, sizeof(SweepSync)));
     CK(cudaMallocHost(&c->h_sync, sizeof(SweepSync)));
     std::memset(c->h_sync, 0, sizeof(SweepSync));
@@ -272,6 +274,8 @@ void ctx_free(Ctx* c) {
     if (c->h_kerr) { cudaFreeHost(c->h_kerr); c->h_kerr = nullptr; }
     if (c->copy_done) { cudaEventDestroy(c->copy_done); c->copy_done = nullptr; }
     if (c->stream) { cudaStreamDestroy(c->stream); c->stream = nullptr; }
+    for (cudaStream_t& s : c->side) if (s) { cudaStreamDestroy(s); s = nullptr; }
+    for (cudaEvent_t* e : {&c->ev_fork, &c->ev_radii, &c->ev_jac, &c->ev_side1}) if (*e) { cudaEventDestroy(*e); *e = nullptr; }
 }
 
 CaseRec* case_find(Ctx* c, int id) {

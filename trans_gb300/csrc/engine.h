@@ -113,6 +113,10 @@ struct Ctx {
     struct SweepPair { int p_first, p_count, o_off, o_count; };
     std::vector<SweepPair> pair_lo, pair_up;
     int* d_orph = nullptr;
+    // branches of the captured iterations: side[0] the spectral radii and the sweeps' Jacobian terms,
+    // side[1] the outlets, the convective fluxes, the norms
+    cudaStream_t side[2] = {nullptr, nullptr};
+    cudaEvent_t ev_fork = nullptr, ev_radii = nullptr, ev_jac = nullptr, ev_side1 = nullptr;
     // the terms that faces of the FP64 path share (AuxTerm), where they fit: device memory and budget
     // are left for everything else first
     double* d_aux = nullptr;

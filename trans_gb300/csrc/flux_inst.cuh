@@ -23,18 +23,18 @@ void shg(cudaStream_t s, const DevBlock* b, const Tile* t, int nt) {
 void bcg(cudaStream_t s, const DevBlock* b, const BCEntry* e, int n) {
     if (n > 0) k_bc_grad<TG_R><<<(n + 127) / 128, 128, 0, s>>>(b, e, n);
 }
-void ff(cudaStream_t s, const DevBlock* b, const Tile* t, int nt, const CaseDev* cd, bool terms) {
+void ff(cudaStream_t s, cudaStream_t sc, const DevBlock* b, const Tile* t, int nt, const CaseDev* cd, bool terms) {
     if (nt <= 0) return;
     // viscous, then convective fluxes (two register budgets)
     if constexpr (sizeof(TG_R) == 8) {
         if (terms) {
             k_face_flux<TG_R, 1, FaceTerms><<<nt, FACE_TILE, 0, s>>>(b, t, cd);
-            k_face_flux<TG_R, 2, FaceTerms><<<nt, FACE_TILE, 0, s>>>(b, t, cd);
+            k_face_flux<TG_R, 2, FaceTerms><<<nt, FACE_TILE, 0, sc>>>(b, t, cd);
             return;
         }
     }
     k_face_flux<TG_R, 1><<<nt, FACE_TILE, 0, s>>>(b, t, cd);
-    k_face_flux<TG_R, 2><<<nt, FACE_TILE, 0, s>>>(b, t, cd);
+    k_face_flux<TG_R, 2><<<nt, FACE_TILE, 0, sc>>>(b, t, cd);
 }
 void ga(cudaStream_t s, const DevBlock* b, const Tile* t, int nt, const CaseDev* cd) {
     if (nt > 0) k_gather<TG_R><<<nt, CELL_TILE, 0, s>>>(b, t, cd);

@@ -102,7 +102,8 @@ struct FluxLaunchers {
     void (*gradient)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*, bool terms);
     void (*shock_ghost)(cudaStream_t, const DevBlock*, const Tile*, int);
     void (*bc_grad)(cudaStream_t, const DevBlock*, const BCEntry*, int);
-    void (*face_flux)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*, bool terms);
+    // (viscous fluxes on the first stream, convective on the second)
+    void (*face_flux)(cudaStream_t, cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*, bool terms);
     void (*gather)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*);
     void (*sst_fc1)(cudaStream_t, const DevBlock*, const Tile*, int, const CaseDev*);
     // cross-rank 1-to-1 segment: words (host-built table, device staging) into the ghost layers

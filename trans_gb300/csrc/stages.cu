@@ -528,7 +528,7 @@ int tune_resid(Ctx* c) {
                 launch_resid_tma(d + 1, s, c->d_blk, c->d_rtiles[d], c->n_rtiles[d], c->d_cdev, c->d_rmaps, c->d_kerr,
                                  c->resid_spin);
         } else {
-            c->fl->face_flux(s, c->d_blk, c->d_face, (int)c->face_tiles.size(), c->d_cdev, false);
+            c->fl->face_flux(s, s, c->d_blk, c->d_face, (int)c->face_tiles.size(), c->d_cdev, false);
             c->fl->gather(s, c->d_blk, c->d_cell, nct, c->d_cdev);
         }
     };
@@ -572,6 +572,23 @@ namespace {
 
 // One stage.  capture: inside a CUDA-graph capture (no host synchronisation, no parameter
 // upload, the norms go to history slot `slot`).
+// Branches of a captured iteration.  Kernels that do not depend on one another become parallel branches
+// of the graph: the small blocks' kernels fill a fraction of the chip each and are bound by their latency,
+// the large ones' last waves fill up.  us an iteration, in a row and in branches: 24x16x5 cells FP64 506
+// and 429, the 96x48x8 channel mixed 179 and 158 and FP64 1,205 and 1,150, the coarse cascade mixed 461
+// and 431, 1,966,080 cells mixed 1,801 and 1,757 and FP64 21,490 and 21,433.  fork: side stream q goes on
+// from here; join: the main stream waits for what was recorded.
+// (Runge-Kutta's stage update changes what the Jacobian terms are formed from)
+bool jac_branch(const Ctx* c, bool capture) { return capture && c->march && !c->mixed && c->sweep_lanes == 1; }
+// the convective fluxes apart from the viscous ones (not the TMA-staged form, which has all in one)
+bool face_branch(const Ctx* c, bool capture) { return capture && !(c->mixed && c->resid_tma == 1); }
+cudaStream_t fork(Ctx* c, int q) {
+    cudaEventRecord(c->ev_fork, c->stream);
+    cudaStreamWaitEvent(c->side[q], c->ev_fork, 0);
+    return c->side[q];
+}
+void join(Ctx* c, cudaEvent_t e) { cudaStreamWaitEvent(c->stream, e, 0); }
+
 // seq: the stage is one of a whole iteration's, with nothing between it and the stages before
 int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot, bool seq) {
     if (c->cases.empty()) return fail(c, TRANS_E_ARG, "no case");
@@ -586,18 +603,29 @@ int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot, bool seq) {
         case TRANS_STAGE_SPECRAD: {
             if (!capture && (rc = upload_cdev(c))) return rc;
             KScope t(c, K_SPECRAD);
-            if (c->mixed) launch_specrad_mixed(s, c->d_blk, c->d_cell, nct, c->d_cdev);
-            else launch_specrad(s, c->d_blk, c->d_cell, nct, c->d_cdev);
+            cudaStream_t s0 = capture ? fork(c, 0) : s;       // read from the primitives (mixed) or the preparation on
+            if (c->mixed) launch_specrad_mixed(s0, c->d_blk, c->d_cell, nct, c->d_cdev);
+            else launch_specrad(s0, c->d_blk, c->d_cell, nct, c->d_cdev);
+            if (capture) cudaEventRecord(c->ev_radii, s0);
             c->launches++;
             break;
         }
         case TRANS_STAGE_BC_STATE:
             if (!capture && (rc = upload_cdev(c))) return rc;
-            { KScope t(c, K_BC_STATE); launch_bc_state(s, c->d_blk, c->d_bc, (int)c->bc.size(), c->d_cdev); }
             {
-                KScope t(c, K_BC_OUTLET);
-                if (c->mixed) launch_bc_outlet_mixed(s, c->d_blk, c->d_outlet, c->d_lines, (int)c->lines.size(), c->d_cdev);
-                else launch_bc_outlet(s, c->d_blk, c->d_outlet, c->d_lines, (int)c->lines.size(), c->d_cdev);
+                // the outlets' ghost cells are theirs alone, and both kernels read interior cells
+                const bool branch = capture && !c->lines.empty();
+                cudaStream_t s1 = branch ? fork(c, 1) : s;
+                { KScope t(c, K_BC_STATE); launch_bc_state(s, c->d_blk, c->d_bc, (int)c->bc.size(), c->d_cdev); }
+                {
+                    KScope t(c, K_BC_OUTLET);
+                    if (c->mixed) launch_bc_outlet_mixed(s1, c->d_blk, c->d_outlet, c->d_lines, (int)c->lines.size(), c->d_cdev);
+                    else launch_bc_outlet(s1, c->d_blk, c->d_outlet, c->d_lines, (int)c->lines.size(), c->d_cdev);
+                }
+                if (branch) {
+                    cudaEventRecord(c->ev_side1, s1);
+                    join(c, c->ev_side1);
+                }
             }
             c->launches += 1 + (c->lines.empty() ? 0 : 1);
             break;
@@ -606,10 +634,16 @@ int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot, bool seq) {
             if (c->mixed) {
                 // the FP32 kernels read FP32 copies of this sub-iteration's state, primitives and radii
                 KScope t(c, K_PRIMS);
+                if (capture) join(c, c->ev_radii);
                 launch_prims_mixed(s, c->d_blk, (int)c->blk.size(), c->total_cells, c->d_off);
             } else {
                 KScope t(c, K_PRIMS);
                 launch_prims(s, c->d_blk, (int)c->blk.size(), c->total_cells, c->d_off);
+            }
+            if (jac_branch(c, capture)) {          // from the primitives and the radii
+                cudaStream_t s0 = fork(c, 0);
+                launch_march64_jac(s0, c->d_blk, c->d_mtiles, c->d_mruns, c->n_mruns, c->sv.rec);
+                cudaEventRecord(c->ev_jac, s0);
             }
             // the face averages, and with an iteration to follow the fluxes' other shared terms
             if (c->d_aux) {
@@ -618,7 +652,8 @@ int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot, bool seq) {
                 c->launches++;
             }
             { KScope t(c, K_GRADIENT); c->fl->gradient(s, c->d_blk, c->d_cell, nct, c->d_cdev, c->d_aux != nullptr); }
-            { KScope t(c, K_SHOCK_GHOST); c->fl->shock_ghost(s, c->d_blk, c->d_ghost, (int)c->ghost_tiles.size()); }
+            // (the convective fluxes follow on this branch)
+            { KScope t(c, K_SHOCK_GHOST); c->fl->shock_ghost(face_branch(c, capture) ? fork(c, 1) : s, c->d_blk, c->d_ghost, (int)c->ghost_tiles.size()); }
             c->launches += 3;
             break;
         case TRANS_STAGE_BC_GRAD:
@@ -646,13 +681,19 @@ int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot, bool seq) {
                     launch_face_terms(s, c->d_blk, (int)c->blk.size(), c->total_cells, c->d_off, c->d_cdev, 1);
                     c->launches++;
                 }
-                c->fl->face_flux(s, c->d_blk, c->d_face, (int)c->face_tiles.size(), c->d_cdev, terms);
+                cudaStream_t s1 = capture ? c->side[1] : s;
+                c->fl->face_flux(s, s1, c->d_blk, c->d_face, (int)c->face_tiles.size(), c->d_cdev, terms);
+                if (capture) {
+                    cudaEventRecord(c->ev_side1, s1);
+                    join(c, c->ev_side1);
+                }
             }
             { KScope t(c, K_GATHER); c->fl->gather(s, c->d_blk, c->d_cell, nct, c->d_cdev); }
             c->launches += 3;
             break;
         case TRANS_STAGE_LUSGS: {
             if (!capture && (rc = upload_cdev(c))) return rc;
+            if (capture && !c->mixed) join(c, c->ev_radii);
             if (c->sweep_lanes == 2) {
                 // Runge-Kutta: TIME_RK_Save + TIME_RK on the mean flow, then the k-omega LU-SGS
                 // of TURBTWO_TIME_LUSGS_SST on the new state (main.F90:152-158)
@@ -669,6 +710,7 @@ int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot, bool seq) {
                 KScope t(c, K_PREP);
                 c->fl->prep(s, c->d_blk, c->d_cell, nct, c->d_qpos, c->sv, c->d_cdev, c->march);
                 if (!c->march) c->fl->jac(s, c->d_blk, c->sv, c->d_cdev);
+                else if (jac_branch(c, capture)) join(c, c->ev_jac);
                 else if (!c->mixed) launch_march64_jac(s, c->d_blk, c->d_mtiles, c->d_mruns, c->n_mruns, c->sv.rec);
             }
             c->launches += 2;
@@ -697,7 +739,10 @@ int stage_exec(Ctx* c, int stage, int itr, bool capture, int slot, bool seq) {
                 if (c->sweep_lanes == 2) launch_rk_vupdate(s, c->d_blk, c->d_cell, nct, c->d_cdev, c->d_parts, c->mixed ? 1 : 0);
                 else if (c->mixed) launch_update_mixed(s, c->d_blk, c->d_cell, nct, c->d_cdev, c->d_parts);
                 else launch_update(s, c->d_blk, c->d_cell, nct, c->d_cdev, c->d_parts, 0);
-                launch_block_norms(s, c->d_blk, nblk, c->d_parts, c->d_tile_first, c->d_norms + (size_t)slot * nblk);
+                // (joined with this branch's convective fluxes of the next iteration, and at the end)
+                cudaStream_t s1 = face_branch(c, capture) ? fork(c, 1) : s;
+                launch_block_norms(s1, c->d_blk, nblk, c->d_parts, c->d_tile_first, c->d_norms + (size_t)slot * nblk);
+                if (face_branch(c, capture)) cudaEventRecord(c->ev_side1, s1);
             }
             c->launches += 2;
             if (capture) break;
@@ -786,6 +831,7 @@ int capture_iterations(Ctx* c, int n) {
         if (rc == TRANS_OK) rc = stage_exec(c, TRANS_STAGE_UPDATE_U, nsub, true, q, true);
     }
     if (rc == TRANS_OK) {
+        if (face_branch(c, true)) join(c, c->ev_side1);
         cudaMemcpyAsync(c->h_norms, c->d_norms, sizeof(BlockNorms) * (size_t)nblk * n, cudaMemcpyDeviceToHost, s);
         cudaMemcpyAsync(c->h_sync, c->d_sync, sizeof(SweepSync), cudaMemcpyDeviceToHost, s);
         cudaMemcpyAsync(c->h_kerr, c->d_kerr, sizeof(int), cudaMemcpyDeviceToHost, s);
