@@ -1078,8 +1078,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (PART == 1 ? TG_FACE_MIN
 // D of every interior cell in the reference's accumulation order (main.F90:92-133):
 //   D = 0 - Fv(i) + Fv(i+1) - Fv(j) + Fv(j+1) - Fv(k) + Fv(k+1) - Fc(i) + Fc(i+1) - ...
 // ---------------------------------------------------------------------------------------
-// (the sums unrolled, so that their loads go out together: mixed, 352,256 cells 28 -> 22 us, 1,966,080
-// cells 98 -> 88)
+// (the sums unrolled and every load before the first store, so that the loads go out together: mixed,
+// 352,256 cells 28 -> 22 us, 1,966,080 cells 98 -> 90, a batch of five cascades 133 -> 121)
 template <typename R>
 __global__ void k_gather(const DevBlock* __restrict__ blks, const Tile* __restrict__ tiles, const CaseDev* __restrict__ cdev) {
     const Tile t = tiles[blockIdx.x];
@@ -1093,6 +1093,7 @@ __global__ void k_gather(const DevBlock* __restrict__ blks, const Tile* __restri
     const size_t nc = (size_t)b.ncell;
     const R* FX = rs<R>(b, S_FX);
     const R om = cparams<R>(cdev[b.cs]).omega0;
+    R out[7];                                      // every load before the first store
 #pragma unroll
     for (int L = 0; L < 7; ++L) {
         R acc = R(0.0);
@@ -1123,8 +1124,10 @@ __global__ void k_gather(const DevBlock* __restrict__ blks, const Tile* __restri
             add(FX_TK + L - 5);
             add(FX_CK + L - 5);
         }
-        rs<R>(b, S_D + L)[c] = acc;
+        out[L] = acc;
     }
+#pragma unroll
+    for (int L = 0; L < 7; ++L) rs<R>(b, S_D + L)[c] = out[L];
 }
 
 // ---------------------------------------------------------------------------------------
