@@ -457,6 +457,7 @@ __global__ void k_prims(const DevBlock* __restrict__ blks, int nblk, long long t
     while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (off[mid] <= g) lo = mid; else hi = mid - 1; }
     const DevBlock b = blks[lo];
     int c = (int)(g - off[lo]);
+    if (!read_cell(b, c)) return;
     f64 v1 = rs<f64>(b, S_V)[c];
     rs<f64>(b, S_PRIM)[c] = rs<f64>(b, S_V + 1)[c] / v1;
     rs<f64>(b, S_PRIM + 1)[c] = rs<f64>(b, S_V + 2)[c] / v1;
