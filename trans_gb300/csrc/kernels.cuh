@@ -548,12 +548,13 @@ __global__ void k_mirror(const DevBlock* __restrict__ blks, int nblk, long long 
 #endif  // TG_COMMON_KERNELS
 
 
-// ---------------------------------------------------------------------------------------
+// (FP32 bound by load latency: with the bound below the compiler takes 113 registers for loads in flight, 93
+// without; 1,966,080 cells 112 -> 108 us, a batch of five cascades 158 -> 151; at three CTAs per SM 124)
 // ---------------------------------------------------------------------------------------
 // Space/DIFF_DqDxyz.F90:25-74, 232-265, 300-381 (gradients and shock sensor, interior cells)
 // ---------------------------------------------------------------------------------------
 template <typename R, bool TERMS = false>
-__global__ void k_gradient(const DevBlock* __restrict__ blks, const Tile* __restrict__ tiles, const CaseDev* __restrict__ cdev) {
+__global__ void __launch_bounds__(CELL_TILE, 1) k_gradient(const DevBlock* __restrict__ blks, const Tile* __restrict__ tiles, const CaseDev* __restrict__ cdev) {
     const Tile t = tiles[blockIdx.x];
     if ((int)threadIdx.x >= t.count) return;
     const DevBlock b = blks[t.blk];
