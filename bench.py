@@ -178,14 +178,13 @@ ALG_WORDS = {
     "k_sweep": 24,          # the L -> U hand-off: DeltaQ 7 + Rds 3 + diagonals 2, written and read once
     "k_update": 37, "k_gradient": 46, "k_specrad": 24, "k_lusgs_prep": 60, "k_gather": 46,
 }
-# FP64 thread-instructions per face of k_face_flux<double> (MDCD + AUSMPW+ + SST), counted by
-# ncu (DADD + DMUL + DFMA over the three directions) on the 339,968-cell cascade
-# (profiles/k_face_flux_fp64_cascade_339968cells.md), and DRAM bytes per face of the viscous
-# and convective kernels the flux is now split into (profiles/launches_cascade_5blk_1966080cells_fp64.md)
-FACE_FP64_INST = 2541.0
-FACE_DRAM_BYTES = 479.1
-FACE_DRAM_SOURCE = ("ncu dram__bytes_read+write per face of the viscous and convective kernels together on the "
-                    "491,520-cell cascade, scaled by faces")
+# FP64 thread-instructions per face of the FP64 face fluxes (MDCD + AUSMPW+ + SST; DADD + DMUL + DFMA of
+# k_face_terms, the viscous and the convective kernel: 87 + 372 + 621), and their DRAM bytes per face, counted by
+# ncu on the 352,256-cell cascade (profiles/fp64_kernels_cascade_352256cells.md)
+FACE_FP64_INST = 1080.0
+FACE_DRAM_BYTES = 1328.0
+FACE_DRAM_SOURCE = ("ncu dram__bytes_read+write per face of the shared terms, viscous and convective kernels together on "
+                    "the 352,256-cell cascade, scaled by faces")
 # kernel classes that run in FP32 in the mixed path (their algorithmic words are 4 bytes there)
 FP32_KERNELS = ("k_face_flux", "k_resid_tma", "k_gather", "k_sweep", "k_gradient")
 # bounded serving leg of the default line: 4 requests/s as the serving configuration states,
