@@ -255,6 +255,13 @@ int build_march(Ctx* c) {
     const size_t word = (c->mixed ? MARCH_EDGES : M64_EDGES) * sizeof(ulonglong2);     // 8 floats or 7 doubles, every 32 bits with the tag
     const size_t nj = (size_t)s0 * MARCH_K * word, nk = (size_t)s0 * MARCH_J * word, places = (size_t)s0 * 32;
     const size_t nrec = places * (c->mixed ? (size_t)NCREC : (size_t)M64_WIDTH) * c->fl->elem, ndq = places * DQ_STRIDE * c->fl->elem;
+    // (where they would take more than half of the free device memory, the hyperplane order, which is
+    // smaller for blocks of few lines, and leaves the rest of the work lists their room)
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || nj + nk + nrec + ndq > free_b / 2) {
+        cudaGetLastError();
+        return TRANS_OK;
+    }
     auto room = [](void* p, size_t bytes) { return cudaMalloc((void**)p, bytes) == cudaSuccess; };
     if (!room(&c->d_medgeJ, nj) || !room(&c->d_medgeK, nk) || !room(&c->d_rec, nrec) || !room(&c->d_dqs, ndq)) {
         cudaGetLastError();
@@ -300,7 +307,7 @@ int build_march(Ctx* c) {
 }
 
 // Memory for the FP64 face fluxes' shared terms, after everything else of the context has its own:
-// within the budget that is left, and within a quarter of the free device memory (the fluxes form the
+// within the budget that is left, and within an eighth of the free device memory (the fluxes form the
 // terms themselves without it)
 int build_terms(Ctx* c) {
     if (c->mixed) return TRANS_OK;
@@ -309,7 +316,7 @@ int build_terms(Ctx* c) {
     for (const DevBlock& b : c->blk) n += (size_t)b.ncell * entries(b);
     const size_t bytes = n * sizeof(double);
     if (c->budget > 0 && c->in_use + (long long)bytes > c->budget) return TRANS_OK;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 4 || cudaMalloc(&c->d_aux, bytes) != cudaSuccess) {
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 8 || cudaMalloc(&c->d_aux, bytes) != cudaSuccess) {
         cudaGetLastError();
         c->d_aux = nullptr;
         return TRANS_OK;
