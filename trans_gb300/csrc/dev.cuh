@@ -337,6 +337,14 @@ template <typename R> __device__ inline R alimiter(R var1, R var2) {
 
 // c x + y with c a power of two: c x is exact, so this is the rounding of the plain sum
 __device__ __forceinline__ f64 fma2(double c, f64 x, f64 y) { return f64(__fma_rn(c, x.v, y.v)); }
+// a + c v with c = 0.5, -0.5, 2: the product is exact, so FP64 takes one instruction (with the zero terms of
+// ausmpw_flux and jac_terms: face fluxes of 1,966,080 cells 12.97 -> 12.77 ms, preparation 1.72 -> 1.68)
+template <typename R> __device__ __forceinline__ R add_half(R a, R v) { return a + R(0.5) * v; }
+template <typename R> __device__ __forceinline__ R sub_half(R a, R v) { return a - R(0.5) * v; }
+template <typename R> __device__ __forceinline__ R add_twice(R a, R v) { return a + R(2.0) * v; }
+template <> __device__ __forceinline__ f64 add_half<f64>(f64 a, f64 v) { return fma2(0.5, v, a); }
+template <> __device__ __forceinline__ f64 sub_half<f64>(f64 a, f64 v) { return fma2(-0.5, v, a); }
+template <> __device__ __forceinline__ f64 add_twice<f64>(f64 a, f64 v) { return fma2(2.0, v, a); }
 // the larger of two non-negative values, as integers
 __device__ __forceinline__ f64 umax(f64 a, f64 b) {
     return __double_as_longlong(a.v) < __double_as_longlong(b.v) ? b : a;
@@ -589,8 +597,8 @@ __device__ inline void roe_flux(const ParamsT<R>& p, R PLo, R PRo, R TLo, R TRo,
     const R ga = R(1.4), ga1 = R(1.4 - 1.0);
     R VAMLo = ULo * ULo + VLo * VLo + WLo * WLo;
     R VAMRo = URo * URo + VRo * VRo + WRo * WRo;
-    R HLo = PLo * ga / (DENLo * ga1) + R(0.5) * VAMLo - R(0.5) * (rLo * rLo);
-    R HRo = PRo * ga / (DENRo * ga1) + R(0.5) * VAMRo - R(0.5) * (rRo * rRo);
+    R HLo = sub_half(add_half(PLo * ga / (DENLo * ga1), VAMLo), rLo * rLo);
+    R HRo = sub_half(add_half(PRo * ga / (DENRo * ga1), VAMRo), rRo * rRo);
     R rrorl = sqrt(DENRo / DENLo);
     R rrorlp1 = R(1.0) + rrorl;
     R rm = sqrt(DENRo * DENLo);
@@ -600,7 +608,7 @@ __device__ inline void roe_flux(const ParamsT<R>& p, R PLo, R PRo, R TLo, R TRo,
     R hm = (HLo + HRo * rrorl) / rrorlp1;
     R vm2 = um * um + vm * vm + wm * wm;
     R rccm = (rLo + rrorl * rRo) / rrorlp1;
-    R am2 = ga1 * fabs(hm - R(0.5) * vm2 + R(0.5) * (rccm * rccm));
+    R am2 = ga1 * fabs(add_half(sub_half(hm, vm2), rccm * rccm));
     R am = sqrt(am2);
     R sav1n = sav1 / sav, sav2n = sav2 / sav, sav3n = sav3 / sav;
     R unormaln = (sav1n * um + sav2n * vm + sav3n * wm);
@@ -663,8 +671,8 @@ __device__ inline void ausmpw_flux(const ParamsT<R>& p, R PLo, R PRo, R TLo, R T
     const R ga = R(1.4), ga1 = R(1.4 - 1.0);
     R VAMLo = ULo * ULo + VLo * VLo + WLo * WLo;
     R VAMRo = URo * URo + VRo * VRo + WRo * WRo;
-    R HLo = PLo * ga / (DENLo * ga1) + R(0.5) * VAMLo;
-    R HRo = PRo * ga / (DENRo * ga1) + R(0.5) * VAMRo;
+    R HLo = add_half(PLo * ga / (DENLo * ga1), VAMLo);
+    R HRo = add_half(PRo * ga / (DENRo * ga1), VAMRo);
     R ULn = (sav1n * ULo + sav2n * VLo + sav3n * WLo);
     R URn = (sav1n * URo + sav2n * VRo + sav3n * WRo);
     R astar_L = sqrt(R(2) * ga1 * HLo / (ga + R(1)));
@@ -673,7 +681,10 @@ __device__ inline void ausmpw_flux(const ParamsT<R>& p, R PLo, R PRo, R TLo, R T
     R aas_R = astar_R * astar_R / dmax(sqrt(VAMRo), astar_R);
     R Acc = dmin(aas_L, aas_R);
     R MaL = ULn / Acc, MaR = URn / Acc;
-    const R c316 = R(0.0);    // 3/16 is integer division in the reference (CONVECT_AUSMPW_Plus.F90:274,286)
+    // 3/16 is integer division in the reference (CONVECT_AUSMPW_Plus.F90:274,286), so the polynomials' second
+    // terms are signed zeros on values that are never -0; FP64 leaves them out (12 instructions a face)
+    constexpr bool ZERO_TERMS = sizeof(R) == 4;
+    const R c316 = R(0.0);
     const R tiny = R(p.Tiny);
     R MaL_plus, pL_plus, MaR_neg, pR_neg;
     if (fabs(MaL) > R(1.0)) {
@@ -681,14 +692,16 @@ __device__ inline void ausmpw_flux(const ParamsT<R>& p, R PLo, R PRo, R TLo, R T
         pL_plus = R(0.5) * (MaL + fabs(MaL)) / (MaL + tiny);
     } else {
         MaL_plus = R(0.25) * sq(MaL + R(1));
-        pL_plus = R(0.25) * sq(MaL + R(1)) * (R(2) - MaL) + c316 * MaL * sq(MaL * MaL - R(1));
+        pL_plus = R(0.25) * sq(MaL + R(1)) * (R(2) - MaL);
+        if constexpr (ZERO_TERMS) pL_plus = pL_plus + c316 * MaL * sq(MaL * MaL - R(1));
     }
     if (fabs(MaR) > R(1.0)) {
         MaR_neg = R(0.5) * (MaR - fabs(MaR));
         pR_neg = R(0.5) * (MaR - fabs(MaR)) / (MaR + tiny);
     } else {
         MaR_neg = R(-1) * R(0.25) * sq(MaR - R(1));
-        pR_neg = R(0.25) * sq(MaR - R(1)) * (R(2) + MaR) - c316 * MaR * sq(MaR * MaR - R(1));
+        pR_neg = R(0.25) * sq(MaR - R(1)) * (R(2) + MaR);
+        if constexpr (ZERO_TERMS) pR_neg = pR_neg - c316 * MaR * sq(MaR * MaR - R(1));
     }
     R pS = pL_plus * PLo + pR_neg * PRo;
     R Mas = MaL_plus + MaR_neg;
@@ -720,36 +733,38 @@ __device__ inline void jac_terms(R pVx, R pVy, R pVz, R aSDx, R aSDy, R aSDz, R 
     const R pGam = R(1.4);
     R VP = pVx * aSDx + pVy * aSDy + pVz * aSDz + R(0.0);
     R Ut2 = pVx * pVx + pVy * pVy + pVz * pVz;
+    // the grid speed's zero added to VP, which is never -0: nothing (left to the compiler in FP32)
     const R aSDt = R(0.0);
+    auto with_grid_speed = [&](R x) { return sizeof(R) == 8 ? x : aSDt + x; };
     const R Gm1 = R(1.4 - 1.0), Gm2 = R(1.4 - 2.0);
     R AA2 = pGam * pPP * roinv;
     R gUt2 = R(0.5) * Gm1 * Ut2;
     J[JC_R1 + 0] = aSDx * gUt2 - pVx * VP;
-    J[JC_R1 + 1] = aSDt + VP - aSDx * Gm2 * pVx;
+    J[JC_R1 + 1] = with_grid_speed(VP) - aSDx * Gm2 * pVx;
     J[JC_R1 + 2] = aSDy * pVx - aSDx * Gm1 * pVy;
     J[JC_R1 + 3] = aSDz * pVx - aSDx * Gm1 * pVz;
     J[JC_R1 + 4] = aSDx * Gm1;
     J[JC_R2 + 0] = aSDy * gUt2 - pVy * VP;
     J[JC_R2 + 1] = aSDx * pVy - aSDy * Gm1 * pVx;
-    J[JC_R2 + 2] = aSDt + VP - aSDy * Gm2 * pVy;
+    J[JC_R2 + 2] = with_grid_speed(VP) - aSDy * Gm2 * pVy;
     J[JC_R2 + 3] = aSDz * pVy - aSDy * Gm1 * pVz;
     J[JC_R2 + 4] = aSDy * Gm1;
     J[JC_R3 + 0] = aSDz * gUt2 - pVz * VP;
     J[JC_R3 + 1] = aSDx * pVz - aSDz * Gm1 * pVx;
     J[JC_R3 + 2] = aSDy * pVz - aSDz * Gm1 * pVy;
-    J[JC_R3 + 3] = aSDt + VP - aSDz * Gm2 * pVz;
+    J[JC_R3 + 3] = with_grid_speed(VP) - aSDz * Gm2 * pVz;
     J[JC_R3 + 4] = aSDz * Gm1;
     J[JC_R0 + 0] = aSDx;
     J[JC_R0 + 1] = aSDy;
     J[JC_R0 + 2] = aSDz;
     R GEt1 = R(0.5) * Gm2 * Ut2 - AA2 / Gm1;
-    R GEt2 = R(0.5) * Ut2 + AA2 / Gm1;
+    R GEt2 = add_half(AA2 / Gm1, Ut2);
     J[JC_VP] = VP;
     J[JC_GET1] = GEt1;
     J[JC_R4 + 0] = aSDx * GEt2 - Gm1 * pVx * VP;
     J[JC_R4 + 1] = aSDy * GEt2 - Gm1 * pVy * VP;
     J[JC_R4 + 2] = aSDz * GEt2 - Gm1 * pVz * VP;
-    J[JC_R4 + 3] = aSDt + pGam * VP;
+    J[JC_R4 + 3] = with_grid_speed(pGam * VP);
     // contravariant speed of TURBTWO_TIME_LUSGS_SST (no "+ 0" there)
     J[JC_VPT] = pVx * aSDx + pVy * aSDy + pVz * aSDz;
 }

@@ -825,9 +825,9 @@ __device__ __forceinline__ void face_flux_body(const int DIR, const ParamsT<R>& 
         R DwDxL = g[2][0], DwDyL = g[2][1], DwDzL = g[2][2];
         R DTDxL = g[3][0], DTDyL = g[3][1], DTDzL = g[3][2];
         R div = DuDxL + DvDyL + DwDzL;
-        R Txx = RmiuL * (NMD * div + R(2.0) * DuDxL) + RmiuTL * (NMD * div + R(2.0) * DuDxL);
-        R Tyy = RmiuL * (NMD * div + R(2.0) * DvDyL) + RmiuTL * (NMD * div + R(2.0) * DvDyL);
-        R Tzz = RmiuL * (NMD * div + R(2.0) * DwDzL) + RmiuTL * (NMD * div + R(2.0) * DwDzL);
+        R Txx = RmiuL * add_twice(NMD * div, DuDxL) + RmiuTL * add_twice(NMD * div, DuDxL);
+        R Tyy = RmiuL * add_twice(NMD * div, DvDyL) + RmiuTL * add_twice(NMD * div, DvDyL);
+        R Tzz = RmiuL * add_twice(NMD * div, DwDzL) + RmiuTL * add_twice(NMD * div, DwDzL);
         R Txy = RmiuL * (DuDyL + DvDxL) + RmiuTL * (DuDyL + DvDxL);
         R Tyz = RmiuL * (DvDzL + DwDyL) + RmiuTL * (DvDzL + DwDyL);
         R Tzx = RmiuL * (DuDzL + DwDxL) + RmiuTL * (DuDzL + DwDxL);
