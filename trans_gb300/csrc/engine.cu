@@ -138,6 +138,14 @@ long long case_bytes(const trans_params* p, int nblocks, const trans_block* bloc
     return b;
 }
 
+// TRANS_SWEEP_SPIN=n bounds every device-side wait of the sweep schedules at n polls (for tests of the
+// timeout path: a small n makes the waits run out).  Read when a context is created and when its
+// iterations are captured.
+void read_spin_limit(Ctx* c) {
+    const char* sp = std::getenv("TRANS_SWEEP_SPIN");
+    c->spin_limit = sp ? (unsigned)std::max(0L, std::strtol(sp, nullptr, 10)) : SWEEP_SPIN_LIMIT;
+}
+
 int ctx_init(Ctx* c, int precision, long long budget) {
     c->precision = precision;
     c->mixed = precision == TRANS_MIXED;
@@ -186,10 +194,7 @@ int ctx_init(Ctx* c, int precision, long long budget) {
     // TRANS_SWEEP_PF=n forces an L2 prefetch distance of n hyperplanes (for tests)
     const char* pf = std::getenv("TRANS_SWEEP_PF");
     if (pf) c->sweep_pf = std::max(0, std::atoi(pf));
-    // TRANS_SWEEP_SPIN=n bounds every device-side wait of the cooperative sweep schedules at n
-    // polls (for tests of the timeout path: a small n makes the waits run out)
-    const char* sp = std::getenv("TRANS_SWEEP_SPIN");
-    if (sp) c->spin_limit = (unsigned)std::max(0L, std::strtol(sp, nullptr, 10));
+    read_spin_limit(c);
     // sweep schedule: TRANS_SWEEP=planes | coop | flow | tiles | clusters | pairs | march forces one (for tests);
     // default: tuned
     const char* m = std::getenv("TRANS_SWEEP");

@@ -180,6 +180,9 @@ struct Ctx {
     int sweep_lanes = 1;                 // DeltaQ components swept: 1 = all, 2 = k and omega only (Runge-Kutta)
     SweepSync* d_sync = nullptr;
     SweepSync* h_sync = nullptr;         // pinned
+    // d_sync may hold the flag of a wait that ran out (a marching sweep launched by itself clears it, its
+    // captured form does not): cleared before the next graph replay
+    bool sync_stale = true;
     unsigned spin_limit = SWEEP_SPIN_LIMIT;   // polls of one device-side wait before it gives up
     std::string sweep_tuning;
     // ---- instrumentation ----
@@ -212,6 +215,7 @@ struct KScope {
 bool params_supported(const trans_params* p);
 int validate_case(const trans_params* p, int nblocks, const trans_block* blocks);
 int ctx_init(Ctx* c, int precision, long long budget);
+void read_spin_limit(Ctx* c);
 void ctx_free(Ctx* c);
 long long case_bytes(const trans_params* p, int nblocks, const trans_block* blocks);
 // sub-iterations of one outer iteration: 3 SSP-RK3 stages, Kchld dual-time steps or 1 (main.F90:54-56)

@@ -296,8 +296,11 @@ int sweep_once(Ctx* c, int mode, int grid, int block, bool capture = false) {
     }
     if (mode == 6) {
         if (!c->march) return fail(c, TRANS_E_ARG, "the sweep arrays are not in the marching order");
-        // (graph replays keep the flag cleared here or by the run that reported it)
-        if (!capture) CK(cudaMemsetAsync(c->d_sync, 0, sizeof(SweepSync), s));
+        // (replays of a captured sweep start from a flag that run_iterations cleared)
+        if (!capture) {
+            CK(cudaMemsetAsync(c->d_sync, 0, sizeof(SweepSync), s));
+            c->sync_stale = true;
+        }
         auto launch = c->mixed ? launch_sweep_march : launch_sweep_march64;
         CK(launch(s, c->sv, c->d_mtiles, c->n_mtiles, c->d_medgeJ, c->d_medgeK, c->d_mctl, c->d_sync, c->sweep_lanes, c->spin_limit));
         if (!capture) CK(cudaMemcpyAsync(c->h_sync, c->d_sync, sizeof(SweepSync), cudaMemcpyDeviceToHost, s));
@@ -810,6 +813,7 @@ bool switches_fixed(Ctx* c, int n) {
 // capture n iterations into c->iter_exec (n = GRAPH_ITERS) or c->iter1_exec (n = 1)
 int capture_iterations(Ctx* c, int n) {
     cudaGraphExec_t& exec = n == 1 ? c->iter1_exec : c->iter_exec;
+    read_spin_limit(c);
     if (exec) { cudaGraphExecDestroy(exec); exec = nullptr; }
     if (n != 1) c->iter_n = 0;
     if (c->sweep_mode == 3 && !c->d_tiles) {          // allocations cannot happen inside the capture
@@ -890,6 +894,10 @@ int run_iterations(Ctx* c, int n) {
             ++done;
             continue;
         }
+        if (c->sync_stale) {
+            CK(cudaMemsetAsync(c->d_sync, 0, sizeof(SweepSync), c->stream));
+            c->sync_stale = false;
+        }
         CK(cudaGraphLaunch(graph ? c->iter_exec : c->iter1_exec, c->stream));
         CK(cudaStreamSynchronize(c->stream));
         c->launches += graph ? c->iter_launches : c->iter1_launches;
@@ -905,7 +913,7 @@ int run_iterations(Ctx* c, int n) {
         for (int q = 1; q < m; ++q) advance();  // KI of the last replayed iteration
         done += m;
         if (sweep_timed_out(c)) {
-            CK(cudaMemsetAsync(c->d_sync, 0, sizeof(SweepSync), c->stream));
+            c->sync_stale = true;
             return fail(c, TRANS_E_TIMEOUT, "LU-SGS sweep wait timed out");
         }
         if (*c->h_kerr) return fail(c, TRANS_E_TIMEOUT, "residual tile staging wait timed out");

@@ -287,7 +287,6 @@ int build_march(Ctx* c) {
     CK(cudaMemsetAsync(c->d_rec, 0, nrec, c->stream));          // the places outside the blocks stay finite
     CK(cudaMemsetAsync(c->d_dqs, 0, ndq, c->stream));
     CK(cudaMemsetAsync(c->d_mctl, 0, sizeof(MarchCtl), c->stream));
-    CK(cudaMemsetAsync(c->d_sync, 0, sizeof(SweepSync), c->stream));
     std::vector<int> qpos(c->cell_tiles.size() * (size_t)CELL_TILE, -1);
     for (size_t t = 0; t < c->cell_tiles.size(); ++t) {
         const Tile& tl = c->cell_tiles[t];
