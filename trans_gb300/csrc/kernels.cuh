@@ -1770,13 +1770,17 @@ __device__ inline void sweep_item(const int* __restrict__ nbp, const R* __restri
                 Dif = AinRo * k[d][4] * k[d][5] + AinRx * k[d][0] + AinRy * k[d][1] + AinRz * k[d][2] + AinRe * k[d][3];
             }
             if constexpr (sizeof(R) == 8) {
-                if (pc && (L == 0 || L == 4)) {
-                    // low-Mach preconditioning: PrecondDW of the neighbour's whole A(Q) DeltaQ
-                    // (TIME_LUSGS.F90:235-248); its rows as the lanes form them, then the map
+                // low-Mach preconditioning: PrecondDW of the neighbour's whole A(Q) DeltaQ
+                // (TIME_LUSGS.F90:235-248), for the density and the energy; its rows as the lanes form them, then the
+                // map.  Both components by one comparison, so that their lanes take the ~65 FP64 instructions
+                // together: by two they entered one after the other (lane-major launches of 96x48x8 cells, both sweeps
+                // 8.8 ms; 4.9 this way, 4.9 with a warp per component)
+                if (pc && (L & 3) == 0) {
                     const int jd = NBREC * (side + d);
                     R A[5];
                     A[0] = AinRo * R(0.0) + AinRx * REC(jd + JC_R0) + AinRy * REC(jd + JC_R0 + 1) + AinRz * REC(jd + JC_R0 + 2) +
                            AinRe * R(0.0);
+#pragma unroll
                     for (int l = 1; l < 4; ++l) {
                         const int o = jd + JC_R1 + 5 * (l - 1);
                         A[l] = AinRo * REC(o) + AinRx * REC(o + 1) + AinRy * REC(o + 2) + AinRz * REC(o + 3) + AinRe * REC(o + 4);
@@ -1786,7 +1790,7 @@ __device__ inline void sweep_item(const int* __restrict__ nbp, const R* __restri
                     R tpc[NPC];
                     for (int m = 0; m < NPC; ++m) tpc[m] = pc[sw_at(q, (side + d) * NPC + m, 6 * NPC)];
                     precond_apply<R>(A, tpc);
-                    Dif = A[L];
+                    Dif = L == 0 ? A[0] : A[4];
                 }
             }
             const R Din = L == 0 ? AinRo : L == 1 ? AinRx : L == 2 ? AinRy : L == 3 ? AinRz : AinRe;
