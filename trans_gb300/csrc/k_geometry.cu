@@ -35,6 +35,7 @@
 #include <algorithm>
 #include <cmath>
 #include <string>
+#include <memory>
 #include <vector>
 
 #include "../../include/trans_gpu.h"
@@ -99,18 +100,84 @@ __device__ __forceinline__ float warp_extreme(float x) {
     return x;
 }
 
+// Points in the caller's order may lie anywhere, and a warp whose points lie far apart meets most chunks and scans
+// what any lane needs.  So they are grouped by the cell of a 2^b x 2^b x 2^b grid over their box, in
+// Morton order: index idx[c] of the c-th (within a cell in any order: a point's result does not depend on its
+// warp).
+struct PointGrid { double lo[3], scale[3]; int bits; };
+__device__ __forceinline__ unsigned point_bin(const PointGrid& g, const double* x) {
+    unsigned key = 0;
+    for (int m = 0; m < 3; ++m) {
+        const double t = (x[m] - g.lo[m]) * g.scale[m];
+        const unsigned q = (unsigned)fmin(fmax(t, 0.0), (double)((1 << g.bits) - 1));
+        for (int b = 0; b < g.bits; ++b) key |= (q >> b & 1u) << (3 * b + m);
+    }
+    return key;
+}
+__global__ void k_point_count(unsigned n, const double* __restrict__ pts, PointGrid g, unsigned* __restrict__ bins) {
+    const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < n) atomicAdd(bins + point_bin(g, pts + 3 * (size_t)c), 1u);
+}
+// counts into first places, one CTA of 1,024 threads, each with a run of bins in 16-byte words, many in flight
+// (2^15 bins one by one took 51 us, as long as the search of 200,000 points on a small surface)
+__global__ void __launch_bounds__(1024) k_point_scan(unsigned* __restrict__ bins, unsigned nbins) {
+    __shared__ unsigned warp_sum[32];
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned words = nbins / 4, per = (words + 1023) / 1024, b0 = min(threadIdx.x * per, words), b1 = min(b0 + per, words);
+    uint4* const v = reinterpret_cast<uint4*>(bins);
+    unsigned sum = 0;
+#pragma unroll 8
+    for (unsigned b = b0; b < b1; ++b) {
+        const uint4 c = v[b];
+        sum += c.x + c.y + c.z + c.w;
+    }
+    unsigned at = sum;                             // inclusive over the warp, then over the warps
+    for (int w = 1; w < 32; w <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, at, w);
+        if (lane >= (unsigned)w) at += y;
+    }
+    if (lane == 31) warp_sum[warp] = at;
+    __syncthreads();
+    if (warp == 0) {
+        unsigned x = warp_sum[lane];
+        for (int w = 1; w < 32; w <<= 1) {
+            const unsigned y = __shfl_up_sync(0xffffffffu, x, w);
+            if (lane >= (unsigned)w) x += y;
+        }
+        warp_sum[lane] = x;
+    }
+    __syncthreads();
+    unsigned place = at - sum + (warp ? warp_sum[warp - 1] : 0u);
+#pragma unroll 8
+    for (unsigned b = b0; b < b1; ++b) {
+        const uint4 c = v[b];
+        const uint4 first = make_uint4(place, place + c.x, place + c.x + c.y, place + c.x + c.y + c.z);
+        v[b] = first;
+        place = first.w + c.w;
+    }
+}
+__global__ void k_point_place(unsigned n, const double* __restrict__ pts, PointGrid g, unsigned* __restrict__ bins,
+                              unsigned* __restrict__ idx) {
+    const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < n) idx[atomicAdd(bins + point_bin(g, pts + 3 * (size_t)c), 1u)] = c;
+}
+
 // One thread per point, a warp's points together: its lanes first test 32 chunks at a time against the box
 // of the warp's points, then each of those left against the points, and scan its panels where a lane
 // needs them; panel loads have one address in all lanes.  Bound by the issue of FP32 instructions
 // and the latency of the chunk loops (issue 55% busy): the coarse O-block, 208,896 cells and 26,368 panels,
-// 5.65 ms with every panel scanned, 3.5 with the chunks but warps along lines, 0.69 now.
+// 5.65 ms with every panel scanned, 3.5 with the chunks but warps along lines, 0.69 with a warp's points a brick.
+// ONE: a warp per point, its lanes over a chunk's panels; no points of its own to wait for, so a few points
+// take the time of one (64 points on 26,368 panels 0.39 ms the whole call, 2.4 a lane per point).
+template <bool ONE>
 __global__ void __launch_bounds__(WD_THREADS)
-k_wall_distance(long long n, const double* __restrict__ pts, const float4* __restrict__ pan32, const float4* __restrict__ pan_lo,
+k_wall_distance(long long n, const double* __restrict__ pts, const unsigned* __restrict__ idx, const float4* __restrict__ pan32, const float4* __restrict__ pan_lo,
                 const double* __restrict__ pan64, const WallChunk* __restrict__ chunks, const int* __restrict__ coff, int nsurf, float eabs, double tiny,
                 double* __restrict__ dst) {
     const unsigned full = 0xffffffffu;
-    const long long c = (long long)blockIdx.x * WD_THREADS + threadIdx.x;
-    const bool live = c < n;
+    const long long place = ((long long)blockIdx.x * WD_THREADS + threadIdx.x) >> (ONE ? 5 : 0);
+    const bool live = place < n;
+    const long long c = idx && live ? idx[place] : place;
     const double px = live ? pts[3 * c] : 0.0, py = live ? pts[3 * c + 1] : 0.0, pz = live ? pts[3 * c + 2] : 0.0;
     const float fx = (float)px, fy = (float)py, fz = (float)pz;
     const float lx = (float)(px - (double)fx), ly = (float)(py - (double)fy), lz = (float)(pz - (double)fz);
@@ -132,7 +199,7 @@ k_wall_distance(long long n, const double* __restrict__ pts, const float4* __res
         // f(k) for the chunks whose distance to the warp's box is at most that of the farthest reach
         auto near_chunks = [&](auto&& reach, auto&& f) {
             for (int k = k0; k < k1; k += 32) {
-                const float far2 = warp_extreme<true>(live ? reach() : 0.0f);
+                const float far2 = ONE ? reach() : warp_extreme<true>(live ? reach() : 0.0f);
                 const float4* w = reinterpret_cast<const float4*>(chunks + min(k + lane, k1 - 1));
                 unsigned left = __ballot_sync(full, k + lane < k1 && boxes2f(wlo, whi, __ldg(w), __ldg(w + 1)) <= far2);
                 for (; left; left &= left - 1) f(k + __ffs(left) - 1);
@@ -142,6 +209,11 @@ k_wall_distance(long long n, const double* __restrict__ pts, const float4* __res
         auto scan = [&](int k) {
             const float4* q = pan32 + chunks[k].first;
             const int cnt = chunks[k].n;
+            if constexpr (ONE) {
+                for (int r = lane; r < cnt; r += 32) m = fminf(m, d2f(fx, fy, fz, __ldg(q + r)));
+                m = warp_extreme<false>(m);
+                return;
+            }
             int r = 0;
 #pragma unroll 4
             for (; r + 1 < cnt; r += 2) {
@@ -207,7 +279,7 @@ k_wall_distance(long long n, const double* __restrict__ pts, const float4* __res
             const long long p0 = chunks[k].first;
             const int cnt = chunks[k].n;
 #pragma unroll 4
-            for (int r = 0; r < cnt; ++r)
+            for (int r = ONE ? lane : 0; r < cnt; r += ONE ? 32 : 1)
                 if (d2f(fx, fy, fz, __ldg(pan32 + p0 + r)) <= thr) take(p0 + r);
         });
         // the candidates within the final limit, gathered to the front
@@ -221,10 +293,15 @@ k_wall_distance(long long n, const double* __restrict__ pts, const float4* __res
                 if (DDD < a) a = DDD;
             }
         }
+        if constexpr (ONE) {             // (values that are not negative, in the order of their bits)
+            long long v = __double_as_longlong(a);
+            for (int w = 16; w > 0; w >>= 1) v = min(v, __shfl_xor_sync(full, v, w));
+            a = __longlong_as_double(v);
+        }
         if (d < tiny) d = tiny;          // amax1(dst_minimum, tiny)
         if (a < d) d = a;
     }
-    if (live) dst[c] = sqrt(d);
+    if (live && (!ONE || lane == 0)) dst[c] = sqrt(d);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -494,25 +571,40 @@ namespace tg {
 namespace {
 
 // panel centres of the wall surfaces (the reference's expression), their FP32 copies, chunk by chunk, the
-// chunks and each surface's first one, and the largest coordinate magnitude
+// chunks and each surface's first one, and the largest coordinate magnitude; all of it one buffer, which
+// goes to the device as one allocation and one copy (on small surfaces the call is mostly those)
 struct Panels {
-    std::vector<WallChunk> chunks;
-    std::vector<int> coff{0};
-    std::vector<double> p64;
-    std::vector<float> p32, plo;          // rounded to FP32, and what the rounding left
+    std::unique_ptr<char[]> buf;
+    size_t bytes = 0, at32 = 0, at_lo = 0, at64 = 0, at_chunk = 0, at_first = 0;
+    int nchunk = 0;
     double R = 0.0;
 };
 
 int make_panels(int nsurf, const int* dims, const double* nodes, Panels& P) {
-    long long np = 0;
+    size_t np = 0, nc = 0;
     for (int s = 0; s < nsurf; ++s) {
         const int ni = dims[2 * s], nj = dims[2 * s + 1];
         if (ni < 1 || nj < 1) return wd_fail(TRANS_E_ARG, "bad surface dimensions");
-        np += (long long)(ni - 1) * (nj - 1);
+        np += (size_t)(ni - 1) * (nj - 1);
+        nc += (size_t)((ni - 1 + WD_CHUNK - 1) / WD_CHUNK) * ((nj - 1 + WD_CHUNK - 1) / WD_CHUNK);
     }
-    P.p64.assign((size_t)(3 * np), 0.0);
-    P.p32.assign((size_t)(4 * np), 0.0f);
-    P.plo.assign((size_t)(4 * np), 0.0f);
+    auto take = [&](size_t bytes) {
+        const size_t at = P.bytes;
+        P.bytes += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    P.at32 = take(sizeof(float) * 4 * np);         // rounded to FP32,
+    P.at_lo = take(sizeof(float) * 4 * np);        // and what the rounding left
+    P.at64 = take(sizeof(double) * 3 * np);
+    P.at_chunk = take(sizeof(WallChunk) * nc);
+    P.at_first = take(sizeof(int) * ((size_t)nsurf + 1));
+    P.buf.reset(new char[P.bytes]);
+    float* const p32 = reinterpret_cast<float*>(P.buf.get() + P.at32);
+    float* const plo = reinterpret_cast<float*>(P.buf.get() + P.at_lo);
+    double* const p64 = reinterpret_cast<double*>(P.buf.get() + P.at64);
+    WallChunk* const chunks = reinterpret_cast<WallChunk*>(P.buf.get() + P.at_chunk);
+    int* const first = reinterpret_cast<int*>(P.buf.get() + P.at_first);
+    first[0] = 0;
     size_t base = 0;
     long long p = 0;
     for (int s = 0; s < nsurf; ++s) {
@@ -533,23 +625,23 @@ int make_panels(int nsurf, const int* dims, const double* nodes, Panels& P) {
                         for (int m = 0; m < 3; ++m) {
                             if (!std::isfinite(x[m])) return wd_fail(TRANS_E_ARG, "surface coordinates not finite");
                             const float f = (float)x[m];
-                            P.p64[3 * p + m] = x[m];
-                            P.p32[4 * p + m] = f;
-                            P.plo[4 * p + m] = (float)(x[m] - (double)f);
+                            p64[3 * p + m] = x[m];
+                            p32[4 * p + m] = f;
+                            plo[4 * p + m] = (float)(x[m] - (double)f);
                             k.lo[m] = std::min(k.lo[m], f);
                             k.hi[m] = std::max(k.hi[m], f);
                             P.R = std::max(P.R, std::fabs(x[m]));
                         }
+                        p32[4 * p + 3] = plo[4 * p + 3] = 0.0f;
                     }
-                P.chunks.push_back(k);
+                chunks[P.nchunk++] = k;
             }
-        P.coff.push_back((int)P.chunks.size());
+        first[s + 1] = P.nchunk;
         base += 3 * plane;
     }
     return TRANS_OK;
 }
 
-// device memory released at scope exit
 struct DevBufs {
     std::vector<void*> v;
     ~DevBufs() { for (void* p : v) cudaFree(p); }
@@ -560,31 +652,70 @@ struct DevBufs {
     }
 };
 
+// Which warps take which points: a warp a point while these warps are few, the points grouped where there is
+// enough to pass over, otherwise as they come.  Whole calls on points in no order, ms (a lane per point as
+// they come, grouped, a warp per point; before, with every panel scanned from shared memory): 208,896 points on
+// 64 panels 0.70, 0.74, 1.09 (0.70), on 1,024 panels 0.95, 0.80, 1.11 (0.85), on 26,368 panels 6.28, 1.85, 3.42
+// (6.25); 32,768 points on 64 panels 0.23, 0.26, 0.28 (0.22), on 1,024 panels 0.33, 0.31, 0.29 (0.29), on 26,368
+// panels 2.71, 1.30, 0.92 (2.42); 64 points on 64 panels 0.13, 0.16, 0.12 (0.13), on 26,368 panels 2.37, 2.32, 0.39
+// (2.09).
+bool one_point_a_warp(long long n, const Panels& P) {
+    return n <= std::min(32768LL, std::max(4096LL, 2048LL * P.nchunk));
+}
+bool group_by_place(long long n, const Panels& P) {
+    return !one_point_a_warp(n, P) && P.nchunk >= 16 && n <= 0x7fffffffLL;
+}
+
 // the wall distance of n device points (x y z interleaved) into d_dst, on stream st
-int run_wall_distance(cudaStream_t st, long long n, const double* d_pts, int nsurf, const Panels& P, double R, double tiny,
-                      double* d_dst, DevBufs& bufs) {
+int run_wall_distance(cudaStream_t st, long long n, const double* d_pts, const unsigned* d_idx, int nsurf, const Panels& P,
+                      double R, double tiny, double* d_dst, DevBufs& bufs) {
     if (R > 1.0e18) return wd_fail(TRANS_E_ARG, "coordinates beyond 1e18");   // FP32 squares stay finite
     const float eabs = std::max((float)(1.0e-6 * R), 1.0e-37f);
-    double* d_p64 = nullptr;
-    float4 *d_p32 = nullptr, *d_plo = nullptr;
-    WallChunk* d_chunks = nullptr;
-    int* d_off = nullptr;
+    char* d = nullptr;
     cudaError_t e;
-    if ((e = bufs.get(&d_p64, sizeof(double) * P.p64.size())) != cudaSuccess ||
-        (e = bufs.get(&d_p32, sizeof(float) * P.p32.size())) != cudaSuccess ||
-        (e = bufs.get(&d_plo, sizeof(float) * P.plo.size())) != cudaSuccess ||
-        (e = bufs.get(&d_chunks, sizeof(WallChunk) * P.chunks.size())) != cudaSuccess ||
-        (e = bufs.get(&d_off, sizeof(int) * P.coff.size())) != cudaSuccess ||
-        (e = cudaMemcpyAsync(d_p64, P.p64.data(), sizeof(double) * P.p64.size(), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(d_p32, P.p32.data(), sizeof(float) * P.p32.size(), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(d_plo, P.plo.data(), sizeof(float) * P.plo.size(), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(d_chunks, P.chunks.data(), sizeof(WallChunk) * P.chunks.size(), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(d_off, P.coff.data(), sizeof(int) * P.coff.size(), cudaMemcpyHostToDevice, st)) != cudaSuccess)
+    if ((e = bufs.get(&d, P.bytes)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(d, P.buf.get(), P.bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess)
         return wd_fail(TRANS_E_CUDA, std::string("wall distance set-up: ") + cudaGetErrorString(e));
-    const unsigned grid = (unsigned)((n + WD_THREADS - 1) / WD_THREADS);
-    k_wall_distance<<<grid, WD_THREADS, 0, st>>>(n, d_pts, d_p32, d_plo, d_p64, d_chunks, d_off, nsurf, eabs, tiny, d_dst);
+    auto run = [&](auto kernel, long long threads) {
+        kernel<<<(unsigned)((threads + WD_THREADS - 1) / WD_THREADS), WD_THREADS, 0, st>>>(
+            n, d_pts, d_idx, reinterpret_cast<const float4*>(d + P.at32), reinterpret_cast<const float4*>(d + P.at_lo),
+            reinterpret_cast<const double*>(d + P.at64), reinterpret_cast<const WallChunk*>(d + P.at_chunk),
+            reinterpret_cast<const int*>(d + P.at_first), nsurf, eabs, tiny, d_dst);
+    };
+    if (one_point_a_warp(n, P)) run(k_wall_distance<true>, 32 * n);
+    else run(k_wall_distance<false>, n);
     if ((e = cudaGetLastError()) != cudaSuccess) return wd_fail(TRANS_E_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     return TRANS_OK;
+}
+
+// The points' grouping (k_point_count): where there is one, its grid; bits 0: as they come
+PointGrid group_grid(long long n, const double* xyz, const Panels& P) {
+    constexpr int SAMPLE = 1024;                   // points whose box stands for all (others: the outermost cells)
+    PointGrid g{};
+    if (!group_by_place(n, P)) return g;
+    g.bits = 2;
+    while (g.bits < 6 && (16LL << (3 * g.bits)) < n) ++g.bits;     // 2 to 16 points a cell; at most 2^18 cells
+    for (int m = 0; m < 3; ++m) {
+        double lo = xyz[m], hi = lo;
+        for (long long k = 1; k < SAMPLE; ++k) {
+            const double x = xyz[3 * (n / SAMPLE * k + n % SAMPLE * k / SAMPLE) + m];
+            lo = std::min(lo, x);
+            hi = std::max(hi, x);
+        }
+        g.lo[m] = lo;
+        g.scale[m] = hi > lo ? (1 << g.bits) / (hi - lo) : 0.0;
+        if (!std::isfinite(g.scale[m])) g.scale[m] = 0.0;
+    }
+    return g;
+}
+// the points' order, in bins[0 .. cells - 1] and behind them n indexes
+const unsigned* group_points(cudaStream_t st, long long n, const double* d_pts, const PointGrid& g, unsigned* bins) {
+    const unsigned nbins = 1u << (3 * g.bits), grid = (unsigned)((n + 255) / 256);
+    cudaMemsetAsync(bins, 0, sizeof(unsigned) * nbins, st);
+    k_point_count<<<grid, 256, 0, st>>>((unsigned)n, d_pts, g, bins);
+    k_point_scan<<<1, 1024, 0, st>>>(bins, nbins);
+    k_point_place<<<grid, 256, 0, st>>>((unsigned)n, d_pts, g, bins, bins + nbins);
+    return bins + nbins;
 }
 
 struct StreamGuard {
@@ -614,14 +745,22 @@ extern "C" int trans_wall_distance(long long n, const double* xyz, int nsurf, co
     }
     StreamGuard sg;
     DevBufs bufs;
-    double *d_pts = nullptr, *d_dst = nullptr;
+    double* d_pts = nullptr;                       // points, distances and, where they are grouped, cells and order
+    PointGrid g = group_grid(n, xyz, P);
+    const size_t words = sizeof(double) * 4 * (size_t)n;
+    auto room = [&]() { return bufs.get(&d_pts, words + (g.bits ? sizeof(unsigned) * (((size_t)1 << (3 * g.bits)) + (size_t)n) : 0)); };
     cudaError_t e;
-    if ((e = cudaStreamCreateWithFlags(&sg.s, cudaStreamNonBlocking)) != cudaSuccess ||
-        (e = bufs.get(&d_pts, sizeof(double) * 3 * (size_t)n)) != cudaSuccess ||
-        (e = bufs.get(&d_dst, sizeof(double) * (size_t)n)) != cudaSuccess ||
+    if ((e = cudaStreamCreateWithFlags(&sg.s, cudaStreamNonBlocking)) == cudaSuccess && (e = room()) != cudaSuccess && g.bits) {
+        cudaGetLastError();
+        g.bits = 0;
+        e = room();
+    }
+    if (e != cudaSuccess ||
         (e = cudaMemcpyAsync(d_pts, xyz, sizeof(double) * 3 * (size_t)n, cudaMemcpyHostToDevice, sg.s)) != cudaSuccess)
         return wd_fail(TRANS_E_CUDA, std::string("set-up: ") + cudaGetErrorString(e));
-    if ((rc = run_wall_distance(sg.s, n, d_pts, nsurf, P, R, tiny, d_dst, bufs))) { cudaStreamSynchronize(sg.s); return rc; }
+    double* const d_dst = d_pts + 3 * (size_t)n;
+    const unsigned* d_idx = g.bits ? group_points(sg.s, n, d_pts, g, reinterpret_cast<unsigned*>(d_dst + n)) : nullptr;
+    if ((rc = run_wall_distance(sg.s, n, d_pts, d_idx, nsurf, P, R, tiny, d_dst, bufs))) { cudaStreamSynchronize(sg.s); return rc; }
     if ((e = cudaMemcpyAsync(dst, d_dst, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, sg.s)) != cudaSuccess ||
         (e = cudaStreamSynchronize(sg.s)) != cudaSuccess)
         return wd_fail(TRANS_E_CUDA, std::string("wall distance: ") + cudaGetErrorString(e));
@@ -674,7 +813,7 @@ extern "C" int trans_block_metrics(int ni, int nj, int nk, const double* xyz, in
     k_geo_bface<<<blocks(nb), T, 0, sg.s>>>(g);
     k_geo_len_vol<<<blocks(ncell), T, 0, sg.s>>>(g, tiny, d_bad);
     if ((e = cudaGetLastError()) != cudaSuccess) return wd_fail(TRANS_E_CUDA, std::string("launch: ") + cudaGetErrorString(e));
-    if ((rc = run_wall_distance(sg.s, nplace, d_pts, nsurf, pan, R, tiny, d_dst, bufs))) { cudaStreamSynchronize(sg.s); return rc; }
+    if ((rc = run_wall_distance(sg.s, nplace, d_pts, nullptr, nsurf, pan, R, tiny, d_dst, bufs))) { cudaStreamSynchronize(sg.s); return rc; }
     k_geo_dst<<<blocks(nplace), T, 0, sg.s>>>(g, d_dst);
     int bad = 0;
     if ((e = cudaGetLastError()) != cudaSuccess ||
