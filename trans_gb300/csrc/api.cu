@@ -189,8 +189,7 @@ long long trans_device_bytes(void* ctx) {
     long long b = 0;
     for (const CaseRec* cs : c->cases)
         b += (long long)(cs->arena_doubles * (sizeof(double) + (cs->farena ? sizeof(float) : 0)));
-    const long long dq_arrays = c->fl->sweep_pair ? 2 : 1;      // the mixed path's two-plane schedule keeps a second one
-    b += (c->sv.n + 31) / 32 * 32 * ((long long)(c->fl->rec_width + dq_arrays * DQ_STRIDE) * (long long)c->fl->elem + 8LL * (long long)sizeof(int));
+    b += c->sweep_bytes + c->aux_bytes;
     return b;
 }
 

@@ -111,7 +111,7 @@ int trans_batch_case_norms(void* ctx, int case_id, int* iterations, trans_norms*
 
 long long trans_batch_bytes_in_use(void* ctx) {
     Ctx* c = static_cast<Ctx*>(ctx);
-    return c ? c->in_use : 0;
+    return c ? c->in_use + c->extra : 0;
 }
 
 int trans_batch_get_integrals(void* ctx, int case_id, trans_integrals* out) {

@@ -118,22 +118,25 @@ int upload_walls(Ctx* c, const HostBlock& h, const DevBlock& b) {
 
 }  // namespace
 
-// Device bytes one case takes: its slot arena (+ FP32 copies in the mixed path) and its share
-// of the sweep-order arrays and work lists.
+// The sweep arrays' bytes a case is charged for an interior cell: those of the hyperplane order (DeltaQ
+// arrays: the sweep's, the tuner's copy, and in the mixed path the two-plane schedule's second one).
+size_t case_cell_bytes(bool mixed, bool precond) {
+    static_assert(sizeof(SweepCell) == 16, "");
+    return plane_cell_bytes(mixed ? NCREC : NREC, mixed ? 3 : 2, DQ_STRIDE, mixed ? 4 : 8, precond ? 6 * NPC : 0);
+}
+
+// Device bytes one case is charged: its slot arena (+ FP32 copies in the mixed path) and its share
+// of the sweep-order arrays and work lists.  What the lists take beyond it where there is room (the marching
+// order of blocks that fill its tiles badly, the face fluxes' shared terms) is Ctx::extra.
 long long case_bytes(const trans_params* p, int nblocks, const trans_block* blocks) {
-    const int precision = p->precision;
+    const bool mixed = p->precision == TRANS_MIXED;
     long long padded = 0, interior = 0;
     for (int n = 0; n < nblocks; ++n) {
         padded += (long long)padded_pi(blocks[n].ni) * (blocks[n].nj + 5) * (blocks[n].nk + 5);
         interior += (long long)(blocks[n].ni - 1) * (blocks[n].nj - 1) * (blocks[n].nk - 1);
     }
-    const long long elem = precision == TRANS_MIXED ? 4 : 8;
-    long long b = padded * case_slots(*p) * (8 + (precision == TRANS_MIXED ? 4 : 0));
-    const long long rec = precision == TRANS_MIXED ? NCREC : NREC;      // sweep record entries per position
-    // DeltaQ arrays: the sweep's, the tuner's copy, and in the mixed path the two-plane schedule's second one
-    const long long ndq = precision == TRANS_MIXED ? 3 : 2;
-    b += interior * ((rec + ndq * DQ_STRIDE) * elem + 8LL * 4 + (long long)sizeof(SweepCell));
-    if (p->IF_Precondition == 1) b += interior * 6LL * NPC * 8;          // the neighbours' PrecondDW coefficients
+    long long b = padded * case_slots(*p) * (8 + (mixed ? 4 : 0));
+    b += interior * (long long)case_cell_bytes(mixed, p->IF_Precondition == 1);
     b += interior / 16 + 4096;           // tiles, norm partials, boundary tables (rounded up)
     return b;
 }
@@ -248,6 +251,8 @@ void free_worklists(Ctx* c) {
     dfree(c->d_aux); dfree(c->d_mtiles); dfree(c->d_mruns); dfree(c->d_medgeJ); dfree(c->d_medgeK); dfree(c->d_mctl);
     c->n_mtiles = c->n_mruns = 0;
     c->march = false;
+    c->sweep_bytes = c->aux_bytes = c->extra = 0;
+    c->sv = SweepView{};
     c->pair_lo.clear(); c->pair_up.clear(); dfree(c->d_parts); dfree(c->d_pc);
     dfree(c->d_cdev); dfree(c->d_stage); dfree(c->d_tile_first); dfree(c->d_norms);
     dfree(c->d_tiles); dfree(c->d_tflags); dfree(c->d_qpos); dfree(c->d_bc_first); dfree(c->d_intg);
@@ -289,6 +294,14 @@ CaseRec* case_find(Ctx* c, int id) {
     return nullptr;
 }
 
+// The work lists given back before the cases change (the next rebuild makes those of the new set).
+static int drop_worklists(Ctx* c) {
+    if (!c->built) return TRANS_OK;
+    CK(cudaStreamSynchronize(c->stream));
+    free_worklists(c);
+    return TRANS_OK;
+}
+
 int case_add(Ctx* c, const trans_params* p, int nblocks, const trans_block* blocks, CaseRec** out) {
     if (!p || !blocks || nblocks <= 0) return fail(c, TRANS_E_ARG, "null case");
     if (!params_supported(p)) return fail(c, TRANS_E_ARG, "option outside the supported configurations");
@@ -305,6 +318,12 @@ int case_add(Ctx* c, const trans_params* p, int nblocks, const trans_block* bloc
     const long long need = case_bytes(p, nblocks, blocks);
     const int nslot = case_slots(*p);
     if (c->budget > 0 && c->in_use + need > c->budget) return fail(c, TRANS_E_MEMORY, "case does not fit the device budget");
+    // what the lists hold beyond the charges gives way to the case
+    const bool had_lists = c->built;
+    if (c->extra > 0 && c->budget > 0 && c->in_use + c->extra + need > c->budget) {
+        const int rc = drop_worklists(c);
+        if (rc) return rc;
+    }
     CaseRec* cs = new CaseRec();
     cs->p = *p;
     cs->dp = make_params(*p);
@@ -335,12 +354,19 @@ int case_add(Ctx* c, const trans_params* p, int nblocks, const trans_block* bloc
         if (cs->arena) cudaFree(cs->arena);
         if (cs->farena) cudaFree(cs->farena);
         delete cs;
+        cudaGetLastError();
+        if (had_lists && !c->built) rebuild(c);       // the cases that are there go on as they were
         return fail(c, code, what);
     };
-    if (cudaMalloc(&cs->arena, total * sizeof(double)) != cudaSuccess) return bail(TRANS_E_MEMORY, "device arena");
+    auto room = [&](void** d, size_t bytes) {
+        if (cudaMalloc(d, bytes) == cudaSuccess) return true;
+        cudaGetLastError();
+        return c->built && drop_worklists(c) == TRANS_OK && cudaMalloc(d, bytes) == cudaSuccess;
+    };
+    if (!room((void**)&cs->arena, total * sizeof(double))) return bail(TRANS_E_MEMORY, "device arena");
     if (cudaMemset(cs->arena, 0, total * sizeof(double)) != cudaSuccess) return bail(TRANS_E_CUDA, "arena clear");
     if (c->mixed) {
-        if (cudaMalloc(&cs->farena, total * sizeof(float)) != cudaSuccess) return bail(TRANS_E_MEMORY, "FP32 arena");
+        if (!room((void**)&cs->farena, total * sizeof(float))) return bail(TRANS_E_MEMORY, "FP32 arena");
         if (cudaMemset(cs->farena, 0, total * sizeof(float)) != cudaSuccess) return bail(TRANS_E_CUDA, "FP32 arena clear");
     }
     size_t pos = 0;
@@ -366,6 +392,7 @@ int case_remove(Ctx* c, int id) {
         CaseRec* cs = c->cases[q];
         if (cs->id != id) continue;
         CK(cudaStreamSynchronize(c->stream));
+        if (c->built) free_worklists(c);
         cudaFree(cs->arena);
         if (cs->farena) cudaFree(cs->farena);
         c->in_use -= cs->bytes;

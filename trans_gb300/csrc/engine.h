@@ -14,6 +14,7 @@
 
 #include "../../include/trans_gpu.h"
 #include "launch.h"
+#include "sweep_bytes.h"
 #include "types.cuh"
 
 namespace tg {
@@ -128,6 +129,8 @@ struct Ctx {
     int2* d_mruns = nullptr;
     int n_mruns = 0;
     void *d_medgeJ = nullptr, *d_medgeK = nullptr;
+    // device bytes of the sweep arrays and of d_aux; of both, those beyond what the cases are charged
+    long long sweep_bytes = 0, aux_bytes = 0, extra = 0;
     MarchCtl* d_mctl = nullptr;
     double* d_pc = nullptr;              // PrecondDW coefficients of the sweep neighbours (IF_Precondition = 1)
     NormPart* d_parts = nullptr;
@@ -165,6 +168,7 @@ struct Ctx {
     int* d_tflags = nullptr;             // 2 x ntiles publish flags + the tile counter
     TileView tv{};
     bool sweep_forced = false;
+    int tuned_mode = -1;                 // the schedule the tuner picked, and
     long long tuned_positions = 0;       // sweep positions the schedule was tuned on (0: never tuned)
     int pdl = 1;                         // chain hyperplane launches (programmatic dependent launch;
                                          // 2 = the mixed path's release of the next launch at entry)
@@ -216,6 +220,7 @@ bool params_supported(const trans_params* p);
 int validate_case(const trans_params* p, int nblocks, const trans_block* blocks);
 int ctx_init(Ctx* c, int precision, long long budget);
 void read_spin_limit(Ctx* c);
+size_t case_cell_bytes(bool mixed, bool precond);
 void ctx_free(Ctx* c);
 long long case_bytes(const trans_params* p, int nblocks, const trans_block* blocks);
 // sub-iterations of one outer iteration: 3 SSP-RK3 stages, Kchld dual-time steps or 1 (main.F90:54-56)

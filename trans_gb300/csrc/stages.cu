@@ -511,6 +511,7 @@ int tune_sweeps(Ctx* c) {
         c->tile_default[0] = pick.ti; c->tile_default[1] = pick.tj; c->tile_default[2] = pick.tk;   // kept over rebuilds
     }
     c->tuned_positions = c->sv.n;
+    c->tuned_mode = pick.mode;
     c->sweep_mode = pick.mode; c->sweep_grid = pick.grid; c->sweep_block = pick.block;
     c->sweep_wpc = pick.wpc;
     c->sweep_pf = pick.pf;

@@ -220,8 +220,8 @@ bool build_resid_tma(Ctx* c) {
 
 // The marching sweeps' tiles (MarchTile, types.cuh), in an order in which a tile's j- and k-neighbours on
 // the lower side come first (by tile diagonal, then block), and the sweep arrays stored in their
-// order.  Leaves c->march false where the places are beyond int indexes or the edge buffers do not
-// fit: the context then keeps the hyperplane order and its schedules.
+// order.  Leaves c->march false where the places are beyond int indexes or the arrays do not fit
+// (march_fits): the context then keeps the hyperplane order and its schedules.
 int build_march(Ctx* c) {
     const int nblk = (int)c->blk.size();
     std::vector<int> ntj(nblk), ntk(nblk);
@@ -236,6 +236,21 @@ int build_march(Ctx* c) {
     std::stable_sort(keys.begin(), keys.end(), [](const Key& a, const Key& b) { return a.d < b.d; });
     std::vector<std::vector<int>> first(nblk);         // first step of tile (tj, tk)
     for (int n = 0; n < nblk; ++n) first[n].assign((size_t)ntj[n] * ntk[n], -1);
+    // sizes first: the cases are charged for the hyperplane order
+    const size_t word = (c->mixed ? MARCH_EDGES : M64_EDGES) * sizeof(ulonglong2);     // 8 floats or 7 doubles, every 32 bits with the tag
+    const size_t width = c->mixed ? (size_t)NCREC : (size_t)M64_WIDTH, elem = c->fl->elem;
+    size_t bytes = 0, charged = 0;
+    for (const DevBlock& b : c->blk) {
+        bytes += march_block_bytes(b.NI1, b.NJ1, b.NK1, MARCH_J, MARCH_K, width, DQ_STRIDE, elem, word, sizeof(MarchTile),
+                                   c->mixed ? 0 : sizeof(int2), M64_JAC_STEPS).bytes;
+        charged += (size_t)b.nint * case_cell_bytes(c->mixed, false);
+    }
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+        cudaGetLastError();
+        return TRANS_OK;
+    }
+    if (!c->sweep_forced && !march_fits(bytes, charged, free_b, c->budget > 0 ? c->budget - c->in_use : -1)) return TRANS_OK;
     long long s0 = 0;
     for (const Key& k : keys) {
         first[k.n][k.tj + (size_t)ntj[k.n] * k.tk] = (int)s0;
@@ -252,16 +267,8 @@ int build_march(Ctx* c) {
                                   at(k.tj, k.tk), {at(k.tj - 1, k.tk), at(k.tj + 1, k.tk)}, {at(k.tj, k.tk - 1), at(k.tj, k.tk + 1)},
                                   k.n, k.tj * MARCH_J + 1, k.tk * MARCH_K + 1});
     }
-    const size_t word = (c->mixed ? MARCH_EDGES : M64_EDGES) * sizeof(ulonglong2);     // 8 floats or 7 doubles, every 32 bits with the tag
     const size_t nj = (size_t)s0 * MARCH_K * word, nk = (size_t)s0 * MARCH_J * word, places = (size_t)s0 * 32;
-    const size_t nrec = places * (c->mixed ? (size_t)NCREC : (size_t)M64_WIDTH) * c->fl->elem, ndq = places * DQ_STRIDE * c->fl->elem;
-    // (where they would take more than half of the free device memory, the hyperplane order, which is
-    // smaller for blocks of few lines, and leaves the rest of the work lists their room)
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || nj + nk + nrec + ndq > free_b / 2) {
-        cudaGetLastError();
-        return TRANS_OK;
-    }
+    const size_t nrec = places * width * elem, ndq = places * DQ_STRIDE * elem;
     auto room = [](void* p, size_t bytes) { return cudaMalloc((void**)p, bytes) == cudaSuccess; };
     if (!room(&c->d_medgeJ, nj) || !room(&c->d_medgeK, nk) || !room(&c->d_rec, nrec) || !room(&c->d_dqs, ndq)) {
         cudaGetLastError();
@@ -302,6 +309,8 @@ int build_march(Ctx* c) {
     c->sv = SweepView{};
     c->sv.rec = c->d_rec; c->sv.dq = c->d_dqs; c->sv.n = (long long)places;
     c->march = true;
+    c->sweep_bytes = (long long)bytes;
+    c->extra = bytes > charged ? (long long)(bytes - charged) : 0;
     return TRANS_OK;
 }
 
@@ -314,12 +323,14 @@ int build_terms(Ctx* c) {
     size_t n = 0, free_b = 0, total_b = 0;
     for (const DevBlock& b : c->blk) n += (size_t)b.ncell * entries(b);
     const size_t bytes = n * sizeof(double);
-    if (c->budget > 0 && c->in_use + (long long)bytes > c->budget) return TRANS_OK;
+    if (c->budget > 0 && c->in_use + c->extra + (long long)bytes > c->budget) return TRANS_OK;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 8 || cudaMalloc(&c->d_aux, bytes) != cudaSuccess) {
         cudaGetLastError();
         c->d_aux = nullptr;
         return TRANS_OK;
     }
+    c->aux_bytes = (long long)bytes;
+    c->extra += (long long)bytes;
     size_t at = 0;
     for (DevBlock& b : c->blk) {
         b.aux = c->d_aux + at;
@@ -472,6 +483,8 @@ int rebuild(Ctx* c) {
                 if ((rc = upload_vec(c, orph.data(), sizeof(int) * orph.size(), (void**)&c->d_orph))) return rc;
             }
             CK(cudaMalloc(&c->d_flags, (size_t)2 * Np * sizeof(int)));
+            c->sweep_bytes = Np * ((long long)(c->fl->rec_width + (c->fl->sweep_pair ? 2 : 1) * DQ_STRIDE) * (long long)c->fl->elem +
+                                   8LL * (long long)sizeof(int));
             c->sv.cells = c->d_sweep; c->sv.nbp = c->d_nbp; c->sv.rec = c->d_rec; c->sv.dq = c->d_dqs; c->sv.n = N;
             c->sv.pc = nullptr;
             if (c->cases[0]->p.IF_Precondition == 1) {      // the neighbours' PrecondDW coefficients (FP64 path)
@@ -504,8 +517,8 @@ int rebuild(Ctx* c) {
     // times ~40 candidate sweeps); the schedule kept is re-captured for the new work lists
     const long long npos = (long long)c->sweep.size();
     if (c->march) c->sweep_mode = 6;
-    else if (!c->sweep_forced && (c->sweep_mode == 6 || c->tuned_positions <= 0 || npos > 2 * c->tuned_positions || 2 * npos < c->tuned_positions))
-        c->sweep_mode = -1;
+    else if (!c->sweep_forced)
+        c->sweep_mode = c->tuned_positions > 0 && npos <= 2 * c->tuned_positions && 2 * npos >= c->tuned_positions ? c->tuned_mode : -1;
     if ((rc = build_terms(c))) return rc;
     c->built = true;
     return TRANS_OK;
