@@ -55,6 +55,16 @@ def test_bytes(rule, mixed, dims):
         assert p == ni * nj * nk * ((160 + 16) * 8 + 48)
 
 
+def test_the_smaller_order_near_the_memory_limit(rule):
+    """A large FP64 block marches whatever is free (the other order needs 1.7 times as much); a block of few
+    lines takes the hyperplane order when marching would take more than half of the free memory."""
+    m, p, chosen = rule(0, (120, 64, 64), free=105)
+    assert m < p / 1.6 and chosen
+    m, p, chosen = rule(0, (400, 3, 3), free=199)
+    assert m > p and not chosen
+    assert rule(0, (400, 3, 3), free=201)[2]
+
+
 @pytest.mark.parametrize("mixed", [0, 1])
 def test_budget(rule, mixed):
     """What the marching arrays take beyond the charge has to fit the budget that is left."""

@@ -24,12 +24,15 @@ inline MarchBytes march_block_bytes(int ni, int nj, int nk, int J, int K, size_t
     return {tiles * steps, tiles * (steps * per_step + tile + runs * run)};
 }
 
-// The marching order, unless what it takes beyond the charge (the hyperplane order's bytes; blocks whose lines
-// fill their tiles badly, or that are short along i: it is padded to whole tiles and steps) does not fit the
-// budget that is left (left < 0: no budget), or the marching arrays would take more than half of the free device
-// memory.
+// The marching order, unless the hyperplane order is the smaller (blocks whose lines fill their tiles badly, or
+// that are short along i: it is padded to whole tiles and steps) and the difference does not fit the
+// budget that is left (left < 0: no budget), or the marching arrays would take more than half of the free
+// device memory, which the context's other lists, the next cases and their fields need too.  Where the marching
+// arrays are the smaller, as on every large FP64 block (656 bytes of record a place against 1,280 a cell), the
+// other order could only need more.
 inline bool march_fits(size_t march, size_t planes, size_t free_bytes, long long left) {
-    if (march > planes && left >= 0 && march - planes > (size_t)left) return false;
+    if (march <= planes) return true;
+    if (left >= 0 && march - planes > (size_t)left) return false;
     return march <= free_bytes / 2;
 }
 
