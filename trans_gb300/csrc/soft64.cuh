@@ -13,7 +13,11 @@
 //         divisor that is biased low, so a digit is never too large; the remainders are exact
 //         64-bit integers (two 32-bit multiplies a digit).  A quotient of two 53-bit significands
 //         is never half-way between two doubles, so 54 quotient bits decide the rounding.
-//   sqrt: the same digit recurrence, R - d (2 s + d), from an FP32 reciprocal square root.
+//   sqrt: the same digit recurrence, R - d (2 s + d), from an FP32 reciprocal square root.  A digit is never
+//         too large if y <= (1 - 2^-24) / r for the root r (the product that forms it may round up by 2^-24).
+//         With an approximation off by at most 2^-22 and one rounding of y, a bias of 3 x 2^-23 leaves that:
+//         (1 + 2^-22) (1 - 1.5 x 2^-22) (1 + 2^-24) < 1 - 2^-24.  The other way a digit falls short by
+//         less than 8, 15 and 2 units (the bounds below), so that the remainders keep to their 23 leading bits.
 #pragma once
 #include <math.h>
 #include <stdint.h>
@@ -65,15 +69,20 @@ SX_FN float fof(uint32_t u) {
     return x;
 #endif
 }
-// 1/x and 1/sqrt(x) to within 2^-22 relative (the hardware approximations; the exact functions
-// on the host): the callers' bias covers either
+// 1/x and 1/sqrt(x) to within 2^-22 relative (the hardware approximations, documented at 1 ulp and
+// 2^-22.9; the rounded functions on the host, where a test may put others within 2^-22): the callers' bias covers
+// either
+#ifndef SX_HOST_RCP
+#define SX_HOST_RCP(x) (1.0f / (x))
+#define SX_HOST_RSQRT(x) (1.0f / sqrtf(x))
+#endif
 SX_FN float rcp_approx(float x) {
 #ifdef __CUDA_ARCH__
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 #else
-    return 1.0f / x;
+    return SX_HOST_RCP(x);
 #endif
 }
 SX_FN float rsqrt_approx(float x) {
@@ -82,7 +91,7 @@ SX_FN float rsqrt_approx(float x) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 #else
-    return 1.0f / sqrtf(x);
+    return SX_HOST_RSQRT(x);
 #endif
 }
 // an integer below 2^23 as a float, and the integer part of a float in [0, 2^23): through the
@@ -159,17 +168,17 @@ SX_FN double sqrt(double a) {
     const uint32_t odd = (ea & 1u) ^ 1u;                 // the unbiased exponent is odd
     const uint64_t X = ((ua & FRAC) | IMPL) << odd;
     const uint32_t e = ((ea + 1023u - odd) >> 1) - 1u;   // biased exponent of the root, less 1
-    // y <= 1 / sqrt(X 2^-52), by less than 2^-21 relative
+    // y <= (1 - 2^-24) / sqrt(X 2^-52)
     const float x24 = small_float((uint32_t)(X >> 31));                        // in units of 2^-21
-    const float y = rsqrt_approx((x24 + 1.0f) * 4.76837158203125e-7f) * 0.99999976158142089844f;  // 1 - 2^-22
-    // digit 1 (below 2^23): the root in units of 2^-22, at most 7 too small
+    const float y = rsqrt_approx((x24 + 1.0f) * 4.76837158203125e-7f) * 0.99999964237213134765625f;  // 1 - 3 2^-23
+    // digit 1 (below 2^23): the root in units of 2^-22, too small by less than 3 r + 2 / r + 0.75 < 8
     const uint32_t d1 = small_int(x24 * (y * 2.0f));
-    uint64_t R = X - (((uint64_t)d1 * d1) << 8);         // 2^8 times the remainder, < 2^36
-    // digit 2: units of 2^-42
+    uint64_t R = X - (((uint64_t)d1 * d1) << 8);         // 2^8 times the remainder, < 2^35
+    // digit 2 (below 2^23): units of 2^-42, less than 15 too small
     const uint32_t d2 = small_int(small_float((uint32_t)(R >> 13)) * (y * 4.0f));
-    R = (R << 32) - mul64x32(((uint64_t)d1 << 21) + d2, d2);
+    R = (R << 32) - mul64x32(((uint64_t)d1 << 21) + d2, d2);                   // < 60 x 2^42
     const uint64_t s = ((uint64_t)d1 << 20) + d2;
-    // digit 3: units of 2^-53
+    // digit 3: units of 2^-53, at most 1 too small
     const uint32_t d3 = small_int(small_float((uint32_t)(R >> 25)) * (y * 0.0078125f));
     R = (R << 22) - mul64x32((s << 12) + d3, d3);
     uint64_t N = (s << 11) + d3;
