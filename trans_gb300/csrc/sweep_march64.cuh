@@ -49,9 +49,10 @@ struct March64Walk {
     int lane, a, b, cell, steps, lastJ, lastK;     // lastJ, lastK: steps with an edge word for this lane
     long long q0;
     bool in_jk, outJ, outK, lost;                  // lost: given up, the tile goes on without the words
+    int stalled;                                   // the step whose inputs did not come, or -1
     __device__ March64Walk(const MarchTile& T_, const f64* rec_, f64* dq_, ulonglong2* bJ, ulonglong2* bK, unsigned tag_, SweepSync* sy_,
                            unsigned limit_)
-        : T(T_), rec(rec_), dq(dq_), bufJ(bJ), bufK(bK), tag(tag_), limit(limit_), sy(sy_), lost(false) {
+        : T(T_), rec(rec_), dq(dq_), bufJ(bJ), bufK(bK), tag(tag_), limit(limit_), sy(sy_), lost(false), stalled(-1) {
         lane = threadIdx.x & 31;
         a = lane % LJ;
         b = lane / LJ;
@@ -77,7 +78,7 @@ struct March64Walk {
 };
 
 // Bulk copies of a step's inputs into a stage, complete on a transaction barrier; the wait for a phase
-// is bounded.  Four stages leave two mean-flow CTAs on an SM: at 1,966,080 cells 3.42 ms for both sweeps,
+// is bounded like the others (and at M64_PHASE_LIMIT polls).  Four stages leave two mean-flow CTAs on an SM: at 1,966,080 cells 3.42 ms for both sweeps,
 // against 3.71 with three stages and CTAs and 4.03 with two stages and four (the CTAs of one SM
 // are on one diagonal, and the steps of each take longer); no difference at the smaller sizes.
 constexpr int M64_STAGES = 4;
@@ -91,14 +92,32 @@ __device__ __forceinline__ void march64_copy(f64* dst, const f64* src, unsigned 
 __device__ __forceinline__ void march64_expect(unsigned bar, unsigned rows) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(rows * 256u) : "memory");
 }
-__device__ __forceinline__ void march64_phase(unsigned bar, unsigned parity, SweepSync* sy) {
-    for (unsigned n = 0; n < M64_PHASE_LIMIT; ++n) {
-        unsigned ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return;
-    }
-    atomicExch(&sy->err, 1);
+__device__ __forceinline__ bool march64_complete(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok;
+}
+// a wait for the inputs of step t that the first look did not end: the step at which the tile gave up, or -1
+static __device__ __noinline__ int march64_wait(unsigned bar, unsigned parity, int t, unsigned limit, SweepSync* sy) {
+    for (unsigned n = 1; !march64_complete(bar, parity); ++n)
+        if (n > min(limit, M64_PHASE_LIMIT) || (n % 1024u == 0 && *((volatile int*)&sy->err))) {
+            atomicExch(&sy->err, 1);
+            return t;
+        }
+    return -1;
+}
+// the inputs of step t are there; should the wait run out (or another have given up), the tile goes on without
+// them, and without further waits and copies (w.stalled: the step)
+template <class W>
+__device__ __forceinline__ void march64_phase(W& w, unsigned bar, unsigned parity, int t) {
+    if (!march64_complete(bar, parity) && w.stalled < 0) w.stalled = march64_wait(bar, parity, t, w.limit, w.sy);
+}
+// the lane that issued the copies, after a wait that ran out: those of steps before `issued` land before the CTA gives
+// up its shared memory
+__device__ __forceinline__ void march64_drain(unsigned full, int issued) {
+    for (int st = 0; st < M64_STAGES && st < issued; ++st)
+        for (unsigned n = 0; n < M64_PHASE_LIMIT && !march64_complete(full + 8 * st, (unsigned)((issued - 1 - st) / M64_STAGES) & 1u); ++n) {}
 }
 
 // The edge words of one component: read a step ahead, polled where they have not arrived.
@@ -190,7 +209,7 @@ struct March64Mean {
                 xj = f64(__shfl_up_sync(0xffffffffu, cj.v, 1));
                 xk = f64(__shfl_up_sync(0xffffffffu, ck.v, LJ));
             }
-            march64_phase(full + 8 * st, ph, w.sy);
+            march64_phase(w, full + 8 * st, ph, t);
             edge.take(w, L, t, xj, xk);
             const f64 v = march64_step<LOWER>(w, L, t, act, q[M64_MEAN_ROWS + L][cell], q[M64_STEPT][cell], q[M64_CVS][cell],
                                               q[M64_FM][cell], xi, xj, xk);
@@ -198,7 +217,7 @@ struct March64Mean {
             asm volatile("bar.sync 1, 160;" ::: "memory");
             if constexpr (ROLE == 2) {
                 // every warp is past step t - 1: its stage takes the inputs of a later step
-                if (lane == 0) copy(t + M64_STAGES - 1);
+                if (lane == 0 && w.stalled < 0) copy(t + M64_STAGES - 1);
             } else {
                 f64 A[5];                          // the step's increments of the lane's cell
 #pragma unroll
@@ -235,7 +254,10 @@ struct March64Mean {
             }
             if (++st == M64_STAGES) { st = 0; ph ^= 1u; }
         }
-        if constexpr (ROLE == 2) asm volatile("bar.sync 2, 128;" ::: "memory");    // the last step's arrivals
+        if constexpr (ROLE == 2) {
+            asm volatile("bar.sync 2, 128;" ::: "memory");                         // the last step's arrivals
+            if (lane == 0 && w.stalled >= 0) march64_drain(full, min(w.stalled + M64_STAGES - 1, w.steps));
+        }
     }
 };
 
@@ -262,7 +284,7 @@ __device__ __forceinline__ void march64_turb(const int L, March64Walk<LOWER>& w,
         const f64(*const q)[32] = in[st];
         const bool act = w.active(t);
         f64 xj = f64(__shfl_up_sync(0xffffffffu, cj.v, 1)), xk = f64(__shfl_up_sync(0xffffffffu, ck.v, MARCH_J));
-        march64_phase(full + 8 * st, ph, w.sy);
+        march64_phase(w, full + 8 * st, ph, t);
         f64 vp[3], rds[3];
 #pragma unroll
         for (int dir = 0; dir < 3; ++dir) {
@@ -272,7 +294,7 @@ __device__ __forceinline__ void march64_turb(const int L, March64Walk<LOWER>& w,
         const f64 own = q[M64_TURB_IN - 1][cell], stept = q[M64_STEPT - M64_TURB_ROW0][cell], cvs = q[M64_CVS - M64_TURB_ROW0][cell],
                   den = q[M64_FT - M64_TURB_ROW0][cell];
         __syncwarp();                              // the stage is read
-        if (lane == 0) copy(t + M64_STAGES);
+        if (lane == 0 && w.stalled < 0) copy(t + M64_STAGES);
         edge.take(w, L, t, xj, xk);
         const f64 v = march64_step<LOWER>(w, L, t, act, own, stept, cvs, den, ci, xj, xk);
         f64 x[3];
@@ -285,6 +307,7 @@ __device__ __forceinline__ void march64_turb(const int L, March64Walk<LOWER>& w,
         w.put_k(L, t, ck);
         if (++st == M64_STAGES) { st = 0; ph ^= 1u; }
     }
+    if (lane == 0 && w.stalled >= 0) march64_drain(full, min(w.stalled + M64_STAGES, w.steps));
 }
 
 // A CTA takes the mean flow of a tile, or k and omega of two.  TURB: the components swept, 0 mean flow,
