@@ -191,8 +191,8 @@ int trans_run_stage(void* ctx, int stage, int ki, int itr_chld);
 int trans_get_norms(void* ctx, trans_norms* norms);
 /* Prepares the context for iteration KI (KI < 0: each case's next iteration) without running it
  * (no reference counterpart): builds
- * the work lists and geometry terms, tunes the LU-SGS sweep schedule on a right-hand side of
- * the current state and captures the iteration graph that trans_time_iterations and
+ * the work lists and geometry terms, where the sweeps are not the marching ones times their schedules on a
+ * right-hand side of the current state, and captures the iteration graph that trans_time_iterations and
  * trans_batch_iterate replay (8 outer iterations per replay).  The interior state is unchanged. */
 int trans_prepare(void* ctx, int ki);
 /* One outer iteration with CUDA events around every stage on the context's stream; ms receives
@@ -298,6 +298,9 @@ int trans_batch_time_iterations(void* ctx, int n, double* ms);
 /* Iterations done by a case, its per-block norms of its first and of its last iteration
  * (arrays of nblocks entries, either may be NULL). */
 int trans_batch_case_norms(void* ctx, int case_id, int* iterations, trans_norms* first, trans_norms* last);
+/* The cases' charges (trans_batch_case_bytes), and what the work lists hold beyond them where the budget
+ * has room (arrays of the marching sweeps, shared terms of the FP64 face fluxes: given back when a case needs
+ * the room). */
 long long trans_batch_bytes_in_use(void* ctx);
 /* As trans_get_integrals / trans_get_wall_cp for one case; one launch covers all cases, so a
  * serving loop reads every case's integrals at once with trans_batch_integrals (ids[k] and
@@ -335,7 +338,7 @@ int trans_update_static_scratch(void* ctx, int ki, trans_norms* norms);
 #define TRANS_NKCLASS 17
 int trans_kernel_times(void* ctx, int ki, double* ms, int* launches, int n);
 const char* trans_kernel_class(int k);
-/* The schedule the context's tuner picked for the LU-SGS sweeps and what it measured (no
+/* The schedule of the LU-SGS sweeps, and what the tuner measured where it picked it (no
  * reference counterpart).  The string lives until the next call on this thread. */
 const char* trans_tuning(void* ctx);
 /* Diagnostic, no reference counterpart: checks on the current device the integer-pipe
@@ -344,8 +347,9 @@ const char* trans_tuning(void* ctx);
  * (signed zeros, infinities, NaN, the float range limits, rounding ties).  mismatches[0]
  * counts double -> float results that differ in any bit, mismatches[1] float -> double (NaN
  * equals NaN); both are 0 on a correct build.  The patterns, taken in pairs, also check the FP64
- * path's integer-pipe quotients (counted in mismatches[0]) and square roots (mismatches[1])
- * against the hardware's.  Errors: TRANS_E_ARG, TRANS_E_CUDA (message in
+ * path's integer-pipe quotients and square roots against the hardware's; their mismatches are added to
+ * mismatches[0] and mismatches[1], and trans_last_error(NULL) then gives the four counts.
+ * Errors: TRANS_E_ARG, TRANS_E_CUDA (message in
  * trans_last_error(NULL)). */
 int trans_check_conversions(long long n, unsigned long long seed, long long* mismatches);
 /* Message of the last failed call on ctx; with ctx = NULL, of the last failed context-free call

@@ -216,11 +216,17 @@ int trans_check_conversions(long long n, unsigned long long seed, long long* mis
         g_stateless_err = "trans_check_conversions: n must be 1..2^32 and mismatches non-NULL";
         return TRANS_E_ARG;
     }
-    const cudaError_t e = check_conversions(n, seed, mismatches);
+    long long m[4] = {0, 0, 0, 0};
+    const cudaError_t e = check_conversions(n, seed, m);
+    mismatches[0] = m[0] + m[2];
+    mismatches[1] = m[1] + m[3];
     if (e != cudaSuccess) {
         g_stateless_err = std::string("trans_check_conversions: ") + cudaGetErrorString(e);
         return TRANS_E_CUDA;
     }
+    if (mismatches[0] || mismatches[1])
+        g_stateless_err = "trans_check_conversions: mismatches of double -> float " + std::to_string(m[0]) + ", float -> double "
+                          + std::to_string(m[1]) + ", quotients " + std::to_string(m[2]) + ", square roots " + std::to_string(m[3]);
     return TRANS_OK;
 }
 

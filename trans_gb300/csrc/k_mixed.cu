@@ -240,7 +240,7 @@ __global__ void k_check_cvt(long long n, unsigned long long seed, unsigned long 
     const unsigned long long z = cvt_mix((unsigned long long)g ^ (seed * 0x2545f4914f6cdd1dull));
     unsigned long long u;
     const int kind = (int)(g & 3);
-    check_arith(z, cvt_mix(z), bad);
+    check_arith(z, cvt_mix(z), bad + 2);
     if (g < CVT_NSPECIAL) {
         u = cvt_special[g];
         const unsigned f = (unsigned)(u >> 32) ^ (unsigned)u;     // a float pattern from it too
@@ -267,9 +267,9 @@ __global__ void k_check_cvt(long long n, unsigned long long seed, unsigned long 
 
 cudaError_t check_conversions(long long n, unsigned long long seed, long long* mismatches) {
     unsigned long long* d = nullptr;
-    cudaError_t e = cudaMalloc(&d, 2 * sizeof(unsigned long long));
+    unsigned long long h[4] = {0, 0, 0, 0};        // double -> float, float -> double, quotients, roots
+    cudaError_t e = cudaMalloc(&d, sizeof(h));
     if (e != cudaSuccess) return e;
-    unsigned long long h[2] = {0, 0};
     e = cudaMemset(d, 0, sizeof(h));
     if (e == cudaSuccess) {
         k_check_cvt<<<(unsigned)((n + 255) / 256), 256>>>(n, seed, d);
@@ -277,8 +277,7 @@ cudaError_t check_conversions(long long n, unsigned long long seed, long long* m
     }
     if (e == cudaSuccess) e = cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost);
     cudaFree(d);
-    mismatches[0] = (long long)h[0];
-    mismatches[1] = (long long)h[1];
+    for (int q = 0; q < 4; ++q) mismatches[q] = (long long)h[q];
     return e;
 }
 }  // namespace tg
