@@ -246,7 +246,7 @@ const char* trans_tuning(void* ctx) {
           + (c->sweep_wpc ? "/wpc" : "")
           + (c->sweep_pf && (c->sweep_mode == 0 || c->sweep_mode == 4 || c->sweep_mode == 5) ? "/pf" + std::to_string(c->sweep_pf) : "")
           + (c->sweep_cta && (c->sweep_mode == 0 || c->sweep_mode == 5) ? "/cta" + std::to_string(c->sweep_cta) : "")
-          + "; measured: " + c->sweep_tuning
+          + (c->sweep_tuning.empty() || c->sweep_mode == 6 ? std::string() : "; measured: " + c->sweep_tuning)
           + (c->mixed ? std::string("; residual=") + (c->resid_tma == 1 ? "tma" : c->resid_tma == 0 ? "gather" : "untuned")
                             + (c->resid_tuning.empty() ? std::string() : " (" + c->resid_tuning + ")")
                       : std::string());
