@@ -179,11 +179,10 @@ ALG_WORDS = {
     "k_update": 37, "k_gradient": 46, "k_specrad": 24, "k_lusgs_prep": 60, "k_gather": 46,
 }
 # FP64 thread-instructions per face of the FP64 face fluxes (MDCD + AUSMPW+ + SST; DADD + DMUL + DFMA of
-# k_face_terms, the viscous and the convective kernel: 87 + 372 + 621), and their DRAM bytes per face, counted by
-# ncu on the 352,256-cell cascade (profiles/fp64_kernels_cascade_352256cells.md), less 18 for the exact products
-# and zero terms taken out since (3 viscous, 15 convective)
-FACE_FP64_INST = 1062.0
-FACE_DRAM_BYTES = 1328.0
+# k_face_terms, the viscous and the convective kernel: 87 + 369 + 607), and their DRAM bytes per face, counted by
+# ncu on the 352,256-cell cascade (profiles/fp64_kernels_cascade_352256cells.md)
+FACE_FP64_INST = 1062.5
+FACE_DRAM_BYTES = 1323.0
 FACE_DRAM_SOURCE = ("ncu dram__bytes_read+write per face of the shared terms, viscous and convective kernels together on "
                     "the 352,256-cell cascade, scaled by faces")
 # kernel classes that run in FP32 in the mixed path (their algorithmic words are 4 bytes there)

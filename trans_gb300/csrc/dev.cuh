@@ -197,7 +197,6 @@ __host__ __device__ inline int cidx(const DevBlock& b, int i, int j, int k) {
     return (i + 2) + b.PI * ((j + 2) + b.PJ * (k + 2));
 }
 __device__ inline double* slot(const DevBlock& b, int s) { return b.base + (size_t)s * (size_t)b.ncell; }
-// row pitch of a block of NI nodes in i (the ghost extent NI+5 rounded up to a multiple of 4)
 // a padded cell that a stencil reads: interior, or a ghost across one face (the edges' and corners' ghosts are
 // read by nothing; their quotients of zeros went to the FP64 pipe, with the whole warp: k_prims of 1,966,080
 // cells 222 -> 81 us, 36,864 cells 30 -> 11; the mixed path's copies lose by it, 84 -> 94, bound by memory)
@@ -206,6 +205,7 @@ __device__ __forceinline__ bool read_cell(const DevBlock& b, int c) {
     const int ghost = (i < 1 || i > b.NI1) + (j < 1 || j > b.NJ1) + (k < 1 || k > b.NK1);
     return ghost <= 1 && i <= b.NI + 2;
 }
+// row pitch of a block of NI nodes in i (the ghost extent NI+5 rounded up to a multiple of 4)
 __host__ __device__ inline int padded_pi(int ni) { return (ni + 5 + 3) & ~3; }
 
 __device__ inline float* fslot(const DevBlock& b, int s) { return b.fbase + (size_t)s * (size_t)b.ncell; }

@@ -199,7 +199,7 @@ int ctx_init(Ctx* c, int precision, long long budget) {
     if (pf) c->sweep_pf = std::max(0, std::atoi(pf));
     read_spin_limit(c);
     // sweep schedule: TRANS_SWEEP=planes | coop | flow | tiles | clusters | pairs | march forces one (for tests);
-    // default: tuned
+    // default: march, or the tuner's where that does not apply
     const char* m = std::getenv("TRANS_SWEEP");
     std::string ms = m ? m : "";
     // clusters: the mixed path's cluster-barrier schedule (the FP64 path takes planes)

@@ -475,7 +475,7 @@ __global__ void k_prims(const DevBlock* __restrict__ blks, int nblk, long long t
 // averages, read by the gradient and twice or three times per face by the fluxes, and the MDCD
 // reconstruction's products and squared second differences, each formed by up to six faces before.
 // The same operations on the same operands, so the same bits.  mdcd: with the latter.  A direction's terms
-// belong to the cells that are interior in the other two; face averages from face 0 to N + 2.
+// belong to the cells that are interior in the other two; face averages from face 0 to N + 1.
 // Bound by the FP64 pipe, like its readers: 72 and 160 instructions a cell against 576 and 720 in the
 // gradient and the faces.  Gradient and face fluxes with this kernel, before and now: the 1,966,080-cell
 // cascade (MDCD) 17.0 and 13.9 ms, 352,256 cells 3.16 and 2.62, the annulus 70x38x26 (three stages) 2.23
@@ -548,10 +548,10 @@ __global__ void k_mirror(const DevBlock* __restrict__ blks, int nblk, long long 
 #endif  // TG_COMMON_KERNELS
 
 
-// (FP32 bound by load latency: with the bound below the compiler takes 113 registers for loads in flight, 93
-// without; 1,966,080 cells 112 -> 108 us, a batch of five cascades 158 -> 151; at three CTAs per SM 124)
 // ---------------------------------------------------------------------------------------
 // Space/DIFF_DqDxyz.F90:25-74, 232-265, 300-381 (gradients and shock sensor, interior cells)
+// FP32 bound by load latency: with the bound below the compiler takes 113 registers for loads in flight, 93
+// without; 1,966,080 cells 112 -> 108 us, a batch of five cascades 158 -> 151; at three CTAs per SM 124.
 // ---------------------------------------------------------------------------------------
 template <typename R, bool TERMS = false>
 __global__ void __launch_bounds__(CELL_TILE, 1) k_gradient(const DevBlock* __restrict__ blks, const Tile* __restrict__ tiles, const CaseDev* __restrict__ cdev) {
@@ -1251,9 +1251,9 @@ __device__ inline R rc_fr1(const ParamsT<R>& p, const DevBlock& b, int I, int J,
     return dmax(dmin(f_rot, R(1.25)), R(0.0));
 }
 
-// (FP32: two resident CTAs of 256 threads per SM, i.e. at most 128 registers)
 #ifndef TG_PREP_MINB
-#define TG_PREP_MINB 3      // resident CTAs per SM of the FP32 preparation (128 registers; 3 CTAs: 82 against 70 us at 352,256 cells)
+#define TG_PREP_MINB 3      // resident CTAs per SM of the FP32 preparation (80 registers, 80-byte spill; at two CTAs, 128 registers, 57
+                            // against 51 us at 352,256 cells, 252 against 225 at 1,966,080, and other multiply-adds are joined)
 #endif
 #ifndef TG_PREP_MINB_F64
 #define TG_PREP_MINB_F64 2  // ... and of the FP64 one (128 registers, 100-byte spill; at one CTA 2,377 against 2,020 us at 1,966,080)

@@ -3,7 +3,7 @@
 // The tiles, their order and the words between them are those of sweep_march.cuh; the arithmetic
 // is the reference's, operation by operation (bit-identical to the hyperplane launches).  An FP64
 // warp instruction takes its sub-partition 63 cycles, dependent or not, and a step of 32 cells has
-// ~215 of them, so a step's work is spread over the SM's four: a warp holds one component of the
+// ~205 of them (181 and 28 in the lower sweep, mean flow and k-omega; 176 and 28 in the upper), so a step's work is spread over the SM's four: a warp holds one component of the
 // tile's 32 lines.  The share of a cell in its neighbour's sum of a component is a value of that
 // component's warp, so it stays in the lane (i), or goes to lane a-1 or b-1 by shuffle (j, k); only
 // the five mean-flow increments of the step cross warps, through shared memory and one barrier.
@@ -15,11 +15,11 @@
 // three neighbours in both sweeps; the hyperplane records keep the six neighbours' (1,280 bytes,
 // each cell's terms formed twice).
 //
-// Bound by the FP64 pipe and the chain of a step: 46 FP64 instructions (1.5 us) and two divisions on
-// the integer pipe on the way from one step to the next, 2.2 us a step of a tile by itself.  Both
-// sweeps with the records' preparation, hyperplane launches before and now: 24x16x5 cells 355 and
-// 283 us, 96x48x8 1,213 and 798 us, a cascade of 352,256 cells 2,400 and 1,932 us, of 1,966,080 cells
-// 8,047 and 5,185 us; k and omega alone (Runge-Kutta, annulus 70x38x26, three stages) 2,162 and 1,268 us.
+// Bound by the FP64 pipe and the chain of a step: 46 FP64 instructions on the fullest sub-partition (1.4 us
+// at 2,070 MHz) and a division on the integer pipe on the way from one step to the next, 2.16 us a step of a
+// tile by itself.  Both sweeps with the records' preparation, hyperplane launches before and now: 24x16x5 cells
+// 355 and 274 us, 96x48x8 1,213 and 779 us, a cascade of 352,256 cells 2,400 and 1,832 us, of 1,966,080 cells
+// 8,047 and 4,838 us; k and omega alone (Runge-Kutta, annulus 70x38x26, three stages) 2,162 and 1,220 us.
 #pragma once
 #include "kernels.cuh"
 #include "launch.h"
